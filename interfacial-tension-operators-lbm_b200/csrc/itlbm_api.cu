@@ -1,4 +1,5 @@
 // itlbm_api.cu -- the C ABI (include/itlbm.h): cases, stepping, diagnostics and the operator seam.
+#include "itlbm_resident.h"
 #include "itlbm_site.cuh"
 
 #include <algorithm>
@@ -165,7 +166,20 @@ struct itlbm_case {
     long long steps = 0;
     int aux_valid = 0;
     int device = 0;
+    // the resident kernel (itlbm_resident.cu), for boxes it takes: its launch arguments, with the
+    // exchange memory and the tile table behind the state buffers
+    ResPlan plan;
+    ResArgs res{};
+    int *res_flag = nullptr;
 };
+
+namespace {
+// After a synchronisation: whether a wait of a resident launch ran out (the state is then undefined).
+int waited(const itlbm_case *c) {
+    if (!c->res_flag || *(volatile int *)c->res_flag == 0) return ITLBM_OK;
+    return fail(ITLBM_E_TIMEOUT, "a wait between the tiles of a step ran out");
+}
+}  // namespace
 
 extern "C" {
 
@@ -248,6 +262,7 @@ void itlbm_case_destroy(itlbm_case *c) {
     if (c->aux) cudaFree(c->aux);
     if (c->tmp) cudaFree(c->tmp);
     diag_free(c->diag);
+    res_flag_put(c->res_flag);
     delete c;
 }
 
@@ -282,7 +297,11 @@ int itlbm_case_create(const itlbm_case_desc *d, itlbm_case **out) {
     fill_shift(h, h.rho0, d->geometry == ITLBM_GEOM_DROP ? d->v0 : 0.0);
     const size_t elem = elem_of(d->precision);
     const size_t per_buf = (size_t)h.buf_elems * elem;
-    if ((e = cudaMalloc(&c->mem, 2 * per_buf)) != cudaSuccess) {
+    c->plan = res_plan_single(d->precision, d->nx, d->ny);
+    if (c->plan.shape >= 0 && !(c->res_flag = res_flag_get())) c->plan = ResPlan();
+    const size_t xbytes = c->plan.shape >= 0 ? res_exchange_bytes(d->precision, c->plan.shape, c->plan.tiles) : 0;
+    const size_t mem_bytes = 2 * per_buf + xbytes + sizeof(ResTile) * c->plan.tiles;
+    if ((e = cudaMalloc(&c->mem, mem_bytes)) != cudaSuccess) {
         itlbm_case_destroy(c);
         return cuda_fail(e, "cudaMalloc(state)");
     }
@@ -305,7 +324,17 @@ int itlbm_case_create(const itlbm_case_desc *d, itlbm_case **out) {
     }
     cudaMemcpy(c->tiles, tl.data(), sizeof(TileRef) * c->ntiles, cudaMemcpyHostToDevice);
     cudaMemcpy(c->dev, &h, sizeof(CaseDev), cudaMemcpyHostToDevice);
-    cudaMemset(c->mem, 0, 2 * per_buf);
+    cudaMemset(c->mem, 0, mem_bytes);
+    if (c->plan.shape >= 0) {
+        std::vector<ResTile> rt;
+        res_tiles(c->plan, 0, 0, rt);
+        char *x = (char *)c->mem + 2 * per_buf;
+        res_exchange_bind(c->res, x, d->precision, c->plan.shape, c->plan.tiles);
+        c->res.cases = c->dev;
+        c->res.tiles = (ResTile *)(x + xbytes);
+        c->res.err = c->res_flag;
+        cudaMemcpy(x + xbytes, rt.data(), sizeof(ResTile) * rt.size(), cudaMemcpyHostToDevice);
+    }
     if ((e = launch_init(h, c->dev, *d, 0)) != cudaSuccess ||
         (e = cudaDeviceSynchronize()) != cudaSuccess) {
         itlbm_case_destroy(c);
@@ -331,6 +360,13 @@ static int ensure_aux(itlbm_case *c) {
     return ITLBM_OK;
 }
 
+// Steps a call must ask for to take the resident kernel, and the most one launch runs.  Its launch
+// costs 20 us (tables, first loads) where a k_step launch costs 8, so it gains from about four steps on:
+// call and synchronisation on a 100^2 drop, k_step / resident, 4 steps: FP64 53 / 52, FP32 34 / 37, fold
+// 39 / 29 us; 6 steps: 76 / 64, 46 / 42, 56 / 34 us.
+constexpr int RES_MIN_STEPS = 6;
+constexpr int RES_MAX_STEPS = 4096;
+
 int itlbm_case_step(itlbm_case *c, int nsteps, int flags, void *stream) {
     if (!c || nsteps < 0) return fail(ITLBM_E_ARG, "bad argument");
     if (nsteps == 0) return ITLBM_OK;
@@ -342,7 +378,26 @@ int itlbm_case_step(itlbm_case *c, int nsteps, int flags, void *stream) {
     }
     cudaStream_t s = (cudaStream_t)stream;
     if (c->steps + nsteps > (long long)INT_MAX - 2) return fail(ITLBM_E_STATE, "step counter overflow");
-    for (int i = 0; i < nsteps; i++) {
+    int i0 = 0;
+    if (c->plan.shape >= 0 && nsteps >= RES_MIN_STEPS) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        // a captured launch would be replayed with the tags of its capture
+        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+            cudaGetLastError();
+        } else {
+            for (; i0 < nsteps; i0 += RES_MAX_STEPS) {
+                ResArgs a = c->res;
+                a.k0 = (int)(c->steps + i0);
+                a.nsteps = std::min(nsteps - i0, RES_MAX_STEPS);
+                a.aux_k = keep ? (int)(c->steps + nsteps - 1) : -1;
+                a.tag0 = (unsigned)a.k0;  // the step counter never returns to a value: neither do the tags
+                const cudaError_t e = res_launch(c->host.prec, c->plan.shape, a, c->plan.tiles, s);
+                if (e != cudaSuccess) return cuda_fail(e, "resident step kernel");
+            }
+            i0 = nsteps;
+        }
+    }
+    for (int i = i0; i < nsteps; i++) {
         const int k = (int)(c->steps + i);
         const int aux_k = (keep && i == nsteps - 1) ? k : -1;
         for (int sh = 0; sh < NSHAPE; sh++) {  // the tile shapes of one step touch disjoint nodes
@@ -363,7 +418,7 @@ int itlbm_case_sync(itlbm_case *c) {
     if (int rd = use_device(c->device)) return rd;
     cudaError_t e = cudaDeviceSynchronize();
     if (e != cudaSuccess) return cuda_fail(e, "synchronize");
-    return ITLBM_OK;
+    return waited(c);
 }
 
 long long itlbm_case_steps_done(const itlbm_case *c) { return c ? c->steps : -1; }
@@ -373,6 +428,7 @@ int itlbm_case_save(itlbm_case *c, const char *path) {
     if (int rd = use_device(c->device)) return rd;
     cudaError_t e = cudaDeviceSynchronize();  // steps may have gone to another stream
     if (e != cudaSuccess) return cuda_fail(e, "synchronize");
+    if (int r = waited(c)) return r;
     return snap_write(path, c->desc, c->steps, c->host, c->host.buf[c->steps & 1]);
 }
 
@@ -428,7 +484,7 @@ int itlbm_case_diag_drop(itlbm_case *c, int step, double x_ini, double y_ini, it
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return cuda_fail(e, "diagnostic copy");
     out->step = step;
-    return ITLBM_OK;
+    return waited(c);
 }
 
 // The same kernels as itlbm_case_diag_drop on a fixed device scratch; no allocation of any kind.
@@ -465,7 +521,7 @@ int itlbm_case_diag_drop_static(itlbm_case *c, int step, double x_ini, double y_
         (e = cudaStreamSynchronize(st)) != cudaSuccess)
         return cuda_fail(e, "diagnostic copy");
     out->step = step;
-    return ITLBM_OK;
+    return waited(c);
 }
 
 int itlbm_case_diag_strip(itlbm_case *c, int step, itlbm_strip_diag *out, void *stream) {
@@ -486,7 +542,7 @@ int itlbm_case_diag_strip(itlbm_case *c, int step, itlbm_strip_diag *out, void *
         (e = cudaStreamSynchronize(s)) != cudaSuccess)
         return cuda_fail(e, "diagnostic copy");
     out->step = step;
-    return ITLBM_OK;
+    return waited(c);
 }
 
 static int ensure_tmp(itlbm_case *c) {
@@ -512,7 +568,7 @@ int itlbm_case_read_pops(itlbm_case *c, int which, double *fR, double *fB) {
     if (e == cudaSuccess) e = launch_export(c->dev, c->host.nx, c->host.ny, cur, which, c->tmp, c->tmp + NV * n, 0);
     if (e == cudaSuccess) e = cudaMemcpy(fR, c->tmp, sizeof(double) * NV * n, cudaMemcpyDeviceToHost);
     if (e == cudaSuccess) e = cudaMemcpy(fB, c->tmp + NV * n, sizeof(double) * NV * n, cudaMemcpyDeviceToHost);
-    return e == cudaSuccess ? ITLBM_OK : cuda_fail(e, "read_pops");
+    return e == cudaSuccess ? waited(c) : cuda_fail(e, "read_pops");
 }
 
 int itlbm_case_write_pops(itlbm_case *c, const double *fR, const double *fB) {
@@ -560,7 +616,7 @@ static int read_fields_as(itlbm_case *c, int form, double *rho_R, double *rho_B,
         for (size_t p = 0; p < n; p++)
             for (int k = 0; k < 3; k++) force[3 * p + k] = a[k * n + p];
     }
-    return e == cudaSuccess ? ITLBM_OK : cuda_fail(e, "read_fields");
+    return e == cudaSuccess ? waited(c) : cuda_fail(e, "read_fields");
 }
 
 int itlbm_case_read_fields(itlbm_case *c, double *rho_R, double *rho_B, double *ux, double *uy,

@@ -1,0 +1,507 @@
+// itlbm_resident.cu -- many time steps in one launch, the state of every case held on chip.
+//
+// k_step (itlbm_step.cu) reads and writes the whole state in HBM every step, and a box of a few
+// hundred nodes a side cannot hide what that costs: on B200 one FP64 step of a 100 x 100 drop took
+// 11 us, of which the launch, the dependent loads of the tile's descriptors and the two round trips
+// for the node and halo loads are most.  Here a CTA keeps one tile of one case for all the steps of a
+// launch: its populations live in shared memory, and per step only what crosses a tile's edge goes
+// through L2, to the CTAs that hold the neighbouring tiles.  All CTAs are resident at once (a
+// cooperative launch), since they wait for one another.
+//
+// Step of a tile of w x h nodes, one node per thread (R in the fold):
+//   1. each thread takes its node's planes from shared memory, forms rho^N, and posts it when the
+//      node lies within the stencil's reach of the tile's edge;
+//   2. the halo's rho^N are taken from the tiles that own those nodes;
+//      (for class P the relaxation, which needs no gradient, comes before that wait);
+//   3. gradient, force, collision (itlbm_node.cuh), and the push of every plane to x + c_i in shared
+//      memory, whose planes have one ghost node on each side;
+//   4. the ghost values are posted, and the ones that enter this tile are taken from its neighbours.
+// The values go as 16-byte packs {values, tag} written and read whole (relaxed b128 accesses), so a
+// pack is its own flag: the reader polls the pack until its tag is that of the step, and no fence
+// and no second round trip is needed.  Packs are double-buffered by the parity of the step: a
+// neighbour posts step k + 2 only after it took what this tile posted at k + 1, which this tile did
+// after it had taken everything of step k.
+// Every wait is bounded: a wait that runs out sets *err and the CTA returns at the end of its step,
+// as do its neighbours in turn.
+//
+// The tile's shape is free (w h <= threads, see res_plan): a 100 x 100 box is 4 x 10 tiles of 25 x 10
+// nodes.  A node's arithmetic does not depend on the tile, so the results are those of k_step to the
+// bit.
+#include "itlbm_node.cuh"
+#include "itlbm_resident.h"
+
+#include <climits>
+
+namespace itlbm {
+
+namespace {
+
+constexpr int SPIN_LIMIT = 1 << 23;  // polls of one wait, each a trip to L2: some seconds
+
+// planes that leave a tile through a side (0 +x, 1 -x, 2 +y, 3 -y): the axis ones, then the two
+// diagonals
+template <bool FOLD>
+__device__ __forceinline__ constexpr int side_plane(int side, int d) {
+    constexpr int t19[20] = {1, 11, 13, 7, 9, 2, 12, 14, 8, 10, 3, 16, 18, 7, 10, 4, 15, 17, 8, 9};
+    constexpr int t9[12] = {1, 5, 7, 2, 6, 8, 3, 5, 8, 4, 6, 7};
+    return FOLD ? t9[side * 3 + d] : t19[side * 5 + d];
+}
+// in-plane velocity of plane d of a side: the axis, and for the last two d the diagonal's other part
+template <bool FOLD>
+__device__ __forceinline__ void side_dir(int side, int d, int &ex, int &ey) {
+    constexpr int NA = FOLD ? 1 : 3;
+    const int s = (side & 1) ? -1 : 1;
+    // side_plane: +x {.., (1,1), (1,-1)}; -x {.., (-1,-1), (-1,1)}; +y {.., (1,1), (-1,1)}; -y {.., (-1,-1), (1,-1)}
+    const int t = d < NA ? 0 : (d == NA ? s : -s);
+    ex = side < 2 ? s : t;
+    ey = side < 2 ? t : s;
+}
+
+__device__ __forceinline__ void st_pack(uint4 *p, unsigned long long lo, unsigned long long hi) {
+    asm volatile("{ .reg .b128 v; mov.b128 v, {%1, %2}; st.relaxed.gpu.global.b128 [%0], v; }" ::"l"(p), "l"(lo), "l"(hi)
+                 : "memory");
+}
+__device__ __forceinline__ void ld_pack(const uint4 *p, unsigned long long &lo, unsigned long long &hi) {
+    asm volatile("{ .reg .b128 v; ld.relaxed.gpu.global.b128 v, [%2]; mov.b128 {%0, %1}, v; }" : "=l"(lo), "=l"(hi) : "l"(p)
+                 : "memory");
+}
+__device__ __forceinline__ void st_pair(unsigned long long *p, unsigned long long v) {
+    asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_pair(const unsigned long long *p) {
+    unsigned long long v;
+    asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+    return v;
+}
+__device__ __forceinline__ unsigned long long pair_of(unsigned a, unsigned b) {
+    return (unsigned long long)a | ((unsigned long long)b << 32);
+}
+
+// first coordinate of tile t of n nodes cut into b tiles (res_tiling keeps the product in 32 bits)
+__device__ __forceinline__ int tile_begin(int t, int n, int b) { return (int)((unsigned)t * (unsigned)n / (unsigned)b); }
+
+// Of a CTA's tile: its case, its place and size, and what the loop needs of them.
+struct Geo {
+    const CaseDev *c;
+    int tipo, x0, y0, w, h;
+    int nring, npacks;  // halo nodes; packs that leave (and enter), with those that the corners leave out
+    int nsteps, cur0;   // steps of this launch, the buffer it starts from
+    int keep_step;      // the step whose force and gradient are kept
+    float rho0;
+    int tx[3], ty[3], begin_x[3], begin_y[3], size_x[3], size_y[3];  // the tile's column and row and the ones beside them
+};
+
+template <class S, bool FOLD, int NT, int R>
+__global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_resident(const __grid_constant__ ResArgs a) {
+    using C = ResCfg<S, FOLD, NT, R>;
+    constexpr int NP = C::NP, ND = C::ND, PS = C::PS, PK = C::PK;
+    constexpr bool F64 = std::is_same<S, double>::value;
+    using PhiPack = std::conditional_t<F64, uint4, unsigned long long>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    S *const pop = reinterpret_cast<S *>(smem_raw);             // [2 NP][PS], planes of (w + 2) x (h + 2)
+    S *const phi = pop + 2 * NP * PS;                           // (w + 4) x (h + 4)
+    unsigned *const rcv = reinterpret_cast<unsigned *>(phi + C::PHIN);  // packs that enter: source << 13 | element
+    unsigned *const hal = rcv + C::NPK;                         // halo nodes: source << 10 | element of phi
+    unsigned short *const snd = reinterpret_cast<unsigned short *>(hal + C::NRING);  // element of each pack that leaves
+    // F1 / F2: the ring-1 gradient and auxiliaries, in the planes' place between their load and the push
+    S *const ringg = pop, *const ringa = pop + 3 * PS;
+
+    // What is the same for all threads sits in shared memory and is read where it is used: kept in
+    // registers it would cost the 64-register forms spills, which a thousand threads per SM cannot
+    // hold in the cache that the shared memory leaves.
+    __shared__ Geo g;
+    const int tid = threadIdx.x;
+    {
+        const ResTile rt = a.tiles[blockIdx.x];
+        const CaseDev &c = a.cases[rt.case_id];
+        const int nsteps = min(a.nsteps, c.chunk_len - a.k0);
+        if (nsteps <= 0) return;
+        const int bx = rt.bx, by = rt.by, H = c.halo;
+        const int ty = rt.tile / bx, tx = rt.tile - ty * bx;
+        if (tid < 6) {  // the tile's column and row and the ones beside them
+            const bool col = tid < 3;
+            const int d = col ? tid : tid - 3, b = col ? bx : by, n = col ? c.nx : c.ny;
+            int t = (col ? tx : ty) + d - 1;
+            t += t < 0 ? b : (t == b ? -b : 0);
+            const int x = tile_begin(t, n, b);
+            (col ? g.tx : g.ty)[d] = t;
+            (col ? g.begin_x : g.begin_y)[d] = x;
+            (col ? g.size_x : g.size_y)[d] = tile_begin(t + 1, n, b) - x;
+        }
+        const int wm = (c.nx + bx - 1) / bx, hm = (c.ny + by - 1) / by;  // largest tile of the case
+        const int nxs = ND * hm, nitems = 2 * ND * (hm + wm);
+        __syncthreads();
+        const int w = g.size_x[1], h = g.size_y[1], PW = w + 2, PP = w + 4;
+        const int nring = 2 * H * (w + h + 2 * H);
+        if (tid == 0) {
+            g.c = &c;
+            g.tipo = c.tipo;
+            g.x0 = g.begin_x[1];
+            g.y0 = g.begin_y[1];
+            g.w = w;
+            g.h = h;
+            g.nring = nring;
+            g.npacks = nitems * PK;
+            g.nsteps = nsteps;
+            g.cur0 = (c.parity0 + a.k0) & 1;
+            g.rho0 = c.pf.rho0;
+            g.keep_step = c.aux == nullptr ? -1 : (c.aux_at_end ? c.chunk_len - 1 : a.aux_k) - a.k0;
+        }
+
+        // the packs of the exchange: index = side offset + d * length + position along the side, the
+        // same for every tile of the case
+        for (int j = tid; j < nitems; j += NT) {
+            const bool xs = j < 2 * nxs;
+            const int L = xs ? hm : wm, r = xs ? j : j - 2 * nxs, dl = r / L, pos = r - dl * L;
+            const int side = (xs ? 0 : 2) + (dl >= ND ? 1 : 0), d = dl >= ND ? dl - ND : dl;
+            const int plane = side_plane<FOLD>(side, d);
+            int ex, ey;
+            side_dir<FOLD>(side, d, ex, ey);
+            // leaving: source (lx, ly) in this tile; a diagonal that leaves through a corner goes by its x side
+            int lx = xs ? (ex > 0 ? w - 1 : 0) : pos, ly = xs ? pos : (ey > 0 ? h - 1 : 0);
+            bool ok = pos < (xs ? h : w) && (xs || (unsigned)(lx + ex) < (unsigned)w);
+            snd[j] = ok ? (unsigned short)(plane * PS + (ly + ey + 1) * PW + lx + ex + 1) : (unsigned short)0xFFFF;
+            // entering: destination (lx, ly) in this tile, from the tile beside it that holds (lx - ex, ly - ey)
+            lx = xs ? (ex > 0 ? 0 : w - 1) : pos;
+            ly = xs ? pos : (ey > 0 ? 0 : h - 1);
+            ok = pos < (xs ? h : w) && (xs || (unsigned)(lx - ex) < (unsigned)w);
+            unsigned v = 0xFFFFFFFFu;
+            if (ok) {
+                const int sx = lx - ex, sy = ly - ey;
+                const int ix = sx < 0 ? 0 : (sx >= w ? 2 : 1), iy = sy < 0 ? 0 : (sy >= h ? 2 : 1);
+                const int spos = xs ? (iy == 0 ? g.size_y[0] - 1 : (iy == 2 ? 0 : sy)) : sx;
+                v = ((unsigned)((rt.base + g.ty[iy] * bx + g.tx[ix]) * C::NPK + j - pos + spos) << 13) |
+                    (unsigned)(plane * PS + (ly + 1) * PW + lx + 1);
+            }
+            rcv[j] = v;
+        }
+        // the halo nodes of rho^N, row by row around the tile
+        for (int j = tid; j < nring; j += NT) {
+            const int B = w + 2 * H, nb = H * B;
+            int px, py;  // relative to the tile's first node
+            if (j < 2 * nb) {
+                const int q = j / B;
+                py = q < H ? q - H : h + q - H;
+                px = j - q * B - H;
+            } else {
+                const int r = j - 2 * nb, k = r & (2 * H - 1);
+                py = H == 1 ? r >> 1 : r >> 2;
+                px = k < H ? k - H : w + k - H;
+            }
+            const int ix = px < 0 ? 0 : (px >= w ? 2 : 1), iy = py < 0 ? 0 : (py >= h ? 2 : 1);
+            const int sx = px < 0 ? px + g.size_x[0] : (px >= w ? px - w : px);
+            const int sy = py < 0 ? py + g.size_y[0] : (py >= h ? py - h : py);
+            const int node = sy * g.size_x[ix] + sx;
+            hal[j] = ((unsigned)((rt.base + g.ty[iy] * bx + g.tx[ix]) * C::NODES + node) << 10) |
+                     (unsigned)((py + 2) * PP + px + 2);
+        }
+    }
+    __syncthreads();
+
+    // the thread's nodes: the element of a node in a plane (13 bits) and in phi (10 bits), whether it
+    // lies within the stencil's reach of the tile's edge, and whether it exists
+    unsigned me[R];
+    const CaseDev &c0 = *g.c;
+#pragma unroll
+    for (int r = 0; r < R; r++) {
+        const int t = tid + r * NT, w = g.w, h = g.h, H = c0.halo;
+        me[r] = 0;
+        if (t < w * h) {
+            const int ly = t / w, lx = t - ly * w;
+            const bool edge = lx < H || lx >= w - H || ly < H || ly >= h - H;
+            me[r] = 0x80000000u | (edge ? 0x40000000u : 0u) | (unsigned)((ly + 2) * (w + 4) + lx + 2) << 13 |
+                    (unsigned)((ly + 1) * (w + 2) + lx + 1);
+            const S *src = (const S *)c0.buf[g.cur0] + node_off(c0, g.x0 + lx, g.y0 + ly);
+#pragma unroll
+            for (int q = 0; q < 2 * NP; q++) pop[q * PS + (me[r] & 8191u)] = src[q * PLANE];
+        }
+    }
+    // the node's element in a state buffer
+    auto home = [&](int r) {
+        const int t = tid + r * NT, ly = t / g.w, lx = t - ly * g.w;
+        return node_off(*g.c, g.x0 + lx, g.y0 + ly);
+    };
+    // the buffer the launch does not end in: a site that is streamed unchanged waits there
+    auto spare = [&]() { return (S *)g.c->buf[(g.cur0 ^ (g.nsteps & 1)) ^ 1]; };
+    int bad = 0;
+    __syncthreads();
+
+    for (int s = 0; s < g.nsteps; s++) {
+        const unsigned tag = a.tag0 + (unsigned)s + 1u;
+        uint4 *const pk = a.packs + ((tag & 1u) ? (size_t)a.slots * (C::NPK * PK) : 0);
+        PhiPack *const ph = (PhiPack *)a.phis + ((tag & 1u) ? (size_t)a.slots * C::NODES : 0);
+
+        // ---- 1: the node's planes and rho^N ----------------------------------------------------
+        S f[R][NP], sa[R], sb[R];
+        double sbd[R];
+        Recolour<S, FOLD> rc[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            sa[r] = S(0);
+            sb[r] = S(0);
+            sbd[r] = 0.0;
+            if (me[r]) {
+                S va[NP], vb[NP];
+#pragma unroll
+                for (int i = 0; i < NP; i++) va[i] = pop[i * PS + (me[r] & 8191u)];
+#pragma unroll
+                for (int i = 0; i < NP; i++) vb[i] = pop[(NP + i) * PS + (me[r] & 8191u)];
+#pragma unroll
+                for (int i = 0; i < NP; i++) sa[r] = sa[r] + va[i];
+#pragma unroll
+                for (int i = 0; i < NP; i++) sb[r] = sb[r] + vb[i];
+                const S p = phase_of(sa[r], sb[r], g.rho0);
+                phi[me[r] >> 13 & 1023u] = p;
+                if (me[r] & 0x40000000u) {
+                    const unsigned o = blockIdx.x * C::NODES + tid + r * NT;
+                    if constexpr (F64) st_pack(ph + o, (unsigned long long)__double_as_longlong(p), tag);
+                    else st_pair(ph + o, pair_of(__float_as_uint(p), tag));
+                }
+                bool keep;  // a site that will be streamed unchanged (rho <= 1e-30)
+                if constexpr (F64) keep = !(sa[r] + sb[r] > 1.0e-30);
+                else keep = !(g.rho0 + sa[r] > 1.0e-30f);
+                if (keep) {
+                    S *tmp = spare() + home(r);
+#pragma unroll
+                    for (int i = 0; i < NP; i++) {
+                        tmp[i * PLANE] = va[i];
+                        tmp[(NP + i) * PLANE] = vb[i];
+                    }
+                }
+                if constexpr (!F64) {
+#pragma unroll
+                    for (int i = 0; i < NP; i++) sbd[r] += (double)vb[i];
+                }
+#pragma unroll
+                for (int i = 0; i < NP; i++) f[r][i] = F64 ? va[i] + vb[i] : va[i];
+                if (g.tipo < ITLBM_OP_F1) {  // class P: while the halo's rho^N are on their way
+                    CaseDev::F32Par pf{};
+                    if constexpr (!F64) pf = load_pf(*g.c);
+                    node_relax<false, S, FOLD>(*g.c, pf, f[r], sa[r], sb[r], S(0), S(0), S(0), rc[r]);
+                }
+            }
+        }
+
+        // ---- 2: the halo's rho^N ----------------------------------------------------------------
+        {
+            constexpr int MI = (C::NRING + NT - 1) / NT;
+            unsigned pend = 0, e[MI];
+#pragma unroll
+            for (int u = 0; u < MI; u++) {
+                e[u] = 0;
+                if (tid + u * NT < g.nring) {
+                    e[u] = hal[tid + u * NT];
+                    pend |= 1u << u;
+                }
+            }
+            int spins = 0;
+            while (pend) {
+                unsigned long long lo[MI], hi[MI];
+#pragma unroll
+                for (int u = 0; u < MI; u++)
+                    if (pend >> u & 1u) {
+                        if constexpr (F64) ld_pack(ph + (e[u] >> 10), lo[u], hi[u]);
+                        else {
+                            lo[u] = ld_pair(ph + (e[u] >> 10));
+                            hi[u] = lo[u] >> 32;
+                        }
+                    }
+#pragma unroll
+                for (int u = 0; u < MI; u++)
+                    if ((pend >> u & 1u) && (unsigned)hi[u] == tag) {
+                        if constexpr (F64) phi[e[u] & 1023u] = __longlong_as_double((long long)lo[u]);
+                        else phi[e[u] & 1023u] = __uint_as_float((unsigned)lo[u]);
+                        pend &= ~(1u << u);
+                    }
+                if (pend && ++spins > SPIN_LIMIT) {
+                    bad = 1;
+                    break;
+                }
+            }
+        }
+        __syncthreads();
+
+        // ---- 3: gradient, force, collision, push --------------------------------------------------
+        const CaseDev &c = *g.c;
+        const int tipo = g.tipo, PW = g.w + 2, PP = g.w + 4;
+        const bool force = tipo >= ITLBM_OP_F1, ring = tipo == ITLBM_OP_F1 || tipo == ITLBM_OP_F2;
+        if (ring) {
+            const int nq = PW * (g.h + 2), M = (65536 + PW - 1) / PW;  // q / PW by multiply and shift, exact for q < 65536 / PW
+            for (int q = tid; q < nq; q += NT) {
+                const int qy = (q * M) >> 16, qx = q - qy * PW;
+                const S *p = phi + (qy + 1) * PP + qx + 1;
+                ring_aux_node<S>(c, tipo, [&](int dx, int dy) { return p[dy * PP + dx]; }, ringg + q * 3, ringa + q * AUXS);
+            }
+            __syncthreads();
+        }
+        CaseDev::F32Par pf{};
+        if constexpr (!F64) pf = load_pf(c);
+        S gmx[R], gmy[R], gmz[R], Fx[R], Fy[R], Fz[R];
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            if (me[r]) {
+                const S *p = phi + (me[r] >> 13 & 1023u);
+                const S *q = ringa + (me[r] & 8191u) * AUXS;
+                node_force<S>(c, tipo, pf, [&](int dx, int dy) { return p[dy * PP + dx]; },
+                              [&](int dx, int dy) { return q + (dy * PW + dx) * AUXS; }, ringg + (me[r] & 8191u) * 3, gmx[r], gmy[r],
+                              gmz[r], Fx[r], Fy[r], Fz[r]);
+                if (force) node_relax<true, S, FOLD>(c, pf, f[r], sa[r], sb[r], Fx[r], Fy[r], Fz[r], rc[r]);
+            }
+        if (ring) __syncthreads();  // the push overwrites the auxiliaries
+#pragma unroll
+        for (int r = 0; r < R; r++)
+            if (me[r]) {
+                S *const at[3] = {pop + (me[r] & 8191u) - PW, pop + (me[r] & 8191u), pop + (me[r] & 8191u) + PW};
+                auto push = [&](auto Q, S v) {
+                    constexpr int q = decltype(Q)::value, i = q % NP;
+                    constexpr int ex = FOLD ? kx(i) : cx(i), ey = FOLD ? ky(i) : cy(i);
+                    at[ey + 1][q * PS + ex] = v;
+                };
+                if constexpr (F64) gradient_size(gmx[r], gmy[r], gmz[r], rc[r]);
+                if (!rc[r].skip) {
+                    if (force) node_finish<true, S, FOLD>(c, pf, f[r], sa[r], gmx[r], gmy[r], gmz[r], rc[r]);
+                    else node_finish<false, S, FOLD>(c, pf, f[r], sa[r], gmx[r], gmy[r], gmz[r], rc[r]);
+                    node_split<S, FOLD>(pf, f[r], sbd[r], rc[r], push);
+                } else {
+                    const S *tmp = spare() + home(r);
+                    sfor<0, 2 * NP>([&](auto Q) { push(Q, tmp[decltype(Q)::value * PLANE]); });
+                }
+                if (s == g.keep_step)
+                    keep_aux(c, g.x0 + (tid + r * NT) % g.w, g.y0 + (tid + r * NT) / g.w, Fx[r], Fy[r], Fz[r], gmx[r], gmy[r], gmz[r]);
+            }
+
+        __syncthreads();
+
+        // ---- 4: what crosses the tile's edges -----------------------------------------------------
+        {
+            constexpr int MI = (C::NPK * PK + NT - 1) / NT;
+            unsigned pend = 0, e[MI];
+#pragma unroll
+            for (int u = 0; u < MI; u++) {
+                const int j = tid + u * NT;
+                e[u] = j < g.npacks ? snd[j / PK] : 0xFFFFu;
+            }
+#pragma unroll
+            for (int u = 0; u < MI; u++) {
+                const int j = tid + u * NT;
+                if (e[u] == 0xFFFFu) continue;
+                uint4 *const o = pk + (size_t)(blockIdx.x * C::NPK) * PK + j;
+                if constexpr (F64) st_pack(o, (unsigned long long)__double_as_longlong(pop[e[u] + (j % PK) * NP * PS]), tag);
+                else st_pack(o, pair_of(__float_as_uint(pop[e[u]]), __float_as_uint(pop[e[u] + NP * PS])), tag);
+            }
+#pragma unroll
+            for (int u = 0; u < MI; u++) {
+                const int j = tid + u * NT;
+                e[u] = j < g.npacks ? rcv[j / PK] : 0xFFFFFFFFu;
+                if (e[u] != 0xFFFFFFFFu) pend |= 1u << u;
+            }
+            int spins = 0;
+            while (pend) {
+                unsigned long long lo[MI], hi[MI];
+#pragma unroll
+                for (int u = 0; u < MI; u++)
+                    if (pend >> u & 1u) ld_pack(pk + (size_t)(e[u] >> 13) * PK + (tid + u * NT) % PK, lo[u], hi[u]);
+#pragma unroll
+                for (int u = 0; u < MI; u++)
+                    if ((pend >> u & 1u) && (unsigned)hi[u] == tag) {
+                        S *const d = pop + (e[u] & 8191u);
+                        if constexpr (F64) d[((tid + u * NT) % PK) * NP * PS] = __longlong_as_double((long long)lo[u]);
+                        else {
+                            d[0] = __uint_as_float((unsigned)lo[u]);
+                            d[NP * PS] = __uint_as_float((unsigned)(lo[u] >> 32));
+                        }
+                        pend &= ~(1u << u);
+                    }
+                if (pend && ++spins > SPIN_LIMIT) {
+                    bad = 1;
+                    break;
+                }
+            }
+        }
+        if (__syncthreads_or(bad)) {
+            if (tid == 0) *a.err = 1;
+            return;
+        }
+    }
+
+    // the state at the top of the next step
+#pragma unroll
+    for (int r = 0; r < R; r++)
+        if (me[r]) {
+            S *dst = (S *)g.c->buf[g.cur0 ^ (g.nsteps & 1)] + home(r);
+#pragma unroll
+            for (int q = 0; q < 2 * NP; q++) dst[q * PLANE] = pop[q * PS + (me[r] & 8191u)];
+        }
+}
+
+template <class S, bool FOLD, int NT, int R>
+struct Entry {
+    using C = ResCfg<S, FOLD, NT, R>;
+    // resident CTAs per SM, asked once per device (the query also sets the shared-memory limit)
+    static int occupancy() {
+        int n = 0;
+        if (cudaFuncSetAttribute(k_resident<S, FOLD, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
+                cudaSuccess ||
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_resident<S, FOLD, NT, R>, NT, C::SMEM) != cudaSuccess) {
+            cudaGetLastError();
+            return 0;
+        }
+        return n;
+    }
+    static cudaError_t launch(const ResArgs &a, int grid, cudaStream_t st) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3((unsigned)grid);
+        cfg.blockDim = dim3(NT);
+        cfg.dynamicSmemBytes = C::SMEM;
+        cfg.stream = st;
+        cudaLaunchAttribute at{};
+        at.id = cudaLaunchAttributeCooperative;
+        at.val.cooperative = 1;
+        cfg.attrs = &at;
+        cfg.numAttrs = 1;
+        return cudaLaunchKernelEx(&cfg, k_resident<S, FOLD, NT, R>, a);
+    }
+};
+
+}  // namespace
+
+// Compiled twice, like itlbm_step.cu: FP64 without FMA contraction, and the FP32 forms.
+#ifdef ITLBM_STEP_F64
+#define RES_SWITCH(prec, shape, what)                                    \
+    switch (shape) {                                                     \
+        case RES_256: return Entry<double, false, 256, 1>::what;         \
+        case RES_128: return Entry<double, false, 128, 1>::what;         \
+        case RES_64: return Entry<double, false, 64, 1>::what;           \
+    }
+int res_occupancy_f64(int prec, int shape) {
+    RES_SWITCH(prec, shape, occupancy())
+    return 0;
+}
+cudaError_t res_launch_f64(int prec, int shape, const ResArgs &a, int grid, cudaStream_t st) {
+    RES_SWITCH(prec, shape, launch(a, grid, st))
+    return cudaErrorInvalidValue;
+}
+#else
+#define RES_SWITCH(prec, shape, what)                                                              \
+    if (prec == ITLBM_PREC_F32) switch (shape) {                                                   \
+        case RES_256: return Entry<float, false, 256, 1>::what;                                    \
+        case RES_128: return Entry<float, false, 128, 1>::what;                                    \
+        case RES_64: return Entry<float, false, 64, 1>::what;                                      \
+    }                                                                                              \
+    else switch (shape) {                                                                          \
+        case RES_256: return Entry<float, true, 256, 1>::what;                                     \
+        case RES_128: return Entry<float, true, 128, 1>::what;                                     \
+        case RES_64: return Entry<float, true, 64, 1>::what;                                       \
+        case RES_256x2: return Entry<float, true, 256, 2>::what;                                   \
+    }
+int res_occupancy_f32(int prec, int shape) {
+    RES_SWITCH(prec, shape, occupancy())
+    return 0;
+}
+cudaError_t res_launch_f32(int prec, int shape, const ResArgs &a, int grid, cudaStream_t st) {
+    RES_SWITCH(prec, shape, launch(a, grid, st))
+    return cudaErrorInvalidValue;
+}
+#endif
+
+}  // namespace itlbm

@@ -1,0 +1,89 @@
+// itlbm_resident.h -- the resident multi-step kernel (itlbm_resident.cu): its launch arguments, its
+// tile configurations and the rule that chooses one for a case.
+#pragma once
+
+#include "itlbm_internal.h"
+
+#include <vector>
+
+namespace itlbm {
+
+// Threads and nodes of a tile.
+enum { RES_256 = 0, RES_128 = 1, RES_64 = 2, RES_256x2 = 3, NRES = 4 };  // x2: two nodes per thread (fold)
+__host__ __device__ constexpr int res_threads(int shape) { return shape == RES_128 ? 128 : (shape == RES_64 ? 64 : 256); }
+__host__ __device__ constexpr int res_nodes(int shape) { return shape == RES_256x2 ? 512 : res_threads(shape); }
+// Largest w + h of a tile of that many nodes: 32 x 16, 32 x 8, 16 x 8, 8 x 8.
+__host__ __device__ constexpr int res_half_perimeter(int nodes) {
+    return nodes == 512 ? 48 : (nodes == 256 ? 40 : (nodes == 128 ? 24 : 16));
+}
+
+// One CTA of a launch: its case, the tile of that case (of bx x by), and the CTA of the case's tile 0.
+struct ResTile {
+    int case_id, tile, base;
+    unsigned short bx, by;
+};
+
+struct ResArgs {
+    const CaseDev *cases;
+    const ResTile *tiles;
+    uint4 *packs;      // exchange of populations: 2 parities x slots x NPK x PK packs
+    void *phis;        // exchange of rho^N: 2 parities x slots x NODES entries of 8 (FP32) or 16 bytes
+    int *err;          // set when a wait ran out
+    int slots;         // CTAs the exchange memory is laid out for (>= the grid)
+    unsigned tag0;     // tags of this launch are tag0 + 1 ... tag0 + nsteps, used by no earlier launch
+    int k0, nsteps, aux_k;
+};
+
+template <class S, bool FOLD, int NT, int R>
+struct ResCfg {
+    static constexpr int NP = FOLD ? NK : NV;          // planes per colour
+    static constexpr int ND = FOLD ? 3 : 5;            // of which leave through one side
+    static constexpr int NODES = NT * R;
+    static constexpr int WH = res_half_perimeter(NODES);
+    static constexpr int PS = NODES + 2 * WH + 4;      // largest (w + 2)(h + 2): stride of a plane
+    static constexpr int PHIN = NODES + 4 * WH + 16;   // largest (w + 4)(h + 4)
+    static constexpr int NPK = 2 * ND * WH;            // exchanged nodes x planes of one tile
+    static constexpr int NRING = 4 * WH + 16;          // halo nodes at reach 2
+    static constexpr int PK = sizeof(S) == 8 ? 2 : 1;  // packs per exchanged plane: both colours in FP32
+    static constexpr int SMEM = (int)sizeof(S) * (2 * NP * PS + PHIN) + 4 * (NPK + NRING) + 2 * NPK;
+    // CTAs per SM the registers are sized for: 64 registers in FP32 and 128 in FP64, as in k_step; twice
+    // that for the small tiles, whose boxes leave the SMs half empty anyway
+    static constexpr int MIN_CTAS = (sizeof(S) == 8 ? 512 : 1024) / NT / (NT < 256 ? 2 : 1);
+    static_assert(NP * PS <= 8192, "element of a pack in 13 bits");
+    static_assert(PHIN <= 1024, "element of phi in 10 bits");
+};
+
+int res_occupancy_f64(int prec, int shape);
+int res_occupancy_f32(int prec, int shape);
+cudaError_t res_launch_f64(int prec, int shape, const ResArgs &a, int grid, cudaStream_t st);
+cudaError_t res_launch_f32(int prec, int shape, const ResArgs &a, int grid, cudaStream_t st);
+inline int res_occupancy(int prec, int shape) {
+    return prec == ITLBM_PREC_F64 ? res_occupancy_f64(prec, shape) : res_occupancy_f32(prec, shape);
+}
+inline cudaError_t res_launch(int prec, int shape, const ResArgs &a, int grid, cudaStream_t st) {
+    return prec == ITLBM_PREC_F64 ? res_launch_f64(prec, shape, a, grid, st) : res_launch_f32(prec, shape, a, grid, st);
+}
+
+
+// How a case is held on chip: the tile configuration and the bx x by tiles, or shape < 0 when the box
+// has more tiles than the device holds at once (or sides below RES_MIN_SIDE).
+constexpr int RES_MIN_SIDE = 8;
+struct ResPlan {
+    int shape = -1, bx = 0, by = 0, tiles = 0;
+};
+// The fewest tiles of configuration `shape` that cover an nx x ny box (0 when none do).
+int res_tiling(int nx, int ny, int shape, int &bx, int &by);
+// CTAs of configuration `shape` the current device holds at once (0: no cooperative launch).
+int res_capacity(int prec, int shape);
+ResPlan res_plan_single(int prec, int nx, int ny);  // one case alone on the device
+ResPlan res_plan_batch(int prec, int nx, int ny);   // one of many cases that share it
+void res_tiles(const ResPlan &p, int case_id, int base, std::vector<ResTile> &out);
+// Bytes of exchange memory for `slots` CTAs, and its binding in a block of that many bytes.
+size_t res_exchange_bytes(int prec, int shape, int slots);
+void res_exchange_bind(ResArgs &a, void *base, int prec, int shape, int slots);
+// A word the resident kernel sets when a wait runs out, in pinned host memory the device writes
+// (process-wide pool; nullptr when it cannot be had), and its return.
+int *res_flag_get();
+void res_flag_put(int *f);
+
+}  // namespace itlbm

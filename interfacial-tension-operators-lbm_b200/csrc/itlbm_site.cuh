@@ -1,13 +1,13 @@
 // itlbm_site.cuh -- per-site device physics of the colour-gradient step.
 //
 // Two forms of the same site update:
-//   * collide_f64: the populations f_R, f_B in FP64, with the reference's arithmetic in the
+//   * relax_f64, finish_f64: the populations f_R, f_B in FP64, with the reference's arithmetic in the
 //     reference's operation order (colisao_comum, Operadores_tensao.cpp:340-373, and the library
 //     functions it calls).  Velocity components equal to zero are skipped in the dot products; with
 //     round-to-nearest that changes no finite result (adding a signed zero to a non-zero partial sum
 //     is exact), and the paired directions c_i, -c_i share one division because negation commutes
 //     with rounding.
-//   * collide_f32: FP32 storage of e_i = f_i - w_i rho0 (the deviation of the total population) and
+//   * relax_f32, finish_f32: FP32 storage of e_i = f_i - w_i rho0 (the deviation of the total population) and
 //     d_i = f_R,i - f_B,i (the colour difference).  Both are linear in (f_R, f_B), so streaming is
 //     unchanged; rho^N = sum d_i / rho, and the BGK update is applied to the deviation so that the
 //     pressure keeps FP32 relative precision on rho - rho0 instead of on rho.
@@ -49,24 +49,24 @@ __device__ __forceinline__ double guo_source_f64(double factor, double Fx, doubl
 
 // Class-P perturbation (perturbacao, Operadores_tensao.cpp:116-133):
 //   f_i += A |g| (w_i (c_i.g)^2 / |g|^2 - B_i), skipped when |g|^2 <= 1e-60 or A == 0.
-// The 9 direction pairs share (c_i.g)^2; c_i.g is summed in the reference's order.
-__device__ __forceinline__ void perturb_f64(double (&f)[NV], double gmx, double gmy, double gmz,
-                                            double A, double B0, double B1, double B2) {
-    const double mod2 = gmx * gmx + gmy * gmy + gmz * gmz;
-    if (mod2 <= 1.0e-60 || A == 0.0) return;
-    const double amod = A * sqrt(mod2);
+// The 9 direction pairs share (c_i.g)^2; c_i.g is summed in the reference's order.  mod = |g|; by_mod2
+// divides by |g|^2.
+template <class DIV>
+__device__ __forceinline__ void perturb_f64(double (&f)[NV], double gmx, double gmy, double gmz, double mod,
+                                            double A, double B0, double B1, double B2, DIV by_mod2) {
+    const double amod = A * mod;
     const double q0 = 0.0;
-    const double qx = ((wgt<double>(1) * gmx) * gmx) / mod2;
-    const double qy = ((wgt<double>(3) * gmy) * gmy) / mod2;
-    const double qz = ((wgt<double>(5) * gmz) * gmz) / mod2;
+    const double qx = by_mod2((wgt<double>(1) * gmx) * gmx);
+    const double qy = by_mod2((wgt<double>(3) * gmy) * gmy);
+    const double qz = by_mod2((wgt<double>(5) * gmz) * gmz);
     const double s7 = gmx + gmy, s9 = gmx - gmy, s11 = gmx + gmz, s13 = gmx - gmz;
     const double s16 = gmy + gmz, s17 = -gmy + gmz;
-    const double d7 = ((wgt<double>(7) * s7) * s7) / mod2;
-    const double d9 = ((wgt<double>(9) * s9) * s9) / mod2;
-    const double d11 = ((wgt<double>(11) * s11) * s11) / mod2;
-    const double d13 = ((wgt<double>(13) * s13) * s13) / mod2;
-    const double d16 = ((wgt<double>(16) * s16) * s16) / mod2;
-    const double d17 = ((wgt<double>(17) * s17) * s17) / mod2;
+    const double d7 = by_mod2((wgt<double>(7) * s7) * s7);
+    const double d9 = by_mod2((wgt<double>(9) * s9) * s9);
+    const double d11 = by_mod2((wgt<double>(11) * s11) * s11);
+    const double d13 = by_mod2((wgt<double>(13) * s13) * s13);
+    const double d16 = by_mod2((wgt<double>(16) * s16) * s16);
+    const double d17 = by_mod2((wgt<double>(17) * s17) * s17);
     const double Q[NV] = {q0, qx,  qx,  qy,  qy,  qz,  qz,  d7,  d7, d9,
                           d9, d11, d11, d13, d13, d16, d16, d17, d17};
     sfor<0, NV>([&](auto I) {
@@ -83,9 +83,20 @@ __device__ __forceinline__ void perturb_f64(double (&f)[NV], double gmx, double 
 struct Recolour64 {
     double cR, cB, frho;   // frho = (beta c_R c_B)... times rho: t_i = (frho_w_i) cos_i
     double fator, rho;
+    double mod2, mod;      // |g|^2 and |g| (gradient_size)
     double k[9];           // cos(phi) of the directions 1, 3, 5, 7, 9, 11, 13, 16, 17
     bool skip;             // rho <= 1e-30: the reference leaves the site unchanged
 };
+// The collision comes in two parts: relax_* (moments, equilibrium, Guo source, BGK), which for class P
+// needs nothing but the node's own populations, and finish_* (perturbation and recolouring), which
+// needs the colour gradient.
+
+// |g|^2 and |g|.  Taken as soon as the gradient is known: k_step takes it before relax_f64, whose
+// arithmetic hides the root (after it, the FP64 step of a 2048^2 class-P drop took 1.2 % longer).
+__device__ __forceinline__ void gradient_size(double gmx, double gmy, double gmz, Recolour64 &rc) {
+    rc.mod2 = gmx * gmx + gmy * gmy + gmz * gmz;
+    rc.mod = sqrt(rc.mod2);
+}
 
 // cos(phi_i) for i = 0..18 from the 9 independent values (pairs i, i+1 are opposite directions)
 __device__ __forceinline__ double cos_of(const Recolour64 &r, int i) {
@@ -123,23 +134,23 @@ __device__ __forceinline__ void split64(const Recolour64 &r, double fi, double &
 // LBM_functions.cpp:1582-1590, index order).  gm is the mediator momentum (= -grad rho^N), F the force
 // (class F only).  On exit f is the post-BGK total and r holds the recolouring split.
 template <bool FORCE>
-__device__ __forceinline__ void collide_f64(double (&f)[NV], double rho_R, double rho_B, double gmx,
-                                            double gmy, double gmz, double Fx, double Fy, double Fz,
-                                            const CaseDev &c, Recolour64 &rc) {
+__device__ __forceinline__ void relax_f64(double (&f)[NV], double rho_R, double rho_B, double Fx, double Fy, double Fz,
+                                          const CaseDev &c, Recolour64 &rc) {
     const double rho = rho_R + rho_B;
     rc.skip = !(rho > 1.0e-30);  // Operadores_tensao.cpp:347 (rho <= 1e-30: return)
     if (rc.skip) return;
-    const double conc_R = rho_R / rho;
-    const double conc_B = 1.0 - conc_R;
-    const double mod = sqrt(gmx * gmx + gmy * gmy + gmz * gmz);
-
     // coll_BGK (Collision_operators.cpp:8-46) with acc = F / rho (class F) or 0 (class P)
     double ax = 0.0, ay = 0.0, az = 0.0;
     if constexpr (FORCE) {
+        rc.cR = rho_R / rho;
         ax = Fx / rho;
         ay = Fy / rho;
         az = Fz / rho;
+    } else {
+        rc.cR = rho_R / rho;
     }
+    rc.cB = 1.0 - rc.cR;
+    rc.rho = rho;
     // calcula (LBM_functions.cpp:1100-1171)
     double r = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
     sfor<0, NV>([&](auto I) {
@@ -185,26 +196,38 @@ __device__ __forceinline__ void collide_f64(double (&f)[NV], double rho_R, doubl
         }
     });
 
+}
+template <bool FORCE, class D2, class DA, class DB>
+__device__ __forceinline__ void finish_f64_by(double (&f)[NV], double gmx, double gmy, double gmz, double mod2, double mod,
+                                              const CaseDev &c, Recolour64 &rc, D2 by_mod2, DA by_den1, DB by_den2) {
     // perturbacao (Operadores_tensao.cpp:116-133), class P only; the sign of g is irrelevant
-    if constexpr (!FORCE) perturb_f64(f, gmx, gmy, gmz, c.A, c.B0, c.B1, c.B2);
-
+    if constexpr (!FORCE)
+        if (!(mod2 <= 1.0e-60 || c.A == 0.0)) perturb_f64(f, gmx, gmy, gmz, mod, c.A, c.B0, c.B1, c.B2, by_mod2);
     // recolloring (LBM_functions.cpp:1713-1746) with grad = gm, |c_i| = 1 or sqrt(2)
-    rc.cR = conc_R;
-    rc.cB = conc_B;
-    rc.rho = rho;
-    rc.fator = (c.beta * conc_R) * conc_B;
+    rc.k[0] = by_den1(gmx);
+    rc.k[1] = by_den1(gmy);
+    rc.k[2] = by_den1(gmz);
+    rc.k[3] = by_den2(gmx + gmy);
+    rc.k[4] = by_den2(gmx - gmy);
+    rc.k[5] = by_den2(gmx + gmz);
+    rc.k[6] = by_den2(gmx - gmz);
+    rc.k[7] = by_den2(gmy + gmz);
+    rc.k[8] = by_den2(-gmy + gmz);
+}
+template <bool FORCE>
+__device__ __forceinline__ void finish_f64(double (&f)[NV], double gmx, double gmy, double gmz, const CaseDev &c,
+                                           Recolour64 &rc) {
+    const double mod2 = rc.mod2, mod = rc.mod;
+    rc.fator = (c.beta * rc.cR) * rc.cB;
+    if (mod == 0.0) {  // no gradient: neither perturbation nor recolouring
+#pragma unroll
+        for (int m = 0; m < 9; m++) rc.k[m] = 0.0;
+        return;
+    }
     const double den1 = mod * 1.0;
     const double den2 = mod * sqrt(2.0);
-    const bool nz = (mod != 0.0);
-    rc.k[0] = nz ? gmx / den1 : 0.0;
-    rc.k[1] = nz ? gmy / den1 : 0.0;
-    rc.k[2] = nz ? gmz / den1 : 0.0;
-    rc.k[3] = nz ? (gmx + gmy) / den2 : 0.0;
-    rc.k[4] = nz ? (gmx - gmy) / den2 : 0.0;
-    rc.k[5] = nz ? (gmx + gmz) / den2 : 0.0;
-    rc.k[6] = nz ? (gmx - gmz) / den2 : 0.0;
-    rc.k[7] = nz ? (gmy + gmz) / den2 : 0.0;
-    rc.k[8] = nz ? (-gmy + gmz) / den2 : 0.0;
+    finish_f64_by<FORCE>(f, gmx, gmy, gmz, mod2, mod, c, rc, [=](double a) { return a / mod2; },
+                         [=](double a) { return a / den1; }, [=](double a) { return a / den2; });
 }
 
 // The whole site update on arrays, for the per-site seam entry points.
@@ -220,21 +243,46 @@ __device__ __forceinline__ void colisao_site_f64(double (&fR)[NV], double (&fB)[
 #pragma unroll
     for (int i = 0; i < NV; i++) f[i] = fR[i] + fB[i];
     Recolour64 rc;
-    collide_f64<FORCE>(f, sa, sb, gmx, gmy, gmz, Fx, Fy, Fz, c, rc);
+    relax_f64<FORCE>(f, sa, sb, Fx, Fy, Fz, c, rc);
     if (rc.skip) return;
+    gradient_size(gmx, gmy, gmz, rc);
+    finish_f64<FORCE>(f, gmx, gmy, gmz, c, rc);
     sfor<0, NV>([&](auto I) {
         constexpr int i = decltype(I)::value;
         split64<i>(rc, f[i], fR[i], fB[i]);
     });
 }
 
-// The shift s of a direction (or class) with x velocity ex: w (s0 + 3 c.J0 + 4.5 (c.J0)(c.U0)), the
-// equilibrium at rho0 and U0 = (u0x, 0) (CaseDev).
+// The shift of a direction (or class) with x velocity ex is s = w S, with S = s0 + 3 c.J0 +
+// 4.5 (c.J0)(c.U0) the equilibrium factor at rho0 and U0 = (u0x, 0) (CaseDev).
 template <int ex>
-__device__ __forceinline__ float shift_of(const CaseDev::F32Par &p, float w) {
-    if constexpr (ex == 0) return w * p.s0;
-    else if constexpr (ex > 0) return w * (p.sx + p.j3);
-    else return w * (p.sx - p.j3);
+__device__ __forceinline__ float shift_of(const CaseDev::F32Par &p) {
+    if constexpr (ex == 0) return p.s0;
+    else if constexpr (ex > 0) return p.sx + p.j3;
+    else return p.sx - p.j3;
+}
+
+// FP32 arithmetic whose rounding the compiler would choose by the code around it (which product of a
+// sum goes into the multiply-add, whether a reciprocal of a square root becomes one instruction): fixed
+// here, so that every kernel that inlines the collision rounds it the same way.
+__device__ __forceinline__ float sqrt_fast(float x) {
+    float r;
+    asm("sqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rsqrt_fast(float x) {
+    float r;
+    asm("rsqrt.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+__device__ __forceinline__ float rcp_fast(float x) {
+    float r;
+    asm("rcp.approx.f32 %0, %1;" : "=f"(r) : "f"(x));
+    return r;
+}
+// 2 beta c_R c_B rho = beta (1 - phi^2) rho / 2
+__device__ __forceinline__ float recolour_amp(float beta, float phi, float rho) {
+    return 0.5f * beta * __fmaf_rn(-phi, phi, 1.0f) * rho;
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -268,31 +316,31 @@ __device__ __forceinline__ T cdotp(T a, T b, T c3) {  // c_i . (a, b, c3), non-z
 // cos(phi_i) = (c_i . g) / (|c_i| |g|); k1 and k2 fold fat2 w_i / (|c_i| |g|) of the two speeds.
 // d_0 is the complement D - sum_{i>=1} d_i, formed by the step kernel with FP64 sums.
 struct Recolour32 {
-    float phi, k1, k2, gx, gy, gz;
+    float phi, rho, k1, k2, gx, gy, gz;
     bool skip;
 };
 
-// d_i and d_{i+1} of the pair (i, i + 1), i odd, from the post-collision e_i, e_{i+1} and the shifts
-// s_i, s_{i+1}.
+// d_i and d_{i+1} of the pair (i, i + 1), i odd, from the post-collision e_i, e_{i+1} and the shift
+// factors S_i, S_{i+1} (s = w S).
 template <int i>
-__device__ __forceinline__ void split32_pair(const Recolour32 &r, float ei, float ej, float si, float sj,
+__device__ __forceinline__ void split32_pair(const Recolour32 &r, float ei, float ej, float Si, float Sj,
                                              float &di, float &dj) {
     const float K = cdotp<i>(r.gx, r.gy, r.gz) * (cc(i) == 1 ? r.k1 : r.k2);
-    di = fmaf(r.phi, si + ei, -K);
-    dj = fmaf(r.phi, sj + ej, K);
+    di = fmaf(r.phi, __fmaf_rn(wgt<float>(i), Si, ei), -K);
+    dj = fmaf(r.phi, __fmaf_rn(wgt<float>(i), Sj, ej), K);
 }
 
 // e_i = f_i - s_i in, post-collision e_i out; drho = sum e_i, D = sum d_i = rho_R - rho_B.
 template <bool FORCE>
-__device__ __forceinline__ void collide_f32(float (&e)[NV], float drho, float D, float gmx,
-                                            float gmy, float gmz, float Fx, float Fy, float Fz,
-                                            const CaseDev::F32Par &p, Recolour32 &rc) {
+__device__ __forceinline__ void relax_f32(float (&e)[NV], float drho, float D, float Fx, float Fy, float Fz,
+                                          const CaseDev::F32Par &p, Recolour32 &rc) {
     const float rho0 = p.rho0;
     const float rho = rho0 + drho;
     rc.skip = !(rho > 1.0e-30f);
     if (rc.skip) return;
     const float inv_rho = 1.0f / rho;
-    const float phi = D * inv_rho;  // rho^N = (rho_R - rho_B) / rho
+    rc.phi = D * inv_rho;  // rho^N = (rho_R - rho_B) / rho
+    rc.rho = rho;
     float ax = 0.f, ay = 0.f, az = 0.f;
     if constexpr (FORCE) {
         ax = Fx * inv_rho;
@@ -344,8 +392,12 @@ __device__ __forceinline__ void collide_f32(float (&e)[NV], float drho, float D,
         e[i] = ei;
         e[i + 1] = ej;
     });
-    const float mod2 = gmx * gmx + gmy * gmy + gmz * gmz;
-    const float mod = sqrtf(mod2);
+}
+template <bool FORCE>
+__device__ __forceinline__ void finish_f32(float (&e)[NV], float drho, float gmx, float gmy, float gmz,
+                                           const CaseDev::F32Par &p, Recolour32 &rc) {
+    const float mod2 = __fmaf_rn(gmz, gmz, __fmaf_rn(gmx, gmx, __fmul_rn(gmy, gmy)));
+    const float mod = sqrt_fast(mod2);
     if constexpr (!FORCE) {
         // class P: f_i += A |g| (w_i (c_i.g)^2 / |g|^2 - B_i), the same for both of a pair
         const float A = p.A;
@@ -371,9 +423,8 @@ __device__ __forceinline__ void collide_f32(float (&e)[NV], float drho, float D,
         float s2 = (e[9] + e[10]) + (e[11] + e[12]), s3 = (e[13] + e[14]) + (e[15] + e[16]);
         e[0] = drho - (((s0 + s1) + (s2 + s3)) + (e[17] + e[18]));
     }
-    const float fat2 = 0.5f * p.beta * (1.0f - phi * phi) * rho;
-    const float inv_mod = mod > 0.0f ? 1.0f / mod : 0.0f;
-    rc.phi = phi;
+    const float fat2 = recolour_amp(p.beta, rc.phi, rc.rho);
+    const float inv_mod = mod > 0.0f ? rsqrt_fast(mod2) : 0.0f;
     rc.k1 = fat2 * wgt<float>(1) * inv_mod;
     rc.k2 = fat2 * wgt<float>(7) * 0.70710678118654752f * inv_mod;
     rc.gx = gmx;
@@ -400,31 +451,32 @@ __device__ __forceinline__ T kdot(T a, T b) {  // e_K . (a, b)
 }
 
 struct RecolourFold {
-    float phi, k1, k2, gx, gy;
+    float phi, rho, k1, k2, gx, gy;
     bool skip;
 };
 
 // d_K and d_{K+1} of the class pair (K, K + 1), K odd, from the post-collision e_K, e_{K+1} and the
-// class shifts s_K, s_{K+1}.
+// class shift factors S_K, S_{K+1}.
 template <int K>
-__device__ __forceinline__ void split_fold_pair(const RecolourFold &r, float eK, float eJ, float sK, float sJ,
+__device__ __forceinline__ void split_fold_pair(const RecolourFold &r, float eK, float eJ, float SK, float SJ,
                                                 float &dK, float &dJ) {
     const float A = kdot<K>(r.gx, r.gy) * (kk(K) == 1 ? r.k1 : r.k2);
-    dK = fmaf(r.phi, sK + eK, -A);
-    dJ = fmaf(r.phi, sJ + eJ, A);
+    dK = fmaf(r.phi, __fmaf_rn(wk<float>(K), SK, eK), -A);
+    dJ = fmaf(r.phi, __fmaf_rn(wk<float>(K), SJ, eJ), A);
 }
 
 // e_K = F_K - s_K of the nine classes in (s_K the class sum of the shifts s_i), post-collision out;
-// drho = sum e_K, D = sum d_K.  The equilibrium is formed from the deviations as in collide_f32.
+// drho = sum e_K, D = sum d_K.  The equilibrium is formed from the deviations as in relax_f32.
 template <bool FORCE>
-__device__ __forceinline__ void collide_fold(float (&e)[NK], float drho, float D, float gmx, float gmy,
-                                             float Fx, float Fy, const CaseDev::F32Par &p, RecolourFold &rc) {
+__device__ __forceinline__ void relax_fold(float (&e)[NK], float drho, float D, float Fx, float Fy,
+                                           const CaseDev::F32Par &p, RecolourFold &rc) {
     const float rho0 = p.rho0;
     const float rho = rho0 + drho;
     rc.skip = !(rho > 1.0e-30f);
     if (rc.skip) return;
     const float inv_rho = 1.0f / rho;
-    const float phi = D * inv_rho;
+    rc.phi = D * inv_rho;
+    rc.rho = rho;
     float ax = 0.f, ay = 0.f;
     if constexpr (FORCE) {
         ax = Fx * inv_rho;
@@ -468,8 +520,12 @@ __device__ __forceinline__ void collide_fold(float (&e)[NK], float drho, float D
         e[K] = eK;
         e[K + 1] = eJ;
     });
-    const float mod2 = gmx * gmx + gmy * gmy;
-    const float mod = sqrtf(mod2);
+}
+template <bool FORCE>
+__device__ __forceinline__ void finish_fold(float (&e)[NK], float drho, float gmx, float gmy,
+                                            const CaseDev::F32Par &p, RecolourFold &rc) {
+    const float mod2 = __fmaf_rn(gmx, gmx, __fmul_rn(gmy, gmy));
+    const float mod = sqrt_fast(mod2);
     if constexpr (!FORCE) {
         const float A = p.A;
         if (!(mod2 <= 1.0e-30f || A == 0.0f)) {
@@ -487,9 +543,8 @@ __device__ __forceinline__ void collide_fold(float (&e)[NK], float drho, float D
         }
     }
     e[0] = drho - (((e[1] + e[2]) + (e[3] + e[4])) + ((e[5] + e[6]) + (e[7] + e[8])));
-    const float fat2 = 0.5f * p.beta * (1.0f - phi * phi) * rho;
-    const float inv_mod = mod > 0.0f ? 1.0f / mod : 0.0f;
-    rc.phi = phi;
+    const float fat2 = recolour_amp(p.beta, rc.phi, rc.rho);
+    const float inv_mod = mod > 0.0f ? rcp_fast(mod) : 0.0f;
     rc.k1 = fat2 * ((1.0f + 0.70710678118654752f) / 18.0f) * inv_mod;
     rc.k2 = fat2 * (0.70710678118654752f / 36.0f) * inv_mod;
     rc.gx = gmx;

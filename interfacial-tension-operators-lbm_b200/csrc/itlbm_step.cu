@@ -18,7 +18,7 @@
 // re-read from L2, where the neighbouring tiles keep them -- then evaluates the mediator gradient,
 // the force of class F on a ring-1 region of auxiliary fields, and collides.  No mediator
 // populations or force fields ever reach HBM.
-#include "itlbm_site.cuh"
+#include "itlbm_node.cuh"
 
 #include <climits>
 
@@ -86,11 +86,6 @@ __device__ __forceinline__ int wrap_near(int a, int n) {
     return r;
 }
 
-// Stride of the per-node auxiliary values in shared memory: 7, odd, so that the 32 lanes reading one
-// component of consecutive nodes hit distinct banks (a stride of 6 words, or 12 for doubles, puts two
-// lanes on each bank).
-constexpr int AUXS = 7;
-
 // Shared memory of a W x Hh tile.
 template <class S, int W, int Hh>
 struct SmemT {
@@ -100,15 +95,6 @@ struct SmemT {
     S g[QY][QX][3];       // ring-1 gradient (F1, F2)
     S aux[QY][QX][AUXS];  // ring-1 normal (F1) or stress (F2), 6 values at an odd stride
 };
-
-// rho^N from the two colour sums.  FP64: (rho_R - rho_B) / (rho_R + rho_B), Imm_OPS.cpp:255-258.
-// FP32: the sums are sum e_i (rho - rho0) and sum d_i (rho_R - rho_B).
-__device__ __forceinline__ double phase_of(double rR, double rB, float) {
-    return (rR - rB) / (rR + rB);
-}
-__device__ __forceinline__ float phase_of(float drho, float D, float rho0) {
-    return D / (rho0 + drho);
-}
 
 // ring position r -> staged-tile coordinates (px, py) for a halo of H (1 or 2) around the W x Hh
 // interior; consecutive r run along x in the top and bottom bands, so loads of consecutive r
@@ -236,23 +222,8 @@ __device__ __forceinline__ void step_tile(const CaseDev &c, int tile, int k, int
             const int qx = q % QX, qy = q / QX;
             const int gx = x0 - 1 + qx, gy = y0 - 1 + qy;
             if (gx < xe + 1 && gy < ye + 1) {
-                S g0, g1, g2;
-                if constexpr (std::is_same<S, float>::value) {
-                    // FP32 (both storage forms): the in-plane class forms, g_z = 0 on the slab
-                    mediator_grad_fold([&](int dx, int dy) { return sm.phi[qy + 1 + dy][qx + 1 + dx]; }, g0, g1);
-                    g0 = -g0;  // the isotropic gradient
-                    g1 = -g1;
-                    g2 = 0.f;
-                    if (tipo == ITLBM_OP_F1) aux_normal_plane(g0, g1, sm.aux[qy][qx]);
-                    else aux_stress_plane(g0, g1, c.pf.sigma, sm.aux[qy][qx]);
-                } else {
-                    iso_grad(sm.phi, qx + 1, qy + 1, g0, g1, g2);
-                    if (tipo == ITLBM_OP_F1) aux_normal(g0, g1, g2, sm.aux[qy][qx]);
-                    else aux_stress(g0, g1, g2, (S)c.sigma, sm.aux[qy][qx]);
-                }
-                sm.g[qy][qx][0] = g0;
-                sm.g[qy][qx][1] = g1;
-                sm.g[qy][qx][2] = g2;
+                ring_aux_node(c, tipo, [&](int dx, int dy) { return sm.phi[qy + 1 + dy][qx + 1 + dx]; },
+                              sm.g[qy][qx], sm.aux[qy][qx]);
             }
         }
         __syncthreads();
@@ -266,48 +237,10 @@ __device__ __forceinline__ void step_tile(const CaseDev &c, int tile, int k, int
         CaseDev::F32Par pf{};  // FP32: the case's parameters in float
         if constexpr (std::is_same<S, float>::value) pf = load_pf(c);
         const int px = lx + HMAX, py = lyj + HMAX;
-        S gmx, gmy, gmz;
+        S gmx, gmy, gmz, Fx, Fy, Fz;
         auto phi_at = [&](int dx, int dy) { return sm.phi[py + dy][px + dx]; };
-        if constexpr (std::is_same<S, float>::value) {
-            mediator_grad_fold(phi_at, gmx, gmy);  // FP32: class form, g_z = 0 on the slab
-            gmz = S(0);
-        } else mediator_grad(sm.phi, px, py, gmx, gmy, gmz);
-        S Fx = S(0), Fy = S(0), Fz = S(0);
-        const bool force = tipo >= ITLBM_OP_F1;
-        if (tipo == ITLBM_OP_F1) {
-            const int qx = lx + 1, qy = lyj + 1;
-            S kappa;
-            if constexpr (std::is_same<S, float>::value)
-                kappa = curvature_plane([&](int dx, int dy) { return sm.aux[qy + dy][qx + dx]; });
-            else
-                kappa = curvature<S, AUXS>(sm.aux, qx, qy);
-            S sig;
-            if constexpr (std::is_same<S, float>::value) sig = pf.sigma;
-            else sig = c.sigma;
-            const S hs = (S(0.5) * sig) * kappa;
-            Fx = hs * sm.g[qy][qx][0];
-            Fy = hs * sm.g[qy][qx][1];
-            Fz = hs * sm.g[qy][qx][2];
-        } else if (tipo == ITLBM_OP_F2) {
-            if constexpr (std::is_same<S, float>::value)
-                stress_div_plane([&](int dx, int dy) { return sm.aux[lyj + 1 + dy][lx + 1 + dx]; }, Fx, Fy);
-            else
-                stress_div<S, AUXS>(sm.aux, lx + 1, lyj + 1, Fx, Fy, Fz);
-        } else if (tipo == ITLBM_OP_F3) {
-            S g0, g1, g2, mu;
-            if constexpr (std::is_same<S, float>::value) {
-                g0 = -gmx;  // the isotropic gradient is the exact negative of the mediator momentum
-                g1 = -gmy;
-                g2 = -gmz;
-                mu = chem_pot_fold(phi_at, pf.kf, pf.bf);
-            } else {
-                iso_grad(sm.phi, px, py, g0, g1, g2);
-                mu = chem_pot(sm.phi, px, py, (S)c.kf, (S)c.bf);
-            }
-            Fx = mu * g0;
-            Fy = mu * g1;
-            Fz = mu * g2;
-        }
+        auto aux_at = [&](int dx, int dy) { return sm.aux[lyj + 1 + dy][lx + 1 + dx]; };
+        node_force<S>(c, tipo, pf, phi_at, aux_at, sm.g[lyj + 1][lx + 1], gmx, gmy, gmz, Fx, Fy, Fz);
         // the destination node x + c_i (periodic) of D3Q19 direction i, or of class i of the fold
         const int xp = (x + 1 == nx) ? 0 : x + 1, xm = (x == 0) ? nx - 1 : x - 1;
         const int yp = (y + 1 == ny) ? 0 : y + 1, ym = (y == 0) ? ny - 1 : y - 1;
@@ -315,76 +248,22 @@ __device__ __forceinline__ void step_tile(const CaseDev &c, int tile, int k, int
             const int ex = FOLD ? kx(i) : cx(i), ey = FOLD ? ky(i) : cy(i);
             return node(dst, ex == 0 ? x : (ex > 0 ? xp : xm), ey == 0 ? y : (ey > 0 ? yp : ym));
         };
-        bool skip;
-        if constexpr (FOLD) {
-            RecolourFold rc;
-            if (force) collide_fold<true>(f[jr], sa[jr], sb[jr], gmx, gmy, Fx, Fy, pf, rc);
-            else collide_fold<false>(f[jr], sa[jr], sb[jr], gmx, gmy, Fx, Fy, pf, rc);
-            skip = rc.skip;
-            if (!skip) {
-                double dsum = 0.0;
-                sfor<0, 4>([&](auto M) {
-                    constexpr int K = 2 * decltype(M)::value + 1;
-                    float dK, dJ;
-                    split_fold_pair<K>(rc, f[jr][K], f[jr][K + 1], shift_of<kx(K)>(pf, wk<float>(K)),
-                                       shift_of<kx(K + 1)>(pf, wk<float>(K + 1)), dK, dJ);
-                    dsum += (double)dK;
-                    dsum += (double)dJ;
-                    float *nK = dst_node(K), *nJ = dst_node(K + 1);
-                    stg(nK + K * PLANE, f[jr][K]);
-                    stg(nK + (NK + K) * PLANE, dK);
-                    stg(nJ + (K + 1) * PLANE, f[jr][K + 1]);
-                    stg(nJ + (NK + K + 1) * PLANE, dJ);
-                });
-                float *n0 = dst_node(0);
-                stg(n0, f[jr][0]);
-                stg(n0 + NK * PLANE, (float)(sbd[jr] - dsum));
-            }
-        } else if constexpr (std::is_same<S, double>::value) {
-            Recolour64 rc;
-            if (force) collide_f64<true>(f[jr], sa[jr], sb[jr], gmx, gmy, gmz, Fx, Fy, Fz, c, rc);
-            else collide_f64<false>(f[jr], sa[jr], sb[jr], gmx, gmy, gmz, Fx, Fy, Fz, c, rc);
-            skip = rc.skip;
-            if (!skip) {
-                sfor<0, NV>([&](auto I) {
-                    constexpr int i = decltype(I)::value;
-                    double r, b;
-                    split64<i>(rc, f[jr][i], r, b);
-                    double *n = dst_node(i);
-                    stg(n + i * PLANE, r);
-                    stg(n + (NV + i) * PLANE, b);
-                });
-            }
+        const bool force = tipo >= ITLBM_OP_F1;
+        Recolour<S, FOLD> rc;
+        if constexpr (std::is_same<S, double>::value) gradient_size(gmx, gmy, gmz, rc);
+        if (force) {
+            node_relax<true, S, FOLD>(c, pf, f[jr], sa[jr], sb[jr], Fx, Fy, Fz, rc);
+            if (!rc.skip) node_finish<true, S, FOLD>(c, pf, f[jr], sa[jr], gmx, gmy, gmz, rc);
         } else {
-            Recolour32 rc;
-            if (force) collide_f32<true>(f[jr], sa[jr], sb[jr], gmx, gmy, gmz, Fx, Fy, Fz, pf, rc);
-            else collide_f32<false>(f[jr], sa[jr], sb[jr], gmx, gmy, gmz, Fx, Fy, Fz, pf, rc);
-            skip = rc.skip;
-            if (!skip) {
-                // d_0 is the complement of the moving d_i against the incoming D, both summed in
-                // FP64: the d_i are O(w_i rho), so FP32 sums would round by ~1e-8 rho per node and
-                // step, coherently over uniform regions, and drift the colour masses (1e-6 in 2000
-                // steps); in FP64 the only rounding left is that of d_0 itself.
-                double dsum = 0.0;
-                sfor<0, 9>([&](auto M) {
-                    constexpr int i = 2 * decltype(M)::value + 1;
-                    float di, dj;
-                    split32_pair<i>(rc, f[jr][i], f[jr][i + 1], shift_of<cx(i)>(pf, wgt<float>(i)),
-                                    shift_of<cx(i + 1)>(pf, wgt<float>(i + 1)), di, dj);
-                    dsum += (double)di;
-                    dsum += (double)dj;
-                    float *ni = dst_node(i), *nj = dst_node(i + 1);
-                    stg(ni + i * PLANE, f[jr][i]);
-                    stg(ni + (NV + i) * PLANE, di);
-                    stg(nj + (i + 1) * PLANE, f[jr][i + 1]);
-                    stg(nj + (NV + i + 1) * PLANE, dj);
-                });
-                float *n0 = dst_node(0);
-                stg(n0, f[jr][0]);
-                stg(n0 + NV * PLANE, (float)(sbd[jr] - dsum));
-            }
+            node_relax<false, S, FOLD>(c, pf, f[jr], sa[jr], sb[jr], Fx, Fy, Fz, rc);
+            if (!rc.skip) node_finish<false, S, FOLD>(c, pf, f[jr], sa[jr], gmx, gmy, gmz, rc);
         }
-        if (skip) {  // rho <= 1e-30: the site is streamed unchanged (Operadores_tensao.cpp:347)
+        if (!rc.skip)
+            node_split<S, FOLD>(pf, f[jr], sbd[jr], rc, [&](auto Q, S v) {
+                constexpr int q = decltype(Q)::value;
+                stg(dst_node(q % NP) + q * PLANE, v);
+            });
+        if (rc.skip) {  // rho <= 1e-30: the site is streamed unchanged (Operadores_tensao.cpp:347)
             const S *own = node(src, x, y);
             sfor<0, NP>([&](auto I) {
                 constexpr int i = decltype(I)::value;
@@ -395,12 +274,7 @@ __device__ __forceinline__ void step_tile(const CaseDev &c, int tile, int k, int
         }
 
         if (c.aux != nullptr && (k == aux_k || (c.aux_at_end && k == c.chunk_len - 1))) {
-            const long long o = aux_off(c, x, y);
-            const long long n = c.aux_stride;
-            c.aux[o] = (double)Fx;
-            c.aux[n + o] = (double)Fy;
-            c.aux[2 * n + o] = (double)Fz;
-            c.aux[3 * n + o] = sqrt((double)gmx * gmx + (double)gmy * gmy + (double)gmz * gmz);
+            keep_aux(c, x, y, Fx, Fy, Fz, gmx, gmy, gmz);
         }
       }
     }

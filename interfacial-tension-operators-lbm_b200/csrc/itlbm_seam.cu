@@ -12,7 +12,8 @@ __global__ void k_perturb(int n, double A, double B0, double B1, double B2, cons
     for (int i = 0; i < NV; i++) v[i] = f[(size_t)k * NV + i];
     const double gx = g[3 * k], gy = g[3 * k + 1], gz = g[3 * k + 2], mod2 = gx * gx + gy * gy + gz * gz;
     if (mod2 <= 1.0e-60 || A == 0.0) return;
-    perturb_f64(v, gx, gy, gz, sqrt(mod2), A, B0, B1, B2, [=](double a) { return a / mod2; });
+    if (quotients_normal(gx, gy, gz) && Recip64::ok(mod2)) perturb_f64(v, gx, gy, gz, sqrt(mod2), A, B0, B1, B2, Recip64(mod2));
+    else perturb_f64(v, gx, gy, gz, sqrt(mod2), A, B0, B1, B2, [=](double a) { return a / mod2; });
     for (int i = 0; i < NV; i++) f[(size_t)k * NV + i] = v[i];
 }
 

@@ -299,8 +299,13 @@ int itlbm_case_create(const itlbm_case_desc *d, itlbm_case **out) {
     const size_t per_buf = (size_t)h.buf_elems * elem;
     c->plan = res_plan_single(d->precision, d->nx, d->ny);
     if (c->plan.shape >= 0 && !(c->res_flag = res_flag_get())) c->plan = ResPlan();
-    const size_t xbytes = c->plan.shape >= 0 ? res_exchange_bytes(d->precision, c->plan.shape, c->plan.tiles) : 0;
-    const size_t mem_bytes = 2 * per_buf + xbytes + sizeof(ResTile) * c->plan.tiles;
+    ResQueues queues;
+    size_t xbytes = 0;
+    if (c->plan.shape >= 0) {
+        queues = res_queues({ResCase{c->plan, 0, 1.0}}, c->plan.tiles);
+        xbytes = res_exchange_bytes(d->precision, c->plan.shape, c->plan.tiles);
+    }
+    const size_t mem_bytes = 2 * per_buf + xbytes + (c->plan.shape >= 0 ? queues.bytes() : 0);
     if ((e = cudaMalloc(&c->mem, mem_bytes)) != cudaSuccess) {
         itlbm_case_destroy(c);
         return cuda_fail(e, "cudaMalloc(state)");
@@ -326,14 +331,14 @@ int itlbm_case_create(const itlbm_case_desc *d, itlbm_case **out) {
     cudaMemcpy(c->dev, &h, sizeof(CaseDev), cudaMemcpyHostToDevice);
     cudaMemset(c->mem, 0, mem_bytes);
     if (c->plan.shape >= 0) {
-        std::vector<ResTile> rt;
-        res_tiles(c->plan, 0, 0, rt);
         char *x = (char *)c->mem + 2 * per_buf;
         res_exchange_bind(c->res, x, d->precision, c->plan.shape, c->plan.tiles);
         c->res.cases = c->dev;
-        c->res.tiles = (ResTile *)(x + xbytes);
         c->res.err = c->res_flag;
-        cudaMemcpy(x + xbytes, rt.data(), sizeof(ResTile) * rt.size(), cudaMemcpyHostToDevice);
+        if ((e = res_queues_upload(c->res, queues, x + xbytes, 0)) != cudaSuccess) {
+            itlbm_case_destroy(c);
+            return cuda_fail(e, "tile table");
+        }
     }
     if ((e = launch_init(h, c->dev, *d, 0)) != cudaSuccess ||
         (e = cudaDeviceSynchronize()) != cudaSuccess) {
@@ -359,13 +364,6 @@ static int ensure_aux(itlbm_case *c) {
     if (e != cudaSuccess) return cuda_fail(e, "cudaMemcpy(case)");
     return ITLBM_OK;
 }
-
-// Steps a call must ask for to take the resident kernel, and the most one launch runs.  Its launch
-// costs 20 us (tables, first loads) where a k_step launch costs 8, so it gains from about four steps on:
-// call and synchronisation on a 100^2 drop, k_step / resident, 4 steps: FP64 53 / 52, FP32 34 / 37, fold
-// 39 / 29 us; 6 steps: 76 / 64, 46 / 42, 56 / 34 us.
-constexpr int RES_MIN_STEPS = 6;
-constexpr int RES_MAX_STEPS = 4096;
 
 int itlbm_case_step(itlbm_case *c, int nsteps, int flags, void *stream) {
     if (!c || nsteps < 0) return fail(ITLBM_E_ARG, "bad argument");

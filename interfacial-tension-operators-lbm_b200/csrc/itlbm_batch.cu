@@ -7,7 +7,9 @@
 //     the case's buffer parity and the number of sub-steps it runs in the current replay;
 //   * tile work tables list the TX x TY tiles of every active case, one per storage form (FP64, FP32,
 //     FP32 fold), with their lengths in device memory;
-//   * one replay is a CUDA graph of `chunk` sub-steps: each non-empty table is a chain of launches on
+//   * cases whose tiles fit the device run a whole replay in the resident kernel (itlbm_resident.cu), as
+//     one launch per storage form; the rest are stepped from the work tables;
+//   * one replay of the tables is a CUDA graph of `chunk` sub-steps: each non-empty table is a chain of launches on
 //     its own stream between a fork and a join, one CTA per table entry (the grid is the table length
 //     rounded up to a bucket); a case whose chunk is shorter skips its tiles in the remaining
 //     sub-steps.  The graph is re-captured only when a table's bucket or storage changes;
@@ -16,6 +18,7 @@
 // Each case stops at its next diagnostic step (every diag_every steps and its last step, as
 // Imm_OPS.cpp:293), is measured there by the same device diagnostics as a single case, and retires at
 // its step count or when the stop rule of Imm_OPS.cpp:346-352 / Imm_INCL.cpp:428-433 fires.
+#include "itlbm_resident.h"
 #include "itlbm_site.cuh"
 
 #include <algorithm>
@@ -63,7 +66,9 @@ struct Active {
     bool diag_at_end = false;
     bool measured = false;  // its last advance ended at one of its diagnostic steps (aux kept there)
     bool held = false;      // retired, state kept for itlbm_batch_read_fields until released
+    ResPlan plan;           // tiles in the resident kernel (shape < 0: the box does not fit it)
 };
+
 
 size_t case_bytes(const itlbm_case_desc &d, bool &need_aux) {
     const size_t elem = elem_of(d.precision);
@@ -116,6 +121,19 @@ struct itlbm_batch {
     int tiles_cap[NTAB] = {};
     int *d_ntiles = nullptr;
     bool tables_dirty = true;
+    // resident launches of the current tables, one per storage form and tile configuration (none when the
+    // caller fixed the launch shape or tiling, or in a replay too short for them)
+    bool resident_ok = false, resident_on = false;
+    struct Resident {
+        void *queues = nullptr, *mem = nullptr;  // queues and exchange memory (device)
+        size_t cap = 0;
+        int ctas = 0;       // of the launch, 0: no case
+        int cases = 0;
+        ResArgs args{};
+        unsigned tag = 0;   // tags used so far in the exchange memory
+    } res[NPREC][NRES];
+    int *res_flag = nullptr;
+    bool graph_stale = true;
     int grid[NTAB] = {};
     int ntab[NTAB] = {};  // current table lengths
     int occ[NTAB] = {};   // resident CTAs per SM of each table's step kernel
@@ -187,10 +205,63 @@ void set_grids(itlbm_batch *b) {
     }
 }
 
+// The resident launches of the active cases: per storage form and configuration the cases with the most
+// tiles first (they need the most CTAs at once; the small ones fill what those leave), in queues over all
+// the CTAs the device holds.
+int build_resident(itlbm_batch *b) {
+    for (int pi = 0; pi < NPREC; pi++)
+        for (int shape = 0; shape < NRES; shape++) {
+            itlbm_batch::Resident &X = b->res[pi][shape];
+            const int prec = prec_of_table(pi * NSHAPE);
+            std::vector<ResCase> cs;
+            X.ctas = X.cases = 0;
+            if (!b->resident_on) continue;
+            for (const Active *a : b->slots)
+                if (a && !a->held && a->desc.precision == prec && a->plan.shape == shape)
+                    // a tile of F1 / F2 takes about 1.3 times as long per step as the others
+                    cs.push_back(ResCase{a->plan, a->slot,
+                                         a->desc.op.tipo == ITLBM_OP_F1 || a->desc.op.tipo == ITLBM_OP_F2 ? 1.3 : 1.0});
+            if (cs.empty()) continue;
+            std::stable_sort(cs.begin(), cs.end(),
+                             [](const ResCase &x, const ResCase &y) { return x.plan.tiles > y.plan.tiles; });
+            int tiles = 0;
+            for (const ResCase &k : cs) tiles = std::min(tiles + k.plan.tiles, 1 << 24);
+            const int cap = res_capacity(prec, shape), ctas = std::min(cap, tiles);
+            const ResQueues q = res_queues(cs, ctas);
+            cudaError_t e = cudaSuccess;
+            if (q.bytes() > X.cap) {
+                if (X.queues) cudaFree(X.queues);
+                X.queues = nullptr;
+                X.cap = 0;
+                const size_t want = 2 * q.bytes();
+                if ((e = cudaMalloc(&X.queues, want)) != cudaSuccess) return cuda_fail(e, "resident tile queues");
+                X.cap = want;
+            }
+            if (!X.mem) {
+                const size_t bytes = res_exchange_bytes(prec, shape, cap);
+                if ((e = cudaMalloc(&X.mem, bytes)) != cudaSuccess) return cuda_fail(e, "exchange memory");
+                if ((e = cudaMemsetAsync(X.mem, 0, bytes, b->stream)) != cudaSuccess) return cuda_fail(e, "exchange memory");
+                X.tag = 0;
+                res_exchange_bind(X.args, X.mem, prec, shape, cap);
+            }
+            if ((e = res_queues_upload(X.args, q, X.queues, b->stream)) != cudaSuccess)
+                return cuda_fail(e, "resident tile queues");
+            // the copies read q, and pageable copies may return before they are done
+            if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) return cuda_fail(e, "resident tile queues");
+            X.ctas = ctas;
+            X.cases = (int)cs.size();
+        }
+    return ITLBM_OK;
+}
+
 int upload_tables(itlbm_batch *b) {
     std::vector<TileRef> t[NTAB];
+    if (build_resident(b) != ITLBM_OK) {  // no room for the exchange memory: every case from the work tables
+        b->resident_on = b->resident_ok = false;
+        build_resident(b);
+    }
     for (Active *a : b->slots) {
-        if (!a || a->held) continue;
+        if (!a || a->held || (b->resident_on && a->plan.shape >= 0)) continue;
         const CaseDev &c = b->h_cases[a->slot];
         case_tiles(c, b->narrow, a->slot, &t[table_of(a->desc.precision) * NSHAPE]);
     }
@@ -287,6 +358,51 @@ cudaError_t enqueue_steps(itlbm_batch *b, int k0, int k1) {
     return e;
 }
 
+// The resident launches of K sub-steps, one after the other when they are of one storage form, else each
+// form on a stream of its own (the forms hold different cases), between a fork and a join on the batch stream.
+cudaError_t enqueue_resident(itlbm_batch *b, int K) {
+    int forms = 0;
+    bool busy[NPREC] = {};
+    for (int pi = 0; pi < NPREC; pi++) {
+        for (const auto &X : b->res[pi]) busy[pi] = busy[pi] || X.ctas > 0;
+        forms += busy[pi];
+    }
+    cudaError_t e = cudaSuccess;
+    if (forms > 1 && (e = cudaEventRecord(b->ev_fork, b->stream)) != cudaSuccess) return e;
+    for (int pi = 0; pi < NPREC; pi++) {
+        if (!busy[pi]) continue;
+        const int prec = prec_of_table(pi * NSHAPE);
+        const cudaStream_t st = forms > 1 ? b->side[pi] : b->stream;
+        if (forms > 1 && (e = cudaStreamWaitEvent(st, b->ev_fork, 0)) != cudaSuccess) return e;
+        for (int shape = 0; shape < NRES; shape++) {
+            itlbm_batch::Resident &X = b->res[pi][shape];
+            if (X.ctas == 0) continue;
+            const int most = std::max(1, std::min(RES_MAX_STEPS, (int)((1ll << 30) / X.cases)));
+            for (int k0 = 0; k0 < K; k0 += most) {
+                ResArgs a = X.args;
+                a.cases = b->d_cases;
+                a.err = b->res_flag;
+                a.k0 = k0;
+                a.nsteps = std::min(K - k0, most);
+                a.aux_k = -1;
+                const unsigned tags = (unsigned)X.cases * (unsigned)a.nsteps;
+                if (X.tag + tags >= 1u << 31) {  // the tags start again on cleared memory
+                    const size_t bytes = res_exchange_bytes(prec, shape, X.args.nslots);
+                    if ((e = cudaMemsetAsync(X.mem, 0, bytes, st)) != cudaSuccess) return e;
+                    X.tag = 0;
+                }
+                a.tag0 = X.tag;
+                X.tag += tags;
+                if ((e = res_launch(prec, shape, a, X.ctas, st)) != cudaSuccess) return e;
+            }
+        }
+        if (forms > 1 && ((e = cudaEventRecord(b->ev_join[pi], st)) != cudaSuccess ||
+                          (e = cudaStreamWaitEvent(b->stream, b->ev_join[pi], 0)) != cudaSuccess))
+            return e;
+    }
+    return e;
+}
+
 // Adds the host wall time of its scope to a counter of the batch, in ms.
 struct ScopeTimer {
     const itlbm_batch *b;
@@ -315,6 +431,7 @@ int capture_graph(itlbm_batch *b) {
     if (e != cudaSuccess) return cuda_fail(e, "end capture");
     e = cudaGraphInstantiate(&b->graph, g, 0);
     cudaGraphDestroy(g);
+    b->graph_stale = e != cudaSuccess;
     return e == cudaSuccess ? ITLBM_OK : cuda_fail(e, "graph instantiate");
 }
 
@@ -483,6 +600,7 @@ int admit_cases(itlbm_batch *b) {
         a->t_submit = p.t_submit;
         a->bytes = bytes;
         const itlbm_case_desc &d = p.desc;
+        if (b->resident_ok) a->plan = res_plan_batch(d.precision, d.nx, d.ny);
         CaseDev h{};
         case_layout(h, d.nx, d.ny, d.precision);
         fill_params(h, d.op, d.tau, d.A_fact, d.beta, d.rho_B > 0 ? d.rho_B : 1.0);
@@ -711,11 +829,13 @@ int itlbm_batch_create(const itlbm_batch_config *cfg, itlbm_batch **out) {
     // measures faster
     b->mode = b->cfg.ctas_per_sm > 0 ? b->cfg.ctas_per_sm : -1;
     b->tuning = b->cfg.ctas_per_sm == 0;
+    b->resident_ok = b->cfg.ctas_per_sm == 0 && (b->res_flag = res_flag_get()) != nullptr;
     // ITLBM_BATCH_TILING=narrow | uniform fixes the tiling instead of timing it
     if (const char *v = getenv("ITLBM_BATCH_TILING")) {
         if (!strcmp(v, "narrow") || !strcmp(v, "uniform")) {
             b->narrow = !strcmp(v, "narrow");
             b->tile_fixed = true;
+            b->resident_ok = false;
         }
     }
     for (int p = 0; p < NTAB; p++) b->occ[p] = step_occupancy(prec_of_table(p));
@@ -774,11 +894,6 @@ int itlbm_batch_create(const itlbm_batch_config *cfg, itlbm_batch **out) {
             return cuda_fail(e, "batch streams");
         }
     b->t0 = std::chrono::steady_clock::now();
-    int r = capture_graph(b);
-    if (r) {
-        itlbm_batch_destroy(b);
-        return r;
-    }
     *out = b;
     return ITLBM_OK;
 }
@@ -799,6 +914,12 @@ void itlbm_batch_destroy(itlbm_batch *b) {
     for (int p = 0; p < NTAB; p++)
         if (b->d_tiles[p]) cudaFree(b->d_tiles[p]);
     if (b->d_ntiles) cudaFree(b->d_ntiles);
+    for (auto &row : b->res)
+        for (auto &x : row) {
+            if (x.mem) cudaFree(x.mem);
+            if (x.queues) cudaFree(x.queues);
+        }
+    res_flag_put(b->res_flag);
     if (b->d_drop) cudaFree(b->d_drop);
     if (b->d_strip) cudaFree(b->d_strip);
     if (b->d_jobs) cudaFree(b->d_jobs);
@@ -902,31 +1023,33 @@ int itlbm_batch_advance(itlbm_batch *b, void *stream) {
     cudaError_t e = cudaMemcpyAsync(b->d_cases, b->h_cases.data(), sizeof(CaseDev) * (size_t)(hi + 1),
                                     cudaMemcpyHostToDevice, b->stream);
     if (e != cudaSuccess) return cuda_fail(e, "case table upload");
-    if (b->tables_dirty) {
+    const bool resident = b->resident_ok && K >= RES_MIN_STEPS;
+    if (b->tables_dirty || resident != b->resident_on) {
         TileRef *old[NTAB];
         int g[NTAB];
         for (int p = 0; p < NTAB; p++) {
             old[p] = b->d_tiles[p];
             g[p] = b->grid[p];
         }
+        b->resident_on = resident;
         r = upload_tables(b);
         if (r) return r;
-        bool changed = false;
-        for (int p = 0; p < NTAB; p++) changed = changed || old[p] != b->d_tiles[p] || g[p] != b->grid[p];
-        if (changed) {
-            r = capture_graph(b);
-            if (r) return r;
-        }
+        for (int p = 0; p < NTAB; p++)
+            b->graph_stale = b->graph_stale || old[p] != b->d_tiles[p] || g[p] != b->grid[p];
         b->tables_dirty = false;
     }
+    bool stepped = false;  // cases stepped from the work tables
+    for (int p = 0; p < NTAB; p++) stepped = stepped || b->grid[p] > 0;
     cudaEventRecord(b->ev0, b->stream);
-    if (b->tuning && K == b->cfg.chunk && K >= 3 * TUNE_MIN_WINDOW) {
+    if ((e = enqueue_resident(b, K)) != cudaSuccess) return cuda_fail(e, "resident step launches");
+    if (stepped && b->tuning && K == b->cfg.chunk && K >= 3 * TUNE_MIN_WINDOW) {
         r = tune_and_run(b, K);
         if (r) return r;
-    } else if (K == b->cfg.chunk) {
+    } else if (stepped && K == b->cfg.chunk) {
+        if (b->graph_stale && (r = capture_graph(b))) return r;
         e = cudaGraphLaunch(b->graph, b->stream);
         if (e != cudaSuccess) return cuda_fail(e, "graph launch");
-    } else {
+    } else if (stepped) {
         if ((e = enqueue_steps(b, 0, K)) != cudaSuccess) return cuda_fail(e, "step launches");
     }
     cudaEventRecord(b->ev1, b->stream);
@@ -952,6 +1075,7 @@ int itlbm_batch_advance(itlbm_batch *b, void *stream) {
         if (e != cudaSuccess) return cuda_fail(e, "diagnostic copy");
     }
     if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) return cuda_fail(e, "replay");
+    if (b->res_flag && *(volatile int *)b->res_flag) return fail(ITLBM_E_TIMEOUT, "a wait between the tiles of a step ran out");
     float ms = 0;
     cudaEventElapsedTime(&ms, b->ev0, b->ev1);
     b->device_ms += ms;

@@ -14,13 +14,21 @@
 //   2. the halo's rho^N are taken from the tiles that own those nodes;
 //      (for class P the relaxation, which needs no gradient, comes before that wait);
 //   3. gradient, force, collision (itlbm_node.cuh), and the push of every plane to x + c_i in shared
-//      memory, whose planes have one ghost node on each side;
-//   4. the ghost values are posted, and the ones that enter this tile are taken from its neighbours.
+//      memory;
+//   4. what left the tile is posted, and what enters it is taken from its neighbours.
+// In a plane the nodes follow one another row by row without gaps, so a push is the same shift of the
+// element for every thread and the warp's accesses hit distinct banks whatever the tile's width (planes
+// with ghost columns cost half as many wavefronts again: 380 x 380 FP32 P3 6.6 us per step against 6.2).
+// A value that leaves the tile lands, by the same shift, where one will enter (or in the padding), and is
+// posted from there before that one is written.
 // The values go as 16-byte packs {values, tag} written and read whole (relaxed b128 accesses), so a
 // pack is its own flag: the reader polls the pack until its tag is that of the step, and no fence
 // and no second round trip is needed.  Packs are double-buffered by the parity of the step: a
 // neighbour posts step k + 2 only after it took what this tile posted at k + 1, which this tile did
 // after it had taken everything of step k.
+// A launch may hold more tiles than the device does at once: each CTA takes the tiles of its queue one
+// after the other.  All queues follow one order of the cases, so the first unfinished case always has
+// all its CTAs, and no wait is circular.
 // Every wait is bounded: a wait that runs out sets *err and the CTA returns at the end of its step,
 // as do its neighbours in turn.
 //
@@ -73,6 +81,14 @@ __device__ __forceinline__ unsigned long long ld_pair(const unsigned long long *
     asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ void st_word(unsigned *p, unsigned v) {
+    asm volatile("st.relaxed.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned ld_word(const unsigned *p) {
+    unsigned v;
+    asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
 __device__ __forceinline__ unsigned long long pair_of(unsigned a, unsigned b) {
     return (unsigned long long)a | ((unsigned long long)b << 32);
 }
@@ -88,34 +104,39 @@ struct Geo {
     int nsteps, cur0;   // steps of this launch, the buffer it starts from
     int keep_step;      // the step whose force and gradient are kept
     float rho0;
+    unsigned tag0;      // the tags of this tile's steps are tag0 + 1 ...
+    int slot[9];        // exchange slots of the tile (4) and the eight beside it, row by row
     int tx[3], ty[3], begin_x[3], begin_y[3], size_x[3], size_y[3];  // the tile's column and row and the ones beside them
 };
 
 template <class S, bool FOLD, int NT, int R>
 __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_resident(const __grid_constant__ ResArgs a) {
     using C = ResCfg<S, FOLD, NT, R>;
-    constexpr int NP = C::NP, ND = C::ND, PS = C::PS, PK = C::PK;
+    constexpr int NP = C::NP, ND = C::ND, PS = C::PS, PAD = C::WH, PK = C::PK;
     constexpr bool F64 = std::is_same<S, double>::value;
     using PhiPack = std::conditional_t<F64, uint4, unsigned long long>;
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    S *const pop = reinterpret_cast<S *>(smem_raw);             // [2 NP][PS], planes of (w + 2) x (h + 2)
+    S *const pop = reinterpret_cast<S *>(smem_raw);             // [2 NP][PS]: node t = ly w + lx of a plane at PAD + t
     S *const phi = pop + 2 * NP * PS;                           // (w + 4) x (h + 4)
     unsigned *const rcv = reinterpret_cast<unsigned *>(phi + C::PHIN);  // packs that enter: source << 13 | element
     unsigned *const hal = rcv + C::NPK;                         // halo nodes: source << 10 | element of phi
     unsigned short *const snd = reinterpret_cast<unsigned short *>(hal + C::NRING);  // element of each pack that leaves
     // F1 / F2: the ring-1 gradient and auxiliaries, in the planes' place between their load and the push
-    S *const ringg = pop, *const ringa = pop + 3 * PS;
+    S *const ringg = pop, *const ringa = pop + 3 * C::RING;
 
     // What is the same for all threads sits in shared memory and is read where it is used: kept in
     // registers it would cost the 64-register forms spills, which a thousand threads per SM cannot
     // hold in the cache that the shared memory leaves.
     __shared__ Geo g;
     const int tid = threadIdx.x;
+    int bad = 0;
+    const int qend = a.first[blockIdx.x + 1];
+    for (int qi = a.first[blockIdx.x]; qi < qend; qi++) {
     {
-        const ResTile rt = a.tiles[blockIdx.x];
+        const ResTile rt = a.tiles[qi];
         const CaseDev &c = a.cases[rt.case_id];
         const int nsteps = min(a.nsteps, c.chunk_len - a.k0);
-        if (nsteps <= 0) return;
+        if (nsteps <= 0) continue;  // and so do its other tiles
         const int bx = rt.bx, by = rt.by, H = c.halo;
         const int ty = rt.tile / bx, tx = rt.tile - ty * bx;
         if (tid < 6) {  // the tile's column and row and the ones beside them
@@ -124,14 +145,15 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
             int t = (col ? tx : ty) + d - 1;
             t += t < 0 ? b : (t == b ? -b : 0);
             const int x = tile_begin(t, n, b);
-            (col ? g.tx : g.ty)[d] = t;
+            (col ? g.tx : g.ty)[d] = col ? t : t * bx;
             (col ? g.begin_x : g.begin_y)[d] = x;
             (col ? g.size_x : g.size_y)[d] = tile_begin(t + 1, n, b) - x;
         }
         const int wm = (c.nx + bx - 1) / bx, hm = (c.ny + by - 1) / by;  // largest tile of the case
         const int nxs = ND * hm, nitems = 2 * ND * (hm + wm);
         __syncthreads();
-        const int w = g.size_x[1], h = g.size_y[1], PW = w + 2, PP = w + 4;
+        if (tid >= 32 && tid < 41) g.slot[tid - 32] = a.slots[rt.peers + g.ty[(tid - 32) / 3] + g.tx[(tid - 32) % 3]];
+        const int w = g.size_x[1], h = g.size_y[1], PP = w + 4;
         const int nring = 2 * H * (w + h + 2 * H);
         if (tid == 0) {
             g.c = &c;
@@ -145,9 +167,11 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
             g.nsteps = nsteps;
             g.cur0 = (c.parity0 + a.k0) & 1;
             g.rho0 = c.pf.rho0;
+            g.tag0 = a.tag0 + (unsigned)rt.order * (unsigned)a.nsteps;
             g.keep_step = c.aux == nullptr ? -1 : (c.aux_at_end ? c.chunk_len - 1 : a.aux_k) - a.k0;
         }
 
+        __syncthreads();
         // the packs of the exchange: index = side offset + d * length + position along the side, the
         // same for every tile of the case
         for (int j = tid; j < nitems; j += NT) {
@@ -160,7 +184,7 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
             // leaving: source (lx, ly) in this tile; a diagonal that leaves through a corner goes by its x side
             int lx = xs ? (ex > 0 ? w - 1 : 0) : pos, ly = xs ? pos : (ey > 0 ? h - 1 : 0);
             bool ok = pos < (xs ? h : w) && (xs || (unsigned)(lx + ex) < (unsigned)w);
-            snd[j] = ok ? (unsigned short)(plane * PS + (ly + ey + 1) * PW + lx + ex + 1) : (unsigned short)0xFFFF;
+            snd[j] = ok ? (unsigned short)(plane * PS + PAD + (ly + ey) * w + lx + ex) : (unsigned short)0xFFFF;
             // entering: destination (lx, ly) in this tile, from the tile beside it that holds (lx - ex, ly - ey)
             lx = xs ? (ex > 0 ? 0 : w - 1) : pos;
             ly = xs ? pos : (ey > 0 ? 0 : h - 1);
@@ -170,8 +194,8 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
                 const int sx = lx - ex, sy = ly - ey;
                 const int ix = sx < 0 ? 0 : (sx >= w ? 2 : 1), iy = sy < 0 ? 0 : (sy >= h ? 2 : 1);
                 const int spos = xs ? (iy == 0 ? g.size_y[0] - 1 : (iy == 2 ? 0 : sy)) : sx;
-                v = ((unsigned)((rt.base + g.ty[iy] * bx + g.tx[ix]) * C::NPK + j - pos + spos) << 13) |
-                    (unsigned)(plane * PS + (ly + 1) * PW + lx + 1);
+                v = ((unsigned)(g.slot[iy * 3 + ix] * C::NPK + j - pos + spos) << 13) |
+                    (unsigned)(plane * PS + PAD + ly * w + lx);
             }
             rcv[j] = v;
         }
@@ -192,14 +216,14 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
             const int sx = px < 0 ? px + g.size_x[0] : (px >= w ? px - w : px);
             const int sy = py < 0 ? py + g.size_y[0] : (py >= h ? py - h : py);
             const int node = sy * g.size_x[ix] + sx;
-            hal[j] = ((unsigned)((rt.base + g.ty[iy] * bx + g.tx[ix]) * C::NODES + node) << 10) |
+            hal[j] = ((unsigned)(g.slot[iy * 3 + ix] * C::NODES + node) << 10) |
                      (unsigned)((py + 2) * PP + px + 2);
         }
     }
     __syncthreads();
 
-    // the thread's nodes: the element of a node in a plane (13 bits) and in phi (10 bits), whether it
-    // lies within the stencil's reach of the tile's edge, and whether it exists
+    // the thread's nodes, t = tid + r NT: whether there is one, whether it lies within the stencil's reach
+    // of the tile's edge, and its row
     unsigned me[R];
     const CaseDev &c0 = *g.c;
 #pragma unroll
@@ -209,13 +233,15 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
         if (t < w * h) {
             const int ly = t / w, lx = t - ly * w;
             const bool edge = lx < H || lx >= w - H || ly < H || ly >= h - H;
-            me[r] = 0x80000000u | (edge ? 0x40000000u : 0u) | (unsigned)((ly + 2) * (w + 4) + lx + 2) << 13 |
-                    (unsigned)((ly + 1) * (w + 2) + lx + 1);
+            me[r] = 0x80000000u | (edge ? 0x40000000u : 0u) | (unsigned)ly;
             const S *src = (const S *)c0.buf[g.cur0] + node_off(c0, g.x0 + lx, g.y0 + ly);
 #pragma unroll
-            for (int q = 0; q < 2 * NP; q++) pop[q * PS + (me[r] & 8191u)] = src[q * PLANE];
+            for (int q = 0; q < 2 * NP; q++) pop[q * PS + PAD + t] = src[q * PLANE];
         }
     }
+    // the node's element of phi, with its halo of two nodes, and of the ring-1 region
+    auto phi_el = [&](int r) { return tid + r * NT + (int)(me[r] & 0xFFFFu) * 4 + 2 * g.w + 10; };
+    auto ring_el = [&](int r) { return tid + r * NT + (int)(me[r] & 0xFFFFu) * 2 + g.w + 3; };
     // the node's element in a state buffer
     auto home = [&](int r) {
         const int t = tid + r * NT, ly = t / g.w, lx = t - ly * g.w;
@@ -223,13 +249,12 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
     };
     // the buffer the launch does not end in: a site that is streamed unchanged waits there
     auto spare = [&]() { return (S *)g.c->buf[(g.cur0 ^ (g.nsteps & 1)) ^ 1]; };
-    int bad = 0;
     __syncthreads();
 
     for (int s = 0; s < g.nsteps; s++) {
-        const unsigned tag = a.tag0 + (unsigned)s + 1u;
-        uint4 *const pk = a.packs + ((tag & 1u) ? (size_t)a.slots * (C::NPK * PK) : 0);
-        PhiPack *const ph = (PhiPack *)a.phis + ((tag & 1u) ? (size_t)a.slots * C::NODES : 0);
+        const unsigned tag = g.tag0 + (unsigned)s + 1u;
+        uint4 *const pk = a.packs + ((tag & 1u) ? (size_t)a.nslots * (C::NPK * PK) : 0);
+        PhiPack *const ph = (PhiPack *)a.phis + ((tag & 1u) ? (size_t)a.nslots * C::NODES : 0);
 
         // ---- 1: the node's planes and rho^N ----------------------------------------------------
         S f[R][NP], sa[R], sb[R];
@@ -243,15 +268,15 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
             if (me[r]) {
                 S va[NP], vb[NP];
 #pragma unroll
-                for (int i = 0; i < NP; i++) va[i] = pop[i * PS + (me[r] & 8191u)];
+                for (int i = 0; i < NP; i++) va[i] = pop[i * PS + PAD + tid + r * NT];
 #pragma unroll
-                for (int i = 0; i < NP; i++) vb[i] = pop[(NP + i) * PS + (me[r] & 8191u)];
+                for (int i = 0; i < NP; i++) vb[i] = pop[(NP + i) * PS + PAD + tid + r * NT];
 #pragma unroll
                 for (int i = 0; i < NP; i++) sa[r] = sa[r] + va[i];
 #pragma unroll
                 for (int i = 0; i < NP; i++) sb[r] = sb[r] + vb[i];
                 const S p = phase_of(sa[r], sb[r], g.rho0);
-                phi[me[r] >> 13 & 1023u] = p;
+                phi[phi_el(r)] = p;
                 if (me[r] & 0x40000000u) {
                     const unsigned o = blockIdx.x * C::NODES + tid + r * NT;
                     if constexpr (F64) st_pack(ph + o, (unsigned long long)__double_as_longlong(p), tag);
@@ -340,10 +365,11 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
 #pragma unroll
         for (int r = 0; r < R; r++)
             if (me[r]) {
-                const S *p = phi + (me[r] >> 13 & 1023u);
-                const S *q = ringa + (me[r] & 8191u) * AUXS;
+                const S *p = phi + phi_el(r);
+                const int o = ring ? ring_el(r) : 0;
+                const S *q = ringa + o * AUXS;
                 node_force<S>(c, tipo, pf, [&](int dx, int dy) { return p[dy * PP + dx]; },
-                              [&](int dx, int dy) { return q + (dy * PW + dx) * AUXS; }, ringg + (me[r] & 8191u) * 3, gmx[r], gmy[r],
+                              [&](int dx, int dy) { return q + (dy * PW + dx) * AUXS; }, ringg + o * 3, gmx[r], gmy[r],
                               gmz[r], Fx[r], Fy[r], Fz[r]);
                 if (force) node_relax<true, S, FOLD>(c, pf, f[r], sa[r], sb[r], Fx[r], Fy[r], Fz[r], rc[r]);
             }
@@ -351,7 +377,8 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
 #pragma unroll
         for (int r = 0; r < R; r++)
             if (me[r]) {
-                S *const at[3] = {pop + (me[r] & 8191u) - PW, pop + (me[r] & 8191u), pop + (me[r] & 8191u) + PW};
+                S *const own = pop + PAD + tid + r * NT;
+                S *const at[3] = {own - g.w, own, own + g.w};
                 auto push = [&](auto Q, S v) {
                     constexpr int q = decltype(Q)::value, i = q % NP;
                     constexpr int ex = FOLD ? kx(i) : cx(i), ey = FOLD ? ky(i) : cy(i);
@@ -389,6 +416,7 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
                 if constexpr (F64) st_pack(o, (unsigned long long)__double_as_longlong(pop[e[u] + (j % PK) * NP * PS]), tag);
                 else st_pack(o, pair_of(__float_as_uint(pop[e[u]]), __float_as_uint(pop[e[u] + NP * PS])), tag);
             }
+            __syncthreads();  // what enters takes the places of what left
 #pragma unroll
             for (int u = 0; u < MI; u++) {
                 const int j = tid + u * NT;
@@ -430,8 +458,27 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
         if (me[r]) {
             S *dst = (S *)g.c->buf[g.cur0 ^ (g.nsteps & 1)] + home(r);
 #pragma unroll
-            for (int q = 0; q < 2 * NP; q++) dst[q * PLANE] = pop[q * PS + (me[r] & 8191u)];
+            for (int q = 0; q < 2 * NP; q++) dst[q * PLANE] = pop[q * PS + PAD + tid + r * NT];
         }
+    // Before its next tile writes into its exchange slot, the CTA knows that the tiles beside this one have
+    // taken what it posted last: each says so when it is done.
+    if (qi + 1 < qend) {
+        const unsigned last = g.tag0 + (unsigned)g.nsteps;
+        if (tid == 0) st_word(a.done + blockIdx.x, last);
+        if (tid < 9) {
+            int spins = 0;
+            while ((int)(ld_word(a.done + g.slot[tid]) - last) < 0)
+                if (++spins > SPIN_LIMIT) {
+                    bad = 1;
+                    break;
+                }
+        }
+    } else if (tid == 0) st_word(a.done + blockIdx.x, g.tag0 + (unsigned)g.nsteps);
+    if (__syncthreads_or(bad)) {
+        if (tid == 0) *a.err = 1;
+        return;
+    }
+    }
 }
 
 template <class S, bool FOLD, int NT, int R>

@@ -17,20 +17,24 @@ __host__ __device__ constexpr int res_half_perimeter(int nodes) {
     return nodes == 512 ? 48 : (nodes == 256 ? 40 : (nodes == 128 ? 24 : 16));
 }
 
-// One CTA of a launch: its case, the tile of that case (of bx x by), and the CTA of the case's tile 0.
+// A tile of a launch: its case, which of the case's bx x by tiles it is, where the CTAs (exchange slots) of
+// the case's tiles are listed, and the case's place in the order the queues follow.
 struct ResTile {
-    int case_id, tile, base;
+    int case_id, tile, peers, order;
     unsigned short bx, by;
 };
 
 struct ResArgs {
     const CaseDev *cases;
-    const ResTile *tiles;
+    const ResTile *tiles;   // the queues of the CTAs, one after the other
+    const int *first;       // CTA b takes tiles [first[b], first[b + 1])
+    const int *slots;       // CTA of each tile of each case, from ResTile::peers on
+    unsigned *done;         // per CTA: the last tag of the last tile it finished
     uint4 *packs;      // exchange of populations: 2 parities x slots x NPK x PK packs
     void *phis;        // exchange of rho^N: 2 parities x slots x NODES entries of 8 (FP32) or 16 bytes
     int *err;          // set when a wait ran out
-    int slots;         // CTAs the exchange memory is laid out for (>= the grid)
-    unsigned tag0;     // tags of this launch are tag0 + 1 ... tag0 + nsteps, used by no earlier launch
+    int nslots;        // CTAs the exchange memory is laid out for (>= the grid)
+    unsigned tag0;     // the case of order o uses the tags tag0 + o nsteps + 1 ..., used by no earlier launch
     int k0, nsteps, aux_k;
 };
 
@@ -40,7 +44,8 @@ struct ResCfg {
     static constexpr int ND = FOLD ? 3 : 5;            // of which leave through one side
     static constexpr int NODES = NT * R;
     static constexpr int WH = res_half_perimeter(NODES);
-    static constexpr int PS = NODES + 2 * WH + 4;      // largest (w + 2)(h + 2): stride of a plane
+    static constexpr int PS = NODES + 2 * WH;          // stride of a plane: the nodes, and w + 1 elements on each side
+    static constexpr int RING = NODES + 2 * WH + 4;    // largest (w + 2)(h + 2)
     static constexpr int PHIN = NODES + 4 * WH + 16;   // largest (w + 4)(h + 4)
     static constexpr int NPK = 2 * ND * WH;            // exchanged nodes x planes of one tile
     static constexpr int NRING = 4 * WH + 16;          // halo nodes at reach 2
@@ -50,6 +55,7 @@ struct ResCfg {
     // that for the small tiles, whose boxes leave the SMs half empty anyway
     static constexpr int MIN_CTAS = (sizeof(S) == 8 ? 512 : 1024) / NT / (NT < 256 ? 2 : 1);
     static_assert(NP * PS <= 8192, "element of a pack in 13 bits");
+    static_assert(10 * RING <= 2 * NP * PS, "ring-1 auxiliaries in the planes' place");
     static_assert(PHIN <= 1024, "element of phi in 10 bits");
 };
 
@@ -65,6 +71,14 @@ inline cudaError_t res_launch(int prec, int shape, const ResArgs &a, int grid, c
 }
 
 
+// Steps a call must ask for to take the resident kernel, and the most one launch runs.  Its launch
+// costs 20 us (tables, first loads) where a k_step launch costs 8, so it gains from about four steps on:
+// call and synchronisation on a 100^2 drop, k_step / resident, 4 steps: FP64 53 / 52, FP32 34 / 37, fold
+// 39 / 29 us; 6 steps: 76 / 64, 46 / 42, 56 / 34 us.
+constexpr int RES_MIN_STEPS = 6;
+constexpr int RES_MAX_STEPS = 4096;
+
+
 // How a case is held on chip: the tile configuration and the bx x by tiles, or shape < 0 when the box
 // has more tiles than the device holds at once (or sides below RES_MIN_SIDE).
 constexpr int RES_MIN_SIDE = 8;
@@ -77,7 +91,20 @@ int res_tiling(int nx, int ny, int shape, int &bx, int &by);
 int res_capacity(int prec, int shape);
 ResPlan res_plan_single(int prec, int nx, int ny);  // one case alone on the device
 ResPlan res_plan_batch(int prec, int nx, int ny);   // one of many cases that share it
-void res_tiles(const ResPlan &p, int case_id, int base, std::vector<ResTile> &out);
+// The queues of a launch: cases in order, each on the least loaded of `ctas` CTAs.  A CTA's load is the time its queue ends, with `cost` the time of one tile.
+struct ResCase {
+    ResPlan plan;
+    int case_id;
+    double cost;
+};
+struct ResQueues {
+    std::vector<ResTile> tiles;
+    std::vector<int> first, slots;
+    size_t bytes() const { return sizeof(ResTile) * tiles.size() + sizeof(int) * (first.size() + slots.size()); }
+};
+ResQueues res_queues(const std::vector<ResCase> &cases, int ctas);
+// The queues copied to device memory of bytes() bytes, on a stream, and bound to the launch arguments.
+cudaError_t res_queues_upload(ResArgs &a, const ResQueues &q, void *mem, cudaStream_t st);
 // Bytes of exchange memory for `slots` CTAs, and its binding in a block of that many bytes.
 size_t res_exchange_bytes(int prec, int shape, int slots);
 void res_exchange_bind(ResArgs &a, void *base, int prec, int shape, int slots);

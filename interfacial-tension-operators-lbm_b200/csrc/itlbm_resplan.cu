@@ -103,18 +103,54 @@ ResPlan res_plan_batch(int prec, int nx, int ny) {
     return plan_of(prec, nx, ny, prec == ITLBM_PREC_F32_FOLD ? RES_256x2 : RES_256);
 }
 
-void res_tiles(const ResPlan &p, int case_id, int base, std::vector<ResTile> &out) {
-    for (int t = 0; t < p.tiles; t++)
-        out.push_back(ResTile{case_id, t, base, (unsigned short)p.bx, (unsigned short)p.by});
+ResQueues res_queues(const std::vector<ResCase> &cases, int ctas) {
+    ResQueues Q;
+    std::vector<std::vector<ResTile>> queue(ctas);
+    std::vector<std::pair<double, int>> load(ctas);  // when the CTA is free, and which
+    for (int c = 0; c < ctas; c++) load[c] = {0.0, c};
+    int order = 0;
+    for (const ResCase &k : cases) {
+        const int n = k.plan.tiles, peers = (int)Q.slots.size();
+        // a case starts when its last CTA is free: the earliest ones
+        if (order) std::partial_sort(load.begin(), load.begin() + n, load.end());
+        const double end = load[n - 1].first + k.cost;
+        for (int t = 0; t < n; t++) {
+            const int c = load[t].second;
+            Q.slots.push_back(c);
+            queue[c].push_back(ResTile{k.case_id, t, peers, order, (unsigned short)k.plan.bx, (unsigned short)k.plan.by});
+            load[t].first = end;
+        }
+        order++;
+    }
+    Q.first.push_back(0);
+    for (const auto &q : queue) {
+        Q.tiles.insert(Q.tiles.end(), q.begin(), q.end());
+        Q.first.push_back((int)Q.tiles.size());
+    }
+    return Q;
+}
+
+cudaError_t res_queues_upload(ResArgs &a, const ResQueues &q, void *mem, cudaStream_t st) {
+    char *p = (char *)mem;
+    a.tiles = (const ResTile *)p;
+    cudaError_t e = cudaMemcpyAsync(p, q.tiles.data(), sizeof(ResTile) * q.tiles.size(), cudaMemcpyHostToDevice, st);
+    p += sizeof(ResTile) * q.tiles.size();
+    a.first = (const int *)p;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(p, q.first.data(), sizeof(int) * q.first.size(), cudaMemcpyHostToDevice, st);
+    p += sizeof(int) * q.first.size();
+    a.slots = (const int *)p;
+    if (e == cudaSuccess) e = cudaMemcpyAsync(p, q.slots.data(), sizeof(int) * q.slots.size(), cudaMemcpyHostToDevice, st);
+    return e;
 }
 
 size_t res_exchange_bytes(int prec, int shape, int slots) {
-    return (size_t)2 * slots * (npk_of(prec, shape) * pk_of(prec) * 16 + res_nodes(shape) * phi_bytes(prec));
+    return (size_t)slots * (2 * (npk_of(prec, shape) * pk_of(prec) * 16 + res_nodes(shape) * phi_bytes(prec)) + sizeof(unsigned));
 }
 void res_exchange_bind(ResArgs &a, void *base, int prec, int shape, int slots) {
     a.packs = (uint4 *)base;
     a.phis = (char *)base + (size_t)2 * slots * npk_of(prec, shape) * pk_of(prec) * 16;
-    a.slots = slots;
+    a.done = (unsigned *)((char *)a.phis + (size_t)2 * slots * res_nodes(shape) * phi_bytes(prec));
+    a.nslots = slots;
 }
 
 int *res_flag_get() {

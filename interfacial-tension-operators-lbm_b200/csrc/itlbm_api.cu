@@ -263,6 +263,7 @@ void itlbm_case_destroy(itlbm_case *c) {
     if (c->tmp) cudaFree(c->tmp);
     diag_free(c->diag);
     res_flag_put(c->res_flag);
+    host_stage_unref();
     delete c;
 }
 
@@ -286,6 +287,7 @@ int itlbm_case_create(const itlbm_case_desc *d, itlbm_case **out) {
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return cuda_fail(e, "cudaGetDevice");
     itlbm_case *c = new itlbm_case();
+    host_stage_ref();
     c->desc = *d;
     c->device = dev;
     CaseDev &h = c->host;
@@ -564,8 +566,8 @@ int itlbm_case_read_pops(itlbm_case *c, int which, double *fR, double *fB) {
     const int cur = (int)(c->steps & 1);
     cudaError_t e = cudaDeviceSynchronize();  // steps may have gone to another stream
     if (e == cudaSuccess) e = launch_export(c->dev, c->host.nx, c->host.ny, cur, which, c->tmp, c->tmp + NV * n, 0);
-    if (e == cudaSuccess) e = cudaMemcpy(fR, c->tmp, sizeof(double) * NV * n, cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess) e = cudaMemcpy(fB, c->tmp + NV * n, sizeof(double) * NV * n, cudaMemcpyDeviceToHost);
+    double *const outs[2] = {fR, fB};
+    if (e == cudaSuccess) e = fetch_arrays(outs, 2, NV * n, c->tmp, 0);
     return e == cudaSuccess ? waited(c) : cuda_fail(e, "read_pops");
 }
 
@@ -601,10 +603,8 @@ static int read_fields_as(itlbm_case *c, int form, double *rho_R, double *rho_B,
     if (e == cudaSuccess)
         e = launch_fields(c->dev, c->host, (int)(c->steps & 1), cls_f, form, t, t + n, t + 2 * n, t + 3 * n,
                           t + 4 * n, 0);
-    if (e == cudaSuccess) e = cudaDeviceSynchronize();
-    double *outs[5] = {rho_R, rho_B, ux, uy, uz};
-    for (int k = 0; k < 5 && e == cudaSuccess; k++)
-        if (outs[k]) e = cudaMemcpy(outs[k], t + k * n, sizeof(double) * n, cudaMemcpyDeviceToHost);
+    double *const outs[5] = {rho_R, rho_B, ux, uy, uz};
+    if (e == cudaSuccess) e = fetch_arrays(outs, 5, n, t, 0);
     if (e == cudaSuccess && force) {
         std::vector<double> a(3 * n);
         for (int k = 0; k < 3 && e == cudaSuccess; k++)

@@ -796,12 +796,14 @@ int itlbm_batch_create(const itlbm_batch_config *cfg, itlbm_batch **out) {
     if (!out) return fail(ITLBM_E_ARG, "NULL argument");
     *out = nullptr;
     itlbm_batch *b = new itlbm_batch();
+    host_stage_ref();
     if (cfg) b->cfg = *cfg;
     if (b->cfg.max_cases <= 0) b->cfg.max_cases = 4096;
     if (b->cfg.chunk <= 0) b->cfg.chunk = 500;
     if (b->cfg.diag_every <= 0) b->cfg.diag_every = 500;
     cudaError_t e = cudaGetDevice(&b->device);
     if (e != cudaSuccess) {
+        host_stage_unref();
         delete b;
         return cuda_fail(e, "cudaGetDevice");
     }
@@ -817,6 +819,7 @@ int itlbm_batch_create(const itlbm_batch_config *cfg, itlbm_batch **out) {
         props.location.type = cudaMemLocationTypeDevice;
         props.location.id = b->device;
         if ((e = cudaMemPoolCreate(&b->pool, &props)) != cudaSuccess) {
+            host_stage_unref();
             delete b;
             return cuda_fail(e, "case memory pool");
         }
@@ -947,6 +950,7 @@ void itlbm_batch_destroy(itlbm_batch *b) {
     if (b->stream) cudaStreamDestroy(b->stream);
     if (b->pool) cudaMemPoolDestroy(b->pool);
     if (b->stage) cudaFreeHost(b->stage);
+    host_stage_unref();
     delete b;
 }
 
@@ -1149,11 +1153,9 @@ int itlbm_batch_read_fields(itlbm_batch *b, long long tag, int form, double *rho
     // the post-collision populations of the last step sit in the buffer of the next step's state
     e = launch_fields(b->d_cases + a->slot, b->h_cases[a->slot], a->parity, force, form, t, t + n, t + 2 * n,
                       t + 3 * n, t + 4 * n, b->stream);
-    double *outs[5] = {rho_R, rho_B, ux, uy, uz};
-    for (int k = 0; k < 5 && e == cudaSuccess; k++)
-        if (outs[k]) e = cudaMemcpyAsync(outs[k], t + k * n, sizeof(double) * n, cudaMemcpyDeviceToHost, b->stream);
+    double *const outs[5] = {rho_R, rho_B, ux, uy, uz};
+    if (e == cudaSuccess) e = fetch_arrays(outs, 5, n, t, b->stream);
     cudaFreeAsync(t, b->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
     return e == cudaSuccess ? ITLBM_OK : cuda_fail(e, "read_fields");
 }
 

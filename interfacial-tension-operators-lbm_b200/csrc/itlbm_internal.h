@@ -317,6 +317,14 @@ int snap_write(const char *path, const itlbm_case_desc &d, long long steps, cons
 int snap_read_header(const char *path, SnapHeader &hd);
 int snap_read_state(const char *path, const CaseDev &h, void *state);
 
+// ---- device arrays to host memory (itlbm_hostcopy.cu) -----------------------------------------
+// Copies n arrays of `each` doubles, consecutive in device memory from src, to dst[0..n) (a NULL one is
+// skipped), after the work queued on st; returns when they are in place.
+cudaError_t fetch_arrays(double *const *dst, int n, size_t each, const double *src, cudaStream_t st);
+// Every case and batch holds a reference to the pinned memory the copies go through.
+void host_stage_ref();
+void host_stage_unref();
+
 // ---- error reporting -------------------------------------------------------------------------
 void set_error(const std::string &msg);
 int fail(int code, const std::string &msg);

@@ -299,7 +299,7 @@ int itlbm_case_create(const itlbm_case_desc *d, itlbm_case **out) {
     fill_shift(h, h.rho0, d->geometry == ITLBM_GEOM_DROP ? d->v0 : 0.0);
     const size_t elem = elem_of(d->precision);
     const size_t per_buf = (size_t)h.buf_elems * elem;
-    c->plan = res_plan_single(d->precision, d->nx, d->ny);
+    c->plan = res_plan_single(d->precision, d->op.tipo, d->nx, d->ny);
     if (c->plan.shape >= 0 && !(c->res_flag = res_flag_get())) c->plan = ResPlan();
     ResQueues queues;
     size_t xbytes = 0;

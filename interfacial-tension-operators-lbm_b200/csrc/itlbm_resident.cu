@@ -98,20 +98,19 @@ __device__ __forceinline__ int tile_begin(int t, int n, int b) { return (int)((u
 
 // Of a CTA's tile: its case, its place and size, and what the loop needs of them.
 struct Geo {
-    const CaseDev *c;
-    int tipo, x0, y0, w, h;
+    int x0, y0, w, h;
     int nring, npacks;  // halo nodes; packs that leave (and enter), with those that the corners leave out
     int nsteps, cur0;   // steps of this launch, the buffer it starts from
     int keep_step;      // the step whose force and gradient are kept
-    float rho0;
     unsigned tag0;      // the tags of this tile's steps are tag0 + 1 ...
     int slot[9];        // exchange slots of the tile (4) and the eight beside it, row by row
     int tx[3], ty[3], begin_x[3], begin_y[3], size_x[3], size_y[3];  // the tile's column and row and the ones beside them
 };
 
-template <class S, bool FOLD, int NT, int R>
-__global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_resident(const __grid_constant__ ResArgs a) {
-    using C = ResCfg<S, FOLD, NT, R>;
+template <class S, bool FOLD, int SHAPE>
+__global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::MIN_CTAS)) k_resident(const __grid_constant__ ResArgs a) {
+    using C = ResCfg<S, FOLD, SHAPE>;
+    constexpr int NT = C::NT, R = C::R;
     constexpr int NP = C::NP, ND = C::ND, PS = C::PS, PAD = C::WH, PK = C::PK;
     constexpr bool F64 = std::is_same<S, double>::value;
     using PhiPack = std::conditional_t<F64, uint4, unsigned long long>;
@@ -128,15 +127,25 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
     // registers it would cost the 64-register forms spills, which a thousand threads per SM cannot
     // hold in the cache that the shared memory leaves.
     __shared__ Geo g;
+    __shared__ std::conditional_t<C::OWN_CASE, CaseDev, const CaseDev *> own_case;
+    auto the_case = [&]() -> const CaseDev & {
+        if constexpr (C::OWN_CASE) return own_case;
+        else return *own_case;
+    };
     const int tid = threadIdx.x;
     int bad = 0;
     const int qend = a.first[blockIdx.x + 1];
     for (int qi = a.first[blockIdx.x]; qi < qend; qi++) {
     {
         const ResTile rt = a.tiles[qi];
-        const CaseDev &c = a.cases[rt.case_id];
-        const int nsteps = min(a.nsteps, c.chunk_len - a.k0);
+        const CaseDev &dc = a.cases[rt.case_id];
+        const int nsteps = min(a.nsteps, dc.chunk_len - a.k0);
         if (nsteps <= 0) continue;  // and so do its other tiles
+        if constexpr (C::OWN_CASE) {
+            for (int i = tid; i < (int)(sizeof(CaseDev) / sizeof(int)); i += NT) ((int *)&own_case)[i] = ((const int *)&dc)[i];
+        } else if (tid == 0) own_case = &dc;
+        __syncthreads();
+        const CaseDev &c = the_case();
         const int bx = rt.bx, by = rt.by, H = c.halo;
         const int ty = rt.tile / bx, tx = rt.tile - ty * bx;
         if (tid < 6) {  // the tile's column and row and the ones beside them
@@ -156,8 +165,6 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
         const int w = g.size_x[1], h = g.size_y[1], PP = w + 4;
         const int nring = 2 * H * (w + h + 2 * H);
         if (tid == 0) {
-            g.c = &c;
-            g.tipo = c.tipo;
             g.x0 = g.begin_x[1];
             g.y0 = g.begin_y[1];
             g.w = w;
@@ -166,7 +173,6 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
             g.npacks = nitems * PK;
             g.nsteps = nsteps;
             g.cur0 = (c.parity0 + a.k0) & 1;
-            g.rho0 = c.pf.rho0;
             g.tag0 = a.tag0 + (unsigned)rt.order * (unsigned)a.nsteps;
             g.keep_step = c.aux == nullptr ? -1 : (c.aux_at_end ? c.chunk_len - 1 : a.aux_k) - a.k0;
         }
@@ -225,16 +231,16 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
     // the thread's nodes, t = tid + r NT: whether there is one, whether it lies within the stencil's reach
     // of the tile's edge, and its row
     unsigned me[R];
-    const CaseDev &c0 = *g.c;
 #pragma unroll
     for (int r = 0; r < R; r++) {
-        const int t = tid + r * NT, w = g.w, h = g.h, H = c0.halo;
+        const CaseDev &c = the_case();
+        const int t = tid + r * NT, w = g.w, h = g.h, H = c.halo;
         me[r] = 0;
         if (t < w * h) {
             const int ly = t / w, lx = t - ly * w;
             const bool edge = lx < H || lx >= w - H || ly < H || ly >= h - H;
             me[r] = 0x80000000u | (edge ? 0x40000000u : 0u) | (unsigned)ly;
-            const S *src = (const S *)c0.buf[g.cur0] + node_off(c0, g.x0 + lx, g.y0 + ly);
+            const S *src = (const S *)c.buf[g.cur0] + node_off(c, g.x0 + lx, g.y0 + ly);
 #pragma unroll
             for (int q = 0; q < 2 * NP; q++) pop[q * PS + PAD + t] = src[q * PLANE];
         }
@@ -245,10 +251,10 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
     // the node's element in a state buffer
     auto home = [&](int r) {
         const int t = tid + r * NT, ly = t / g.w, lx = t - ly * g.w;
-        return node_off(*g.c, g.x0 + lx, g.y0 + ly);
+        return node_off(the_case(), g.x0 + lx, g.y0 + ly);
     };
     // the buffer the launch does not end in: a site that is streamed unchanged waits there
-    auto spare = [&]() { return (S *)g.c->buf[(g.cur0 ^ (g.nsteps & 1)) ^ 1]; };
+    auto spare = [&]() { return (S *)the_case().buf[(g.cur0 ^ (g.nsteps & 1)) ^ 1]; };
     __syncthreads();
 
     for (int s = 0; s < g.nsteps; s++) {
@@ -275,7 +281,7 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
                 for (int i = 0; i < NP; i++) sa[r] = sa[r] + va[i];
 #pragma unroll
                 for (int i = 0; i < NP; i++) sb[r] = sb[r] + vb[i];
-                const S p = phase_of(sa[r], sb[r], g.rho0);
+                const S p = phase_of(sa[r], sb[r], the_case().pf.rho0);
                 phi[phi_el(r)] = p;
                 if (me[r] & 0x40000000u) {
                     const unsigned o = blockIdx.x * C::NODES + tid + r * NT;
@@ -284,7 +290,7 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
                 }
                 bool keep;  // a site that will be streamed unchanged (rho <= 1e-30)
                 if constexpr (F64) keep = !(sa[r] + sb[r] > 1.0e-30);
-                else keep = !(g.rho0 + sa[r] > 1.0e-30f);
+                else keep = !(the_case().pf.rho0 + sa[r] > 1.0e-30f);
                 if (keep) {
                     S *tmp = spare() + home(r);
 #pragma unroll
@@ -299,10 +305,10 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
                 }
 #pragma unroll
                 for (int i = 0; i < NP; i++) f[r][i] = F64 ? va[i] + vb[i] : va[i];
-                if (g.tipo < ITLBM_OP_F1) {  // class P: while the halo's rho^N are on their way
+                if (const CaseDev &c = the_case(); c.tipo < ITLBM_OP_F1) {  // class P: while the halo's rho^N are on their way
                     CaseDev::F32Par pf{};
-                    if constexpr (!F64) pf = load_pf(*g.c);
-                    node_relax<false, S, FOLD>(*g.c, pf, f[r], sa[r], sb[r], S(0), S(0), S(0), rc[r]);
+                    if constexpr (!F64) pf = load_pf(c);
+                    node_relax<false, S, FOLD>(c, pf, f[r], sa[r], sb[r], S(0), S(0), S(0), rc[r]);
                 }
             }
         }
@@ -347,8 +353,8 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
         __syncthreads();
 
         // ---- 3: gradient, force, collision, push --------------------------------------------------
-        const CaseDev &c = *g.c;
-        const int tipo = g.tipo, PW = g.w + 2, PP = g.w + 4;
+        const CaseDev &c = the_case();
+        const int tipo = c.tipo, PW = g.w + 2, PP = g.w + 4;
         const bool force = tipo >= ITLBM_OP_F1, ring = tipo == ITLBM_OP_F1 || tipo == ITLBM_OP_F2;
         if (ring) {
             const int nq = PW * (g.h + 2), M = (65536 + PW - 1) / PW;  // q / PW by multiply and shift, exact for q < 65536 / PW
@@ -456,7 +462,7 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
 #pragma unroll
     for (int r = 0; r < R; r++)
         if (me[r]) {
-            S *dst = (S *)g.c->buf[g.cur0 ^ (g.nsteps & 1)] + home(r);
+            S *dst = (S *)the_case().buf[g.cur0 ^ (g.nsteps & 1)] + home(r);
 #pragma unroll
             for (int q = 0; q < 2 * NP; q++) dst[q * PLANE] = pop[q * PS + PAD + tid + r * NT];
         }
@@ -481,15 +487,15 @@ __global__ void __launch_bounds__(NT, ResCfg<S, FOLD, NT, R>::MIN_CTAS) k_reside
     }
 }
 
-template <class S, bool FOLD, int NT, int R>
+template <class S, bool FOLD, int SHAPE>
 struct Entry {
-    using C = ResCfg<S, FOLD, NT, R>;
+    using C = ResCfg<S, FOLD, SHAPE>;
     // resident CTAs per SM, asked once per device (the query also sets the shared-memory limit)
     static int occupancy() {
         int n = 0;
-        if (cudaFuncSetAttribute(k_resident<S, FOLD, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
+        if (cudaFuncSetAttribute(k_resident<S, FOLD, SHAPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM) !=
                 cudaSuccess ||
-            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_resident<S, FOLD, NT, R>, NT, C::SMEM) != cudaSuccess) {
+            cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_resident<S, FOLD, SHAPE>, C::NT, C::SMEM) != cudaSuccess) {
             cudaGetLastError();
             return 0;
         }
@@ -498,7 +504,7 @@ struct Entry {
     static cudaError_t launch(const ResArgs &a, int grid, cudaStream_t st) {
         cudaLaunchConfig_t cfg{};
         cfg.gridDim = dim3((unsigned)grid);
-        cfg.blockDim = dim3(NT);
+        cfg.blockDim = dim3(C::NT);
         cfg.dynamicSmemBytes = C::SMEM;
         cfg.stream = st;
         cudaLaunchAttribute at{};
@@ -506,7 +512,7 @@ struct Entry {
         at.val.cooperative = 1;
         cfg.attrs = &at;
         cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, k_resident<S, FOLD, NT, R>, a);
+        return cudaLaunchKernelEx(&cfg, k_resident<S, FOLD, SHAPE>, a);
     }
 };
 
@@ -514,11 +520,11 @@ struct Entry {
 
 // Compiled twice, like itlbm_step.cu: FP64 without FMA contraction, and the FP32 forms.
 #ifdef ITLBM_STEP_F64
-#define RES_SWITCH(prec, shape, what)                                    \
-    switch (shape) {                                                     \
-        case RES_256: return Entry<double, false, 256, 1>::what;         \
-        case RES_128: return Entry<double, false, 128, 1>::what;         \
-        case RES_64: return Entry<double, false, 64, 1>::what;           \
+#define RES_SWITCH(prec, shape, what)                            \
+    switch (shape) {                                             \
+        case RES_64: return Entry<double, false, RES_64>::what;   \
+        case RES_128: return Entry<double, false, RES_128>::what; \
+        case RES_256: return Entry<double, false, RES_256>::what; \
     }
 int res_occupancy_f64(int prec, int shape) {
     RES_SWITCH(prec, shape, occupancy())
@@ -529,17 +535,18 @@ cudaError_t res_launch_f64(int prec, int shape, const ResArgs &a, int grid, cuda
     return cudaErrorInvalidValue;
 }
 #else
-#define RES_SWITCH(prec, shape, what)                                                              \
-    if (prec == ITLBM_PREC_F32) switch (shape) {                                                   \
-        case RES_256: return Entry<float, false, 256, 1>::what;                                    \
-        case RES_128: return Entry<float, false, 128, 1>::what;                                    \
-        case RES_64: return Entry<float, false, 64, 1>::what;                                      \
-    }                                                                                              \
-    else switch (shape) {                                                                          \
-        case RES_256: return Entry<float, true, 256, 1>::what;                                     \
-        case RES_128: return Entry<float, true, 128, 1>::what;                                     \
-        case RES_64: return Entry<float, true, 64, 1>::what;                                       \
-        case RES_256x2: return Entry<float, true, 256, 2>::what;                                   \
+#define RES_SWITCH(prec, shape, what)                                    \
+    if (prec == ITLBM_PREC_F32) switch (shape) {                         \
+        case RES_64: return Entry<float, false, RES_64>::what;           \
+        case RES_128: return Entry<float, false, RES_128>::what;         \
+        case RES_256: return Entry<float, false, RES_256>::what;         \
+        case RES_256D: return Entry<float, false, RES_256D>::what;       \
+    }                                                                    \
+    else switch (shape) {                                                \
+        case RES_64: return Entry<float, true, RES_64>::what;            \
+        case RES_128: return Entry<float, true, RES_128>::what;          \
+        case RES_256: return Entry<float, true, RES_256>::what;          \
+        case RES_256x2: return Entry<float, true, RES_256x2>::what;      \
     }
 int res_occupancy_f32(int prec, int shape) {
     RES_SWITCH(prec, shape, occupancy())

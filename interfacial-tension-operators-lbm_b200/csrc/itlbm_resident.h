@@ -8,9 +8,11 @@
 
 namespace itlbm {
 
-// Threads and nodes of a tile.
-enum { RES_256 = 0, RES_128 = 1, RES_64 = 2, RES_256x2 = 3, NRES = 4 };  // x2: two nodes per thread (fold)
-__host__ __device__ constexpr int res_threads(int shape) { return shape == RES_128 ? 128 : (shape == RES_64 ? 64 : 256); }
+// Tile configurations, by threads: 64 and 128 with registers to spare (boxes that leave the SMs half empty
+// anyway), 256 for many tiles per SM, and where the storage form allows more, the box sizes beyond: FP32
+// with four CTAs per SM instead of three (D), the fold with two nodes per thread (x2).
+enum { RES_64 = 0, RES_128 = 1, RES_256 = 2, RES_256D = 3, RES_256x2 = 4, NRES = 5 };
+__host__ __device__ constexpr int res_threads(int shape) { return shape == RES_64 ? 64 : (shape == RES_128 ? 128 : 256); }
 __host__ __device__ constexpr int res_nodes(int shape) { return shape == RES_256x2 ? 512 : res_threads(shape); }
 // Largest w + h of a tile of that many nodes: 32 x 16, 32 x 8, 16 x 8, 8 x 8.
 __host__ __device__ constexpr int res_half_perimeter(int nodes) {
@@ -38,11 +40,12 @@ struct ResArgs {
     int k0, nsteps, aux_k;
 };
 
-template <class S, bool FOLD, int NT, int R>
+template <class S, bool FOLD, int SHAPE>
 struct ResCfg {
+    static constexpr int NT = res_threads(SHAPE), R = res_nodes(SHAPE) / NT;  // threads, nodes per thread
     static constexpr int NP = FOLD ? NK : NV;          // planes per colour
     static constexpr int ND = FOLD ? 3 : 5;            // of which leave through one side
-    static constexpr int NODES = NT * R;
+    static constexpr int NODES = res_nodes(SHAPE);
     static constexpr int WH = res_half_perimeter(NODES);
     static constexpr int PS = NODES + 2 * WH;          // stride of a plane: the nodes, and w + 1 elements on each side
     static constexpr int RING = NODES + 2 * WH + 4;    // largest (w + 2)(h + 2)
@@ -51,10 +54,14 @@ struct ResCfg {
     static constexpr int NRING = 4 * WH + 16;          // halo nodes at reach 2
     static constexpr int PK = sizeof(S) == 8 ? 2 : 1;  // packs per exchanged plane: both colours in FP32
     static constexpr int SMEM = (int)sizeof(S) * (2 * NP * PS + PHIN) + 4 * (NPK + NRING) + 2 * NPK;
-    // CTAs per SM the registers are sized for: 64 registers in FP32 and 128 in FP64, as in k_step; twice
-    // that for the small tiles, whose boxes leave the SMs half empty anyway
-    static constexpr int MIN_CTAS = (sizeof(S) == 8 ? 512 : 1024) / NT / (NT < 256 ? 2 : 1);
-    static_assert(NP * PS <= 8192, "element of a pack in 13 bits");
+    // CTAs per SM the registers are sized for.  Measured on B200: FP32 with three CTAs of 256 threads (80
+    // registers, no spills) runs sweeps of 100 x 100 boxes at 24.0 G updates/s, with four (64, spills) at 20.6.
+    static constexpr bool F64 = sizeof(S) == 8;
+    static constexpr int MIN_CTAS = SHAPE == RES_64 ? (F64 ? 4 : 8) : SHAPE == RES_128 ? (F64 ? 2 : 4) : F64 ? 2 : (SHAPE == RES_256 && !FOLD) ? 3 : 4;
+    // The case's parameters in shared memory, or read through the cache where registers are so short that
+    // what the compiler then keeps of them is spilled (FP64 sweep 9.2 against 9.6 G updates/s, FP32 380 x 380
+    // 6.6 against 6.2 us per step; elsewhere 2 % faster).
+    static constexpr bool OWN_CASE = !(SHAPE == RES_256D || (F64 && SHAPE == RES_256));
     static_assert(10 * RING <= 2 * NP * PS, "ring-1 auxiliaries in the planes' place");
     static_assert(PHIN <= 1024, "element of phi in 10 bits");
 };
@@ -85,11 +92,9 @@ constexpr int RES_MIN_SIDE = 8;
 struct ResPlan {
     int shape = -1, bx = 0, by = 0, tiles = 0;
 };
-// The fewest tiles of configuration `shape` that cover an nx x ny box (0 when none do).
-int res_tiling(int nx, int ny, int shape, int &bx, int &by);
 // CTAs of configuration `shape` the current device holds at once (0: no cooperative launch).
 int res_capacity(int prec, int shape);
-ResPlan res_plan_single(int prec, int nx, int ny);  // one case alone on the device
+ResPlan res_plan_single(int prec, int tipo, int nx, int ny);  // one case alone on the device
 ResPlan res_plan_batch(int prec, int nx, int ny);   // one of many cases that share it
 // The queues of a launch: cases in order, each on the least loaded of `ctas` CTAs.  A CTA's load is the time its queue ends, with `cost` the time of one tile.
 struct ResCase {

@@ -17,6 +17,7 @@ int pk_of(int prec) { return prec == ITLBM_PREC_F64 ? 2 : 1; }
 size_t phi_bytes(int prec) { return prec == ITLBM_PREC_F64 ? 16 : 8; }
 
 constexpr int MAX_DEVICES = 32;
+constexpr long long RING_BALANCED_NODES = 24000;  // see res_plan_single
 struct Device {
     std::once_flag once;
     int sms = 0;
@@ -50,57 +51,85 @@ int res_capacity(int prec, int shape) {
     return v ? v->ctas[prec][shape] * v->sms : 0;
 }
 
-int res_tiling(int nx, int ny, int shape, int &bx, int &by) {
-    const int nodes = res_nodes(shape), wh = res_half_perimeter(nodes);
-    long long best = 0;
-    int best_wh = 0;
-    // tiles at least HMAX wide, so that a halo lies in the tiles beside
-    for (int b = 1; b <= nx / HMAX && b <= 65535 && (long long)b * nx < 1LL << 31; b++) {
-        const int w = (nx + b - 1) / b;
-        const int hmax = std::min(nodes / w, wh - w);
+namespace {
+
+int up(int a, int b) { return (a + b - 1) / b; }
+
+// The tiling of an nx x ny box by configuration `shape` with the least cost(tiles, w, h), then the smallest
+// tiles, then the shortest edge; w and h of the largest tile.
+template <class COST>
+double best_tiling(int prec, int nx, int ny, int shape, ResPlan &p, COST cost) {
+    const int nodes = res_nodes(shape), wh = res_half_perimeter(nodes), cap = res_capacity(prec, shape);
+    double least = 0;
+    int size = 0, edge = 0;
+    p = ResPlan();
+    if (nx < RES_MIN_SIDE || ny < RES_MIN_SIDE || (long long)nx * ny > (long long)cap * nodes) return 0;
+    // tiles at least HMAX wide, so that a halo lies in the tiles beside; begins of tiles in 32 bits
+    for (int bx = 1; bx <= nx / HMAX && bx <= std::min(cap, 65535) && (long long)bx * nx < 1LL << 31; bx++) {
+        const int w = up(nx, bx), hmax = std::min(nodes / w, wh - w);
         if (hmax < HMAX) continue;
-        const int v = (ny + hmax - 1) / hmax;
-        if (v > 65535 || ny / v < HMAX || (long long)v * ny >= 1LL << 31) continue;
-        const int h = (ny + v - 1) / v;
-        const long long n = (long long)b * v;
-        if (best == 0 || n < best || (n == best && w + h < best_wh)) {
-            best = n;
-            best_wh = w + h;
-            bx = b;
-            by = v;
+        for (int by = up(ny, hmax); by <= std::min(ny / HMAX, cap / bx) && by <= 65535 && (long long)by * ny < 1LL << 31; by++) {
+            const int h = up(ny, by);
+            const double v = cost(bx * by, w, h);
+            if (p.shape < 0 || v < least || (v == least && (w * h < size || (w * h == size && w + h < edge)))) {
+                least = v;
+                size = w * h;
+                edge = w + h;
+                p.shape = shape;
+                p.bx = bx;
+                p.by = by;
+                p.tiles = bx * by;
+            }
         }
-        if (w <= HMAX) break;
     }
-    return best > (1 << 20) ? 0 : (int)best;
+    return least;
 }
 
-namespace {
-ResPlan plan_of(int prec, int nx, int ny, int shape) {
-    ResPlan p;
-    if (nx < RES_MIN_SIDE || ny < RES_MIN_SIDE || (long long)nx * ny > 1 << 20) return p;
-    const int n = res_tiling(nx, ny, shape, p.bx, p.by);
-    if (n > 0 && n <= res_capacity(prec, shape)) {
-        p.tiles = n;
-        p.shape = shape;
-    }
-    return p;
-}
 }  // namespace
 
-ResPlan res_plan_single(int prec, int nx, int ny) {
-    // The smallest tile whose count fits: the fewer warps an SM runs, the sooner each step ends.  Measured
-    // on B200, us per step, P3, tiles of 64 / 128 / 256 nodes: FP64 100^2 6.3 / 6.3 / 8.4; FP32 100^2
-    // 2.65 / 2.75 / 3.64, 256^2 3.43 / 3.57 / 4.45; fold 256^2 2.86 / 2.89 / 3.12, 380^2 256 threads with
-    // one node each 4.0, with two 5.7 (k_step: 11.8; 6.8, 8.2; 8.2, 9.3).
-    for (const int shape : {RES_64, RES_128, RES_256, RES_256x2}) {
-        const ResPlan p = plan_of(prec, nx, ny, shape);
+// A case alone.  The smallest configuration that holds it: few warps share an SM, and each step ends the
+// sooner (us per step, P3, 64 / 128 / 256 threads: FP64 100^2 3.6 / 3.8 / 5.4, FP32 100^2 2.70 / 2.75 / 3.2,
+// 256^2 3.46 / 3.42 / 3.9, fold 256^2 2.86 / 2.90 / 3.0; k_step 9.1, 6.8, 8.2, 8.2), in the fewest tiles, or
+// with 256 threads in as many as leave the fewest warps on the fullest SM (FP64 200^2 5.96 against 6.20).
+// F1 / F2 also pass over the ring-1 region, a second time when it has more nodes than the CTA threads:
+// there the configuration and tiling with the fewest warps on the fullest SM, the region's counted half
+// (a second pass, one more), as long as the SMs are not full: FP64 F2 100^2 4.84 against 5.19, 150^2 5.45 /
+// 6.0, 200^2 7.8 / 9.75, FP32 F2 100^2 3.06 / 3.18; FP32 F2 150^2 the same, 256^2 4.63 / 4.20.
+ResPlan res_plan_single(int prec, int tipo, int nx, int ny) {
+    const Device *v = device();
+    if (!v) return ResPlan();
+    const bool ring = (tipo == ITLBM_OP_F1 || tipo == ITLBM_OP_F2) &&
+                      (prec == ITLBM_PREC_F64 || (long long)nx * ny <= RING_BALANCED_NODES);
+    ResPlan best;
+    double least = 0;
+    for (int shape = 0; shape < NRES; shape++) {
+        constexpr double factor[NRES] = {1.0, 1.05, 1.3, 1.5, 1.6};  // same work per step
+        const int threads = res_threads(shape);
+        ResPlan p;
+        const double c = factor[shape] * best_tiling(prec, nx, ny, shape, p, [&](int tiles, int w, int h) {
+                             if (!ring && threads < 256) return (double)tiles;
+                             const int region = (w + 2) * (h + 2);
+                             return up(tiles, v->sms) *
+                                    (up(w * h, 32) + (ring ? 0.5 * up(region, 32) + (region > threads ? 1.0 : 0.0) : 0.0));
+                         });
+        if (p.shape < 0) continue;
+        if (!ring) return p;
+        if (best.shape < 0 || c < least) {
+            best = p;
+            least = c;
+        }
+    }
+    return best;
+}
+
+// In a batch the SMs are full: the fewest tiles, whose lanes are the fullest.
+ResPlan res_plan_batch(int prec, int nx, int ny) {
+    for (const int shape : {RES_256, RES_256D, RES_256x2}) {
+        ResPlan p;
+        best_tiling(prec, nx, ny, shape, p, [](int tiles, int, int) { return (double)tiles; });
         if (p.shape >= 0) return p;
     }
     return ResPlan();
-}
-
-ResPlan res_plan_batch(int prec, int nx, int ny) {
-    return plan_of(prec, nx, ny, prec == ITLBM_PREC_F32_FOLD ? RES_256x2 : RES_256);
 }
 
 ResQueues res_queues(const std::vector<ResCase> &cases, int ctas) {

@@ -98,7 +98,8 @@ __device__ __forceinline__ int tile_begin(int t, int n, int b) { return (int)((u
 
 // Of a CTA's tile: its case, its place and size, and what the loop needs of them.
 struct Geo {
-    int x0, y0, w, h;
+    int tipo, x0, y0, w, h;
+    float rho0;
     int nring, npacks;  // halo nodes; packs that leave (and enter), with those that the corners leave out
     int nsteps, cur0;   // steps of this launch, the buffer it starts from
     int keep_step;      // the step whose force and gradient are kept
@@ -165,6 +166,8 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
         const int w = g.size_x[1], h = g.size_y[1], PP = w + 4;
         const int nring = 2 * H * (w + h + 2 * H);
         if (tid == 0) {
+            g.tipo = c.tipo;
+            g.rho0 = c.pf.rho0;
             g.x0 = g.begin_x[1];
             g.y0 = g.begin_y[1];
             g.w = w;
@@ -281,7 +284,7 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
                 for (int i = 0; i < NP; i++) sa[r] = sa[r] + va[i];
 #pragma unroll
                 for (int i = 0; i < NP; i++) sb[r] = sb[r] + vb[i];
-                const S p = phase_of(sa[r], sb[r], the_case().pf.rho0);
+                const S p = phase_of(sa[r], sb[r], g.rho0);
                 phi[phi_el(r)] = p;
                 if (me[r] & 0x40000000u) {
                     const unsigned o = blockIdx.x * C::NODES + tid + r * NT;
@@ -290,7 +293,7 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
                 }
                 bool keep;  // a site that will be streamed unchanged (rho <= 1e-30)
                 if constexpr (F64) keep = !(sa[r] + sb[r] > 1.0e-30);
-                else keep = !(the_case().pf.rho0 + sa[r] > 1.0e-30f);
+                else keep = !(g.rho0 + sa[r] > 1.0e-30f);
                 if (keep) {
                     S *tmp = spare() + home(r);
 #pragma unroll
@@ -305,7 +308,8 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
                 }
 #pragma unroll
                 for (int i = 0; i < NP; i++) f[r][i] = F64 ? va[i] + vb[i] : va[i];
-                if (const CaseDev &c = the_case(); c.tipo < ITLBM_OP_F1) {  // class P: while the halo's rho^N are on their way
+                if (g.tipo < ITLBM_OP_F1) {  // class P: while the halo's rho^N are on their way
+                    const CaseDev &c = the_case();
                     CaseDev::F32Par pf{};
                     if constexpr (!F64) pf = load_pf(c);
                     node_relax<false, S, FOLD>(c, pf, f[r], sa[r], sb[r], S(0), S(0), S(0), rc[r]);
@@ -354,7 +358,7 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
 
         // ---- 3: gradient, force, collision, push --------------------------------------------------
         const CaseDev &c = the_case();
-        const int tipo = c.tipo, PW = g.w + 2, PP = g.w + 4;
+        const int tipo = g.tipo, PW = g.w + 2, PP = g.w + 4;
         const bool force = tipo >= ITLBM_OP_F1, ring = tipo == ITLBM_OP_F1 || tipo == ITLBM_OP_F2;
         if (ring) {
             const int nq = PW * (g.h + 2), M = (65536 + PW - 1) / PW;  // q / PW by multiply and shift, exact for q < 65536 / PW
@@ -547,6 +551,7 @@ cudaError_t res_launch_f64(int prec, int shape, const ResArgs &a, int grid, cuda
         case RES_128: return Entry<float, true, RES_128>::what;          \
         case RES_256: return Entry<float, true, RES_256>::what;          \
         case RES_256x2: return Entry<float, true, RES_256x2>::what;      \
+        case RES_256x2D: return Entry<float, true, RES_256x2D>::what;    \
     }
 int res_occupancy_f32(int prec, int shape) {
     RES_SWITCH(prec, shape, occupancy())

@@ -9,11 +9,11 @@
 namespace itlbm {
 
 // Tile configurations, by threads: 64 and 128 with registers to spare (boxes that leave the SMs half empty
-// anyway), 256 for many tiles per SM, and where the storage form allows more, the box sizes beyond: FP32
-// with four CTAs per SM instead of three (D), the fold with two nodes per thread (x2).
-enum { RES_64 = 0, RES_128 = 1, RES_256 = 2, RES_256D = 3, RES_256x2 = 4, NRES = 5 };
+// anyway), 256 for many tiles per SM, and for the box sizes beyond: FP32 with four CTAs per SM instead of
+// three (D), the fold with two nodes per thread (x2), with three and with four CTAs per SM.
+enum { RES_64 = 0, RES_128 = 1, RES_256 = 2, RES_256D = 3, RES_256x2 = 4, RES_256x2D = 5, NRES = 6 };
 __host__ __device__ constexpr int res_threads(int shape) { return shape == RES_64 ? 64 : (shape == RES_128 ? 128 : 256); }
-__host__ __device__ constexpr int res_nodes(int shape) { return shape == RES_256x2 ? 512 : res_threads(shape); }
+__host__ __device__ constexpr int res_nodes(int shape) { return shape >= RES_256x2 ? 512 : res_threads(shape); }
 // Largest w + h of a tile of that many nodes: 32 x 16, 32 x 8, 16 x 8, 8 x 8.
 __host__ __device__ constexpr int res_half_perimeter(int nodes) {
     return nodes == 512 ? 48 : (nodes == 256 ? 40 : (nodes == 128 ? 24 : 16));
@@ -55,9 +55,11 @@ struct ResCfg {
     static constexpr int PK = sizeof(S) == 8 ? 2 : 1;  // packs per exchanged plane: both colours in FP32
     static constexpr int SMEM = (int)sizeof(S) * (2 * NP * PS + PHIN) + 4 * (NPK + NRING) + 2 * NPK;
     // CTAs per SM the registers are sized for.  Measured on B200: FP32 with three CTAs of 256 threads (80
-    // registers, no spills) runs sweeps of 100 x 100 boxes at 24.0 G updates/s, with four (64, spills) at 20.6.
+    // registers, no spills) runs sweeps of 100 x 100 boxes at 24.0 G updates/s, with four (64, spills) at
+    // 20.6; the fold's P3 410 x 410 with two nodes per thread takes 4.8 us per step with three, 7.3 with four.
     static constexpr bool F64 = sizeof(S) == 8;
-    static constexpr int MIN_CTAS = SHAPE == RES_64 ? (F64 ? 4 : 8) : SHAPE == RES_128 ? (F64 ? 2 : 4) : F64 ? 2 : (SHAPE == RES_256 && !FOLD) ? 3 : 4;
+    static constexpr int MIN_CTAS = SHAPE == RES_64 ? (F64 ? 4 : 8) : SHAPE == RES_128 ? (F64 ? 2 : 4) :
+                                    F64 ? 2 : ((SHAPE == RES_256 && !FOLD) || SHAPE == RES_256x2) ? 3 : 4;
     // The case's parameters in shared memory, or read through the cache where registers are so short that
     // what the compiler then keeps of them is spilled (FP64 sweep 9.2 against 9.6 G updates/s, FP32 380 x 380
     // 6.6 against 6.2 us per step; elsewhere 2 % faster).

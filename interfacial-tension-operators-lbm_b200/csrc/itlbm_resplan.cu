@@ -103,7 +103,7 @@ ResPlan res_plan_single(int prec, int tipo, int nx, int ny) {
     ResPlan best;
     double least = 0;
     for (int shape = 0; shape < NRES; shape++) {
-        constexpr double factor[NRES] = {1.0, 1.05, 1.3, 1.5, 1.6};  // same work per step
+        constexpr double factor[NRES] = {1.0, 1.05, 1.3, 1.5, 1.4, 1.6};  // same work per step
         const int threads = res_threads(shape);
         ResPlan p;
         const double c = factor[shape] * best_tiling(prec, nx, ny, shape, p, [&](int tiles, int w, int h) {
@@ -122,11 +122,18 @@ ResPlan res_plan_single(int prec, int tipo, int nx, int ny) {
     return best;
 }
 
-// In a batch the SMs are full: the fewest tiles, whose lanes are the fullest.
+// In a batch the CTAs are all taken: what counts is the time of a step over the cases that run side by side.
+// That time is about that of the exchange, worth some ten warps a CTA, and of the tile's own warps.
+// Small cases fill what larger ones leave; of one that takes more than a sixth of the CTAs only whole
+// ones fit side by side, and slightly smaller tiles may fill the same CTAs (fold F2 256 x 256: 24.7 G
+// updates/s in 256 tiles, 27.2 in 296).
 ResPlan res_plan_batch(int prec, int nx, int ny) {
-    for (const int shape : {RES_256, RES_256D, RES_256x2}) {
+    for (int shape = RES_256; shape < NRES; shape++) {
+        const int cap = res_capacity(prec, shape);
         ResPlan p;
-        best_tiling(prec, nx, ny, shape, p, [](int tiles, int, int) { return (double)tiles; });
+        best_tiling(prec, nx, ny, shape, p, [&](int tiles, int w, int h) {
+            return (10 + up(w * h, 32)) / (6 * tiles <= cap ? (double)cap / tiles : (double)(cap / tiles));
+        });
         if (p.shape >= 0) return p;
     }
     return ResPlan();

@@ -7,7 +7,11 @@
 // the case, so a case gives the same bits alone or in a batch.  The shell histogram of the logistic
 // fit is accumulated in 64-bit fixed point (2^-40), which makes its atomics order-independent too.
 // The scalar finalisation (centroid angle, fits, ratios) runs in single-thread kernels, so one
-// diagnostic is a chain of launches on one stream with a single copy of the result at the end.
+// diagnostic is three launches on one stream with a single copy of the result at the end: the block
+// that finishes a pass last (a counter per job) reduces its partials, in block order, and goes on with
+// what follows the pass.  (With a launch for each of the ten stages the row of a small case took 107 us,
+// most of it the launches; it takes 76.)  Two blocks of a pass per SM, at 128 registers with a few spills, beat
+// one at 196: 2048 x 2048 from 0.90 to 0.76 ms.
 //
 // Passes of a drop diagnostic (post-collision populations P(x)_i = dst(x + c_i, i)):
 //   D1  calc_galilean's first loop (Galilean_diagnostics.cpp:31-60) and calc_drop_radius's first
@@ -18,7 +22,7 @@
 //       calc_perfil_logistico (Other_functions.cpp:341-377)
 //   F2  pressures, sigma, axis ratio, line estimators (:530-553, Galilean_diagnostics.cpp:88-104)
 //   FIT calc_perfil_logistico's fit (Other_functions.cpp:381-445)
-//   MOD modos_interface (Operadores_tensao.cpp:382-449), one thread per ray
+//   MOD modos_interface (Operadores_tensao.cpp:382-449), one warp per ray
 #include "itlbm_site.cuh"
 
 #include <cfloat>
@@ -31,6 +35,8 @@ namespace {
 constexpr int DT = 256;        // threads of the reduction kernels
 constexpr int MAXB = 148 * 8;  // at most this many partials per pass
 constexpr double FIX = 1099511627776.0;  // 2^40
+constexpr int RAYS_PER_BLOCK = DT / 32;
+constexpr int MODE_BLOCKS = ITLBM_N_ANG / RAYS_PER_BLOCK;  // blocks per job
 
 // Post-collision populations of node (x, y) in FP64.
 __device__ __forceinline__ void post_pops(const CaseDev &c, int cur, int x, int y, double *fR,
@@ -132,15 +138,26 @@ __device__ __forceinline__ const DiagJob &block_job(const DiagJob *jobs, const i
     return J;
 }
 
+// Whether this block is the last of `blocks` to get here; what the others wrote before is then visible.
+__device__ __forceinline__ bool last_block(unsigned *done, int blocks) {
+    __shared__ bool last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1u) == (unsigned)blocks - 1u;
+    __syncthreads();
+    if (last) __threadfence();
+    return last;
+}
+
 // Reduce nb partials (rows of Q) in block order into res[0..Q) (one block).
 template <int Q, int NS, int NM>
-__device__ void reduce_rows(const double *__restrict__ part, int nb, double *__restrict__ res) {
+__device__ void reduce_rows(const double *part, int nb, double *res) {
     double v[Q];
     init_acc<Q, NS, NM>(v);
     for (int b = threadIdx.x; b < nb; b += DT) {
 #pragma unroll
         for (int q = 0; q < Q; q++) {
-            const double x = part[(long long)b * Q + q];
+            const double x = __ldcg(part + (long long)b * Q + q);  // written by other blocks of this launch
             if (q < NS) v[q] = v[q] + x;
             else if (q < NS + NM) v[q] = (v[q] < x) ? x : v[q];
             else v[q] = (x < v[q]) ? x : v[q];
@@ -173,6 +190,7 @@ constexpr int B_NS = 27, B_NM = 3;
 
 // device-side state of one drop diagnostic
 struct DropState {
+    unsigned done1, done2;  // blocks of each launch that are done
     double a[A_Q];
     double b[B_Q];
     int proceed;      // D1 passed (no bad node, positive masses)
@@ -181,9 +199,18 @@ struct DropState {
     double fit[6];
 };
 
-__global__ void __launch_bounds__(DT) k_drop_d1(const DiagJob *__restrict__ jobs,
+__device__ void drop_f1(const DiagJob &J);
+__device__ void drop_f2(const DiagJob &J);
+__device__ void drop_fit(const DiagJob &J);
+__device__ void drop_modes(const DiagJob &J, int k);
+__device__ void drop_modes_sum(const DiagJob &J);
+
+// D1, and F1 by the last block of the job.
+__global__ void __launch_bounds__(DT, 2) k_drop_d1(const DiagJob *__restrict__ jobs,
                                                 const int *__restrict__ blk_job,
                                                 const __grid_constant__ DiagJob one) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     int lb;
     const DiagJob &J = block_job(jobs, blk_job, one, lb);
     const CaseDev &c = *J.c;
@@ -322,15 +349,17 @@ __global__ void __launch_bounds__(DT) k_drop_d1(const DiagJob *__restrict__ jobs
         v[A_CYS] += phi * sin(ty * y);
     }
     block_reduce<A_Q, A_NS, A_NM>(v, J.part + (long long)lb * A_Q);
+    DropState *st = (DropState *)J.state;
+    if (!last_block(&st->done1, nb)) return;
+    reduce_rows<A_Q, A_NS, A_NM>(J.part, nb, st->a);
+    if (threadIdx.x == 0) drop_f1(J);
 }
 
-__global__ void k_drop_f1(const DiagJob *__restrict__ jobs, int njobs, const __grid_constant__ DiagJob one) {
-    const int jid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (jid >= njobs) return;
-    const DiagJob &J = jobs ? jobs[jid] : one;
+// F1 (one thread)
+__device__ __noinline__ void drop_f1(const DiagJob &J) {
     const CaseDev &c = *J.c;
-    DropState *__restrict__ st = (DropState *)J.state;
-    itlbm_drop_diag *__restrict__ d = (itlbm_drop_diag *)J.out;
+    DropState *st = (DropState *)J.state;
+    itlbm_drop_diag *d = (itlbm_drop_diag *)J.out;
     const double *a = st->a;
     const int nx = c.nx, ny = c.ny;
     const double pi = 3.14159265358979323846;
@@ -393,17 +422,37 @@ __device__ __forceinline__ double min_image(double dx, int L) {
 }
 __device__ __forceinline__ double gi_image(double dx, double L) { return dx - L * floor(dx / L + 0.5); }
 
-__global__ void __launch_bounds__(DT) k_drop_d2(const DiagJob *__restrict__ jobs,
-                                                const int *__restrict__ blk_job,
-                                                const __grid_constant__ DiagJob one) {
-    int lb;
-    const DiagJob &J = block_job(jobs, blk_job, one, lb);
-    const DropState *__restrict__ st = (const DropState *)J.state;
+// MOD (the first MODE_BLOCKS blocks per job: the longest chain of dependent loads first), D2 (the blocks that
+// follow), and by the last block of the job F2, FIT and the sums of MOD.
+__device__ void drop_d2(const DiagJob &J, int lb);
+__global__ void __launch_bounds__(DT, 2) k_drop_d2(const DiagJob *__restrict__ jobs, int njobs,
+                                                   const int *__restrict__ blk_job,
+                                                   const __grid_constant__ DiagJob one) {
+    cudaGridDependencySynchronize();
+    int lb = (int)blockIdx.x - njobs * MODE_BLOCKS;
+    const bool modes = lb < 0;
+    const DiagJob *j = jobs ? jobs + (modes ? (int)blockIdx.x / MODE_BLOCKS : blk_job[lb]) : &one;
+    const DiagJob &J = *j;
+    if (jobs && !modes) lb -= J.block0;
+    DropState *st = (DropState *)J.state;
     if (!st->proceed) return;
+    if (modes) drop_modes(J, ((int)blockIdx.x % MODE_BLOCKS) * RAYS_PER_BLOCK + (threadIdx.x >> 5));
+    else drop_d2(J, lb);
+    if (!last_block(&st->done2, J.nblocks + MODE_BLOCKS)) return;
+    reduce_rows<B_Q, B_NS, B_NM>(J.part, J.nblocks, st->b);
+    if (threadIdx.x == 0) drop_f2(J);
+    __syncthreads();
+    if (!*(volatile int *)&st->proceed) return;
+    drop_fit(J);
+    drop_modes_sum(J);
+}
+
+__device__ __forceinline__ void drop_d2(const DiagJob &J, int lb) {
+    const DropState *__restrict__ st = (const DropState *)J.state;
     const itlbm_drop_diag *__restrict__ d = (const itlbm_drop_diag *)J.out;
     const double v0 = J.v0;
     const double *__restrict__ node = J.node;
-    unsigned long long *__restrict__ shell = J.shell;
+    unsigned long long *shell = J.shell;
     const int nshell = J.nshell, nb = J.nblocks;
     const CaseDev &c = *J.c;
     const int nx = c.nx, ny = c.ny;
@@ -472,13 +521,10 @@ __global__ void __launch_bounds__(DT) k_drop_d2(const DiagJob *__restrict__ jobs
     block_reduce<B_Q, B_NS, B_NM>(v, J.part + (long long)lb * B_Q);
 }
 
-__global__ void k_drop_f2(const DiagJob *__restrict__ jobs, int njobs, const __grid_constant__ DiagJob one) {
-    const int jid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (jid >= njobs) return;
-    const DiagJob &J = jobs ? jobs[jid] : one;
-    DropState *__restrict__ st = (DropState *)J.state;
-    if (!st->proceed) return;
-    itlbm_drop_diag *__restrict__ d = (itlbm_drop_diag *)J.out;
+// F2 (one thread)
+__device__ __noinline__ void drop_f2(const DiagJob &J) {
+    DropState *st = (DropState *)J.state;
+    itlbm_drop_diag *d = (itlbm_drop_diag *)J.out;
     const int step = J.step;
     const double v0 = J.v0, x_ini = J.x_ini, y_ini = J.y_ini;
     const double *__restrict__ node = J.node;
@@ -536,13 +582,9 @@ __global__ void k_drop_f2(const DiagJob *__restrict__ jobs, int njobs, const __g
 }
 
 // calc_perfil_logistico's fit over the shells (one block)
-__global__ void __launch_bounds__(DT) k_drop_fit(const DiagJob *__restrict__ jobs,
-                                                 const __grid_constant__ DiagJob one) {
-    const DiagJob &J = jobs ? jobs[blockIdx.x] : one;
-    DropState *__restrict__ st = (DropState *)J.state;
-    if (!st->proceed) return;
-    itlbm_drop_diag *__restrict__ d = (itlbm_drop_diag *)J.out;
-    const unsigned long long *__restrict__ shell = J.shell;
+__device__ __noinline__ void drop_fit(const DiagJob &J) {
+    itlbm_drop_diag *d = (itlbm_drop_diag *)J.out;
+    const unsigned long long *shell = J.shell;
     const int nshell = J.nshell;
     const double eps = 1.0e-30, d_casca = 0.5;
     double v[6];
@@ -631,13 +673,7 @@ __device__ double fase_em(const double *__restrict__ node, long long n, int nx, 
 // from its interval exactly as the serial bisection forms it), then walks the tree by the signs.  The
 // 12 rounds take the same path and give the same interval, bit for bit, with 12 dependent
 // evaluations instead of 60.
-constexpr int RAYS_PER_BLOCK = DT / 32;
-constexpr int MODE_BLOCKS = ITLBM_N_ANG / RAYS_PER_BLOCK;  // blocks per job
-__global__ void __launch_bounds__(DT) k_drop_modes(const DiagJob *__restrict__ jobs,
-                                                   const __grid_constant__ DiagJob one) {
-    const DiagJob &J = jobs ? jobs[blockIdx.x / MODE_BLOCKS] : one;
-    const DropState *__restrict__ st = (const DropState *)J.state;
-    if (!st->proceed) return;
+__device__ __noinline__ void drop_modes(const DiagJob &J, int k) {
     const itlbm_drop_diag *__restrict__ d = (const itlbm_drop_diag *)J.out;
     const CaseDev &c = *J.c;
     const int nx = c.nx, ny = c.ny;
@@ -645,7 +681,6 @@ __global__ void __launch_bounds__(DT) k_drop_modes(const DiagJob *__restrict__ j
     const double *__restrict__ node = J.node;
     const int N_ANG = ITLBM_N_ANG;
     const int lane = threadIdx.x & 31;
-    const int k = (blockIdx.x % MODE_BLOCKS) * RAYS_PER_BLOCK + (threadIdx.x >> 5);
     const double x0 = d->x0, y0 = d->y0, R_est = d->raio;
     const double th = 2.0 * 3.14159265358979323846 * k / N_ANG, ct = cos(th), st_ = sin(th);
     double a = 0.3 * R_est, b = 1.7 * R_est;
@@ -685,47 +720,51 @@ __global__ void __launch_bounds__(DT) k_drop_modes(const DiagJob *__restrict__ j
     }
 }
 
-// The harmonic sums over the rays in ray order, as the reference loop accumulates them (one block
-// per job).
-__global__ void __launch_bounds__(ITLBM_N_ANG) k_drop_modes_sum(const DiagJob *__restrict__ jobs,
-                                                                const __grid_constant__ DiagJob one) {
-    const DiagJob &J = jobs ? jobs[blockIdx.x] : one;
-    if (!((const DropState *)J.state)->proceed) return;
-    itlbm_drop_diag *__restrict__ d = (itlbm_drop_diag *)J.out;
+// The harmonic sums over the rays in ray order, as the reference loop accumulates them (one block).
+static_assert(DT == ITLBM_N_ANG, "one thread per ray");
+__device__ __noinline__ void drop_modes_sum(const DiagJob &J) {
+    itlbm_drop_diag *d = (itlbm_drop_diag *)J.out;
     const int N_ANG = ITLBM_N_ANG;
-    __shared__ double rs[7][ITLBM_N_ANG];
+    __shared__ double rs[7][ITLBM_N_ANG + 1];
     const int k = threadIdx.x;
 #pragma unroll
     for (int q = 0; q < 7; q++) rs[q][k] = J.rays[q * N_ANG + k];
     __syncthreads();
-    if (k == 0) {
-        double c2 = 0, s2 = 0, c4 = 0, s4 = 0, c8 = 0, s8 = 0, soma = 0, rmin = 1e30, rmax = 0;
+    if (k >= 32) return;
+    // one lane per sum, one for the least and the largest
+    double sum = 0, rmin = 1e30, rmax = 0;
+    if (k < 7) {
+        for (int j = 0; j < N_ANG; j++) sum += rs[k][j];
+    } else if (k == 7) {
         for (int j = 0; j < N_ANG; j++) {
-            const double rr = rs[0][j];
-            soma += rr;
-            c2 += rs[1][j];
-            s2 += rs[2][j];
-            c4 += rs[3][j];
-            s4 += rs[4][j];
-            c8 += rs[5][j];
-            s8 += rs[6][j];
-            rmin = fmin(rmin, rr);
-            rmax = fmax(rmax, rr);
+            rmin = fmin(rmin, rs[0][j]);
+            rmax = fmax(rmax, rs[0][j]);
         }
+    }
+    const double soma = __shfl_sync(0xffffffffu, sum, 0);
+    const double c2 = __shfl_sync(0xffffffffu, sum, 1), s2 = __shfl_sync(0xffffffffu, sum, 2);
+    const double c4 = __shfl_sync(0xffffffffu, sum, 3), s4 = __shfl_sync(0xffffffffu, sum, 4);
+    const double c8 = __shfl_sync(0xffffffffu, sum, 5), s8 = __shfl_sync(0xffffffffu, sum, 6);
+    rmin = __shfl_sync(0xffffffffu, rmin, 7);
+    rmax = __shfl_sync(0xffffffffu, rmax, 7);
+    if (k == 0) {
+        // the multiply-adds written out: which product the compiler takes depends on the code around
         d->R0 = soma / N_ANG;
-        d->a2 = 2.0 * sqrt(c2 * c2 + s2 * s2) / N_ANG / d->R0;
-        d->a4 = 2.0 * sqrt(c4 * c4 + s4 * s4) / N_ANG / d->R0;
-        d->a8 = 2.0 * sqrt(c8 * c8 + s8 * s8) / N_ANG / d->R0;
+        d->a2 = 2.0 * sqrt(__fma_rn(s2, s2, __dmul_rn(c2, c2))) / N_ANG / d->R0;
+        d->a4 = 2.0 * sqrt(__fma_rn(c4, c4, __dmul_rn(s4, s4))) / N_ANG / d->R0;
+        d->a8 = 2.0 * sqrt(__fma_rn(c8, c8, __dmul_rn(s8, s8))) / N_ANG / d->R0;
         d->rmin = rmin;
         d->rmax = rmax;
     }
 }
 
-// Clears what a drop diagnostic accumulates into: its output and its shell histogram (one block per
-// job).
+// Clears what a drop diagnostic accumulates into: its output, its shell histogram and its block counters
+// (one block per job).
 __global__ void __launch_bounds__(DT) k_drop_clear(const DiagJob *__restrict__ jobs,
                                                    const __grid_constant__ DiagJob one) {
+    cudaTriggerProgrammaticLaunchCompletion();
     const DiagJob &J = jobs ? jobs[blockIdx.x] : one;
+    if (threadIdx.x == 0) ((DropState *)J.state)->done1 = ((DropState *)J.state)->done2 = 0u;
     unsigned *o = (unsigned *)J.out;
     for (int w = threadIdx.x; w < (int)(sizeof(itlbm_drop_diag) / 4); w += DT) o[w] = 0u;
     for (int w = threadIdx.x; w < 2 * J.nshell; w += DT) J.shell[w] = 0ull;
@@ -744,6 +783,7 @@ enum {
 constexpr int S_NS = 17, S_NM = 3;
 
 struct StripState {
+    unsigned done1, done2;
     double a[S_Q];
     double K, a0;
     int fit;
@@ -760,9 +800,13 @@ __device__ __forceinline__ double dist_central(int x, int y, int p, int q, int N
     return -d / m;
 }
 
-__global__ void __launch_bounds__(DT) k_strip_s1(const DiagJob *__restrict__ jobs,
+__device__ void strip_f1(const DiagJob &J);
+// S1, and what follows it by the last block of the job.
+__global__ void __launch_bounds__(DT, 2) k_strip_s1(const DiagJob *__restrict__ jobs,
                                                  const int *__restrict__ blk_job,
                                                  const __grid_constant__ DiagJob one) {
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
     int lb;
     const DiagJob &J = block_job(jobs, blk_job, one, lb);
     const CaseDev &c = *J.c;
@@ -837,14 +881,15 @@ __global__ void __launch_bounds__(DT) k_strip_s1(const DiagJob *__restrict__ job
         }
     }
     block_reduce<S_Q, S_NS, S_NM>(v, J.part + (long long)lb * S_Q);
+    StripState *st = (StripState *)J.state;
+    if (!last_block(&st->done1, nb)) return;
+    reduce_rows<S_Q, S_NS, S_NM>(J.part, nb, st->a);
+    if (threadIdx.x == 0) strip_f1(J);
 }
 
-__global__ void k_strip_f1(const DiagJob *__restrict__ jobs, int njobs, const __grid_constant__ DiagJob one) {
-    const int jid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (jid >= njobs) return;
-    const DiagJob &J = jobs ? jobs[jid] : one;
-    StripState *__restrict__ st = (StripState *)J.state;
-    itlbm_strip_diag *__restrict__ r = (itlbm_strip_diag *)J.out;
+__device__ __noinline__ void strip_f1(const DiagJob &J) {
+    StripState *st = (StripState *)J.state;
+    itlbm_strip_diag *r = (itlbm_strip_diag *)J.out;
     const int p = J.p, q = J.q;
     const int N = J.c->nx;
     const double *a = st->a;
@@ -885,12 +930,13 @@ __global__ void k_strip_f1(const DiagJob *__restrict__ jobs, int njobs, const __
     r->ok = (r->n_ruim == 0 && isfinite(r->u_max));
 }
 
-__global__ void __launch_bounds__(DT) k_strip_s2(const DiagJob *__restrict__ jobs,
+__global__ void __launch_bounds__(DT, 2) k_strip_s2(const DiagJob *__restrict__ jobs,
                                                  const int *__restrict__ blk_job,
                                                  const __grid_constant__ DiagJob one) {
+    cudaGridDependencySynchronize();
     int lb;
     const DiagJob &J = block_job(jobs, blk_job, one, lb);
-    const StripState *__restrict__ st = (const StripState *)J.state;
+    StripState *st = (StripState *)J.state;
     const int cur = J.cur, p = J.p, q = J.q, nb = J.nblocks;
     double m[1] = {0.0};
     if (st->fit) {
@@ -918,36 +964,18 @@ __global__ void __launch_bounds__(DT) k_strip_s2(const DiagJob *__restrict__ job
         }
     }
     block_reduce<1, 0, 1>(m, J.part + lb);
-}
-
-__global__ void k_strip_f2(const DiagJob *__restrict__ jobs, int njobs, const __grid_constant__ DiagJob one) {
-    const int jid = blockIdx.x * blockDim.x + threadIdx.x;
-    if (jid >= njobs) return;
-    const DiagJob &J = jobs ? jobs[jid] : one;
-    const StripState *__restrict__ st = (const StripState *)J.state;
-    itlbm_strip_diag *__restrict__ r = (itlbm_strip_diag *)J.out;
-    if (st->fit) r->res = st->res[0] < 0 ? 0.0 : st->res[0];
+    if (!last_block(&st->done2, nb)) return;
+    reduce_rows<1, 0, 1>(J.part, nb, st->res);
+    if (threadIdx.x == 0 && st->fit) ((itlbm_strip_diag *)J.out)->res = st->res[0] < 0 ? 0.0 : st->res[0];
 }
 
 __global__ void __launch_bounds__(DT) k_strip_clear(const DiagJob *__restrict__ jobs,
                                                     const __grid_constant__ DiagJob one) {
+    cudaTriggerProgrammaticLaunchCompletion();
     const DiagJob &J = jobs ? jobs[blockIdx.x] : one;
+    if (threadIdx.x == 0) ((StripState *)J.state)->done1 = ((StripState *)J.state)->done2 = 0u;
     unsigned *o = (unsigned *)J.out;
     for (int w = threadIdx.x; w < (int)(sizeof(itlbm_strip_diag) / 4); w += DT) o[w] = 0u;
-}
-
-// The block reductions of the partials, one block per job, into the job's running state.
-enum { R_DROP_A, R_DROP_B, R_STRIP_A, R_STRIP_RES };
-template <int Q, int NS, int NM, int W>
-__global__ void __launch_bounds__(DT) k_reduce_jobs(const DiagJob *__restrict__ jobs,
-                                                    const __grid_constant__ DiagJob one) {
-    const DiagJob &J = jobs ? jobs[blockIdx.x] : one;
-    double *res;
-    if constexpr (W == R_DROP_A) res = ((DropState *)J.state)->a;
-    else if constexpr (W == R_DROP_B) res = ((DropState *)J.state)->b;
-    else if constexpr (W == R_STRIP_A) res = ((StripState *)J.state)->a;
-    else res = ((StripState *)J.state)->res;
-    reduce_rows<Q, NS, NM>(J.part, J.nblocks, res);
 }
 
 // Per-node output fields of the post-collision state, each value formed with the reference's
@@ -1062,33 +1090,37 @@ constexpr size_t OUT_BYTES =
 constexpr int PART_COLS = 32;  // >= the quantities of any pass
 static_assert(A_Q <= PART_COLS && B_Q <= PART_COLS && S_Q <= PART_COLS, "partial rows");
 
+// A launch that may begin while the one before it in the stream ends; the kernel waits for that one.
+template <class... P, class... A>
+cudaError_t launch_next(void (*k)(P...), int grid, cudaStream_t st, A... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(DT);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k, args...);
+}
+
 cudaError_t run_drop(const DiagJob *jobs, int njobs, const int *blk_job, int total_blocks, const DiagJob &one,
                      cudaStream_t st) {
-    const int g32 = (njobs + 31) / 32;
     k_drop_clear<<<njobs, DT, 0, st>>>(jobs, one);
-    k_drop_d1<<<total_blocks, DT, 0, st>>>(jobs, blk_job, one);
-    k_reduce_jobs<A_Q, A_NS, A_NM, R_DROP_A><<<njobs, DT, 0, st>>>(jobs, one);
-    k_drop_f1<<<g32, 32, 0, st>>>(jobs, njobs, one);
-    k_drop_d2<<<total_blocks, DT, 0, st>>>(jobs, blk_job, one);
-    k_reduce_jobs<B_Q, B_NS, B_NM, R_DROP_B><<<njobs, DT, 0, st>>>(jobs, one);
-    k_drop_f2<<<g32, 32, 0, st>>>(jobs, njobs, one);
-    k_drop_fit<<<njobs, DT, 0, st>>>(jobs, one);
-    k_drop_modes<<<njobs * MODE_BLOCKS, DT, 0, st>>>(jobs, one);
-    k_drop_modes_sum<<<njobs, ITLBM_N_ANG, 0, st>>>(jobs, one);
-    return cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_next(k_drop_d1, total_blocks, st, jobs, blk_job, one);
+    if (e == cudaSuccess) e = launch_next(k_drop_d2, total_blocks + njobs * MODE_BLOCKS, st, jobs, njobs, blk_job, one);
+    return e;
 }
 
 cudaError_t run_strip(const DiagJob *jobs, int njobs, const int *blk_job, int total_blocks, const DiagJob &one,
                       cudaStream_t st) {
-    const int g32 = (njobs + 31) / 32;
     k_strip_clear<<<njobs, DT, 0, st>>>(jobs, one);
-    k_strip_s1<<<total_blocks, DT, 0, st>>>(jobs, blk_job, one);
-    k_reduce_jobs<S_Q, S_NS, S_NM, R_STRIP_A><<<njobs, DT, 0, st>>>(jobs, one);
-    k_strip_f1<<<g32, 32, 0, st>>>(jobs, njobs, one);
-    k_strip_s2<<<total_blocks, DT, 0, st>>>(jobs, blk_job, one);
-    k_reduce_jobs<1, 0, 1, R_STRIP_RES><<<njobs, DT, 0, st>>>(jobs, one);
-    k_strip_f2<<<g32, 32, 0, st>>>(jobs, njobs, one);
-    return cudaGetLastError();
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = launch_next(k_strip_s1, total_blocks, st, jobs, blk_job, one);
+    if (e == cudaSuccess) e = launch_next(k_strip_s2, total_blocks, st, jobs, blk_job, one);
+    return e;
 }
 
 }  // namespace

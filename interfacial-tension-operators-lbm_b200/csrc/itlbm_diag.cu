@@ -6,7 +6,7 @@
 // one-block kernel then reduces the partials in block order.  The order depends only on the size of
 // the case, so a case gives the same bits alone or in a batch.  The shell histogram of the logistic
 // fit is accumulated in 64-bit fixed point (2^-40), which makes its atomics order-independent too.
-// The scalar finalisation (centroid angle, fits, ratios) runs in single-thread kernels, so one
+// One thread runs the scalar finalisation (centroid angle, fits, ratios), and one
 // diagnostic is three launches on one stream with a single copy of the result at the end: the block
 // that finishes a pass last (a counter per job) reduces its partials, in block order, and goes on with
 // what follows the pass.  (With a launch for each of the ten stages the row of a small case took 107 us,

@@ -49,7 +49,10 @@ template <class S, class PHI, class AUX>
 __device__ __forceinline__ void node_force(const CaseDev &c, int tipo, const CaseDev::F32Par &pf, PHI phi_at,
                                            AUX aux_at, const S *g, S &gmx, S &gmy, S &gmz, S &Fx, S &Fy, S &Fz) {
     if constexpr (std::is_same<S, float>::value) {
-        mediator_grad_fold(phi_at, gmx, gmy);  // FP32: class form, g_z = 0 on the slab
+        if (tipo == ITLBM_OP_F1 || tipo == ITLBM_OP_F2) {  // the ring-1 gradient is its exact negative
+            gmx = -g[0];
+            gmy = -g[1];
+        } else mediator_grad_fold(phi_at, gmx, gmy);  // FP32: class form, g_z = 0 on the slab
         gmz = S(0);
     } else mediator_grad_at<S>(phi_at, gmx, gmy, gmz);
     Fx = S(0);

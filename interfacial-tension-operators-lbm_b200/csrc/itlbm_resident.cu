@@ -38,6 +38,7 @@
 #include "itlbm_node.cuh"
 #include "itlbm_resident.h"
 
+#include <algorithm>
 #include <climits>
 
 namespace itlbm {
@@ -118,8 +119,8 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
     extern __shared__ __align__(16) unsigned char smem_raw[];
     S *const pop = reinterpret_cast<S *>(smem_raw);             // [2 NP][PS]: node t = ly w + lx of a plane at PAD + t
     S *const phi = pop + 2 * NP * PS;                           // (w + 4) x (h + 4)
-    unsigned *const rcv = reinterpret_cast<unsigned *>(phi + C::PHIN);  // packs that enter: source << 13 | element
-    unsigned *const hal = rcv + C::NPK;                         // halo nodes: source << 10 | element of phi
+    unsigned *const rcv = reinterpret_cast<unsigned *>(phi + C::PHIN);  // packs that enter: source << EB | element
+    unsigned *const hal = rcv + C::NPK;                         // halo nodes: source << HB | element of phi
     unsigned short *const snd = reinterpret_cast<unsigned short *>(hal + C::NRING);  // element of each pack that leaves
     // F1 / F2: the ring-1 gradient and auxiliaries, in the planes' place between their load and the push
     S *const ringg = pop, *const ringa = pop + 3 * C::RING;
@@ -203,7 +204,7 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
                 const int sx = lx - ex, sy = ly - ey;
                 const int ix = sx < 0 ? 0 : (sx >= w ? 2 : 1), iy = sy < 0 ? 0 : (sy >= h ? 2 : 1);
                 const int spos = xs ? (iy == 0 ? g.size_y[0] - 1 : (iy == 2 ? 0 : sy)) : sx;
-                v = ((unsigned)(g.slot[iy * 3 + ix] * C::NPK + j - pos + spos) << 13) |
+                v = ((unsigned)(g.slot[iy * 3 + ix] * C::NPK + j - pos + spos) << C::EB) |
                     (unsigned)(plane * PS + PAD + ly * w + lx);
             }
             rcv[j] = v;
@@ -225,7 +226,7 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
             const int sx = px < 0 ? px + g.size_x[0] : (px >= w ? px - w : px);
             const int sy = py < 0 ? py + g.size_y[0] : (py >= h ? py - h : py);
             const int node = sy * g.size_x[ix] + sx;
-            hal[j] = ((unsigned)(g.slot[iy * 3 + ix] * C::NODES + node) << 10) |
+            hal[j] = ((unsigned)(g.slot[iy * 3 + ix] * C::NODES + node) << C::HB) |
                      (unsigned)((py + 2) * PP + px + 2);
         }
     }
@@ -335,17 +336,17 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
 #pragma unroll
                 for (int u = 0; u < MI; u++)
                     if (pend >> u & 1u) {
-                        if constexpr (F64) ld_pack(ph + (e[u] >> 10), lo[u], hi[u]);
+                        if constexpr (F64) ld_pack(ph + (e[u] >> C::HB), lo[u], hi[u]);
                         else {
-                            lo[u] = ld_pair(ph + (e[u] >> 10));
+                            lo[u] = ld_pair(ph + (e[u] >> C::HB));
                             hi[u] = lo[u] >> 32;
                         }
                     }
 #pragma unroll
                 for (int u = 0; u < MI; u++)
                     if ((pend >> u & 1u) && (unsigned)hi[u] == tag) {
-                        if constexpr (F64) phi[e[u] & 1023u] = __longlong_as_double((long long)lo[u]);
-                        else phi[e[u] & 1023u] = __uint_as_float((unsigned)lo[u]);
+                        if constexpr (F64) phi[e[u] & ((1u << C::HB) - 1u)] = __longlong_as_double((long long)lo[u]);
+                        else phi[e[u] & ((1u << C::HB) - 1u)] = __uint_as_float((unsigned)lo[u]);
                         pend &= ~(1u << u);
                     }
                 if (pend && ++spins > SPIN_LIMIT) {
@@ -438,11 +439,11 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
                 unsigned long long lo[MI], hi[MI];
 #pragma unroll
                 for (int u = 0; u < MI; u++)
-                    if (pend >> u & 1u) ld_pack(pk + (size_t)(e[u] >> 13) * PK + (tid + u * NT) % PK, lo[u], hi[u]);
+                    if (pend >> u & 1u) ld_pack(pk + (size_t)(e[u] >> C::EB) * PK + (tid + u * NT) % PK, lo[u], hi[u]);
 #pragma unroll
                 for (int u = 0; u < MI; u++)
                     if ((pend >> u & 1u) && (unsigned)hi[u] == tag) {
-                        S *const d = pop + (e[u] & 8191u);
+                        S *const d = pop + (e[u] & ((1u << C::EB) - 1u));
                         if constexpr (F64) d[((tid + u * NT) % PK) * NP * PS] = __longlong_as_double((long long)lo[u]);
                         else {
                             d[0] = __uint_as_float((unsigned)lo[u]);
@@ -503,6 +504,12 @@ struct Entry {
             cudaGetLastError();
             return 0;
         }
+        // the packed table entries hold so many slots
+        int d = 0, sms = 1;
+        cudaGetDevice(&d);
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, d);
+        const long long most = std::min((1ll << (32 - C::EB)) / C::NPK, (1ll << (32 - C::HB)) / C::NODES);
+        while (n > 0 && (long long)n * sms > most) n--;
         return n;
     }
     static cudaError_t launch(const ResArgs &a, int grid, cudaStream_t st) {
@@ -528,6 +535,9 @@ struct Entry {
     switch (shape) {                                             \
         case RES_64: return Entry<double, false, RES_64>::what;   \
         case RES_128: return Entry<double, false, RES_128>::what; \
+        case RES_160: return Entry<double, false, RES_160>::what; \
+        case RES_192: return Entry<double, false, RES_192>::what; \
+        case RES_224: return Entry<double, false, RES_224>::what; \
         case RES_256: return Entry<double, false, RES_256>::what; \
     }
 int res_occupancy_f64(int prec, int shape) {
@@ -544,6 +554,7 @@ cudaError_t res_launch_f64(int prec, int shape, const ResArgs &a, int grid, cuda
         case RES_64: return Entry<float, false, RES_64>::what;           \
         case RES_128: return Entry<float, false, RES_128>::what;         \
         case RES_256: return Entry<float, false, RES_256>::what;         \
+        case RES_256x2: return Entry<float, false, RES_256x2>::what;     \
         case RES_256D: return Entry<float, false, RES_256D>::what;       \
     }                                                                    \
     else switch (shape) {                                                \
@@ -551,7 +562,7 @@ cudaError_t res_launch_f64(int prec, int shape, const ResArgs &a, int grid, cuda
         case RES_128: return Entry<float, true, RES_128>::what;          \
         case RES_256: return Entry<float, true, RES_256>::what;          \
         case RES_256x2: return Entry<float, true, RES_256x2>::what;      \
-        case RES_256x2D: return Entry<float, true, RES_256x2D>::what;    \
+        case RES_256x4: return Entry<float, true, RES_256x4>::what;    \
     }
 int res_occupancy_f32(int prec, int shape) {
     RES_SWITCH(prec, shape, occupancy())

@@ -8,15 +8,18 @@
 
 namespace itlbm {
 
-// Tile configurations, by threads: 64 and 128 with registers to spare (boxes that leave the SMs half empty
-// anyway), 256 for many tiles per SM, and for the box sizes beyond: FP32 with four CTAs per SM instead of
-// three (D), the fold with two nodes per thread (x2), with three and with four CTAs per SM.
-enum { RES_64 = 0, RES_128 = 1, RES_256 = 2, RES_256D = 3, RES_256x2 = 4, RES_256x2D = 5, NRES = 6 };
-__host__ __device__ constexpr int res_threads(int shape) { return shape == RES_64 ? 64 : (shape == RES_128 ? 128 : 256); }
-__host__ __device__ constexpr int res_nodes(int shape) { return shape >= RES_256x2 ? 512 : res_threads(shape); }
-// Largest w + h of a tile of that many nodes: 32 x 16, 32 x 8, 16 x 8, 8 x 8.
+// Tile configurations, by threads: 64, 128 and (FP64) 160, 192 and 224 with registers to spare, for boxes that
+// leave the SMs half empty anyway, 256 for many tiles per SM, with two nodes per thread (x2, the FP32 forms) and, for the box sizes
+// beyond, four (x4, the fold) or four CTAs per SM at 64 registers (D, FP32).
+enum { RES_64 = 0, RES_128, RES_160, RES_192, RES_224, RES_256, RES_256x2, RES_256D, RES_256x4, NRES };
+__host__ __device__ constexpr int res_threads(int shape) {
+    return shape == RES_64 ? 64 : shape == RES_128 ? 128 : shape == RES_160 ? 160 : shape == RES_192 ? 192 : shape == RES_224 ? 224 : 256;
+}
+__host__ __device__ constexpr int res_nodes(int shape) { return shape == RES_256x4 ? 1024 : (shape == RES_256x2 ? 512 : res_threads(shape)); }
+// Largest w + h of a tile of that many nodes: 32 x 32, 32 x 16, 32 x 8, 32 x 7, 24 x 8, 20 x 8, 16 x 8, 8 x 8,
+// a little more for 192 and 160.
 __host__ __device__ constexpr int res_half_perimeter(int nodes) {
-    return nodes == 512 ? 48 : (nodes == 256 ? 40 : (nodes == 128 ? 24 : 16));
+    return nodes == 1024 ? 64 : nodes == 512 ? 48 : nodes == 224 ? 39 : nodes == 192 ? 34 : nodes == 160 ? 30 : (nodes == 256 ? 40 : (nodes == 128 ? 24 : 16));
 }
 
 // A tile of a launch: its case, which of the case's bx x by tiles it is, where the CTAs (exchange slots) of
@@ -54,18 +57,26 @@ struct ResCfg {
     static constexpr int NRING = 4 * WH + 16;          // halo nodes at reach 2
     static constexpr int PK = sizeof(S) == 8 ? 2 : 1;  // packs per exchanged plane: both colours in FP32
     static constexpr int SMEM = (int)sizeof(S) * (2 * NP * PS + PHIN) + 4 * (NPK + NRING) + 2 * NPK;
-    // CTAs per SM the registers are sized for.  Measured on B200: FP32 with three CTAs of 256 threads (80
-    // registers, no spills) runs sweeps of 100 x 100 boxes at 24.0 G updates/s, with four (64, spills) at
-    // 20.6; the fold's P3 410 x 410 with two nodes per thread takes 4.8 us per step with three, 7.3 with four.
+    // CTAs per SM the registers are sized for, measured on B200: FP32 sweeps with one node per thread in three
+    // CTAs of 80 registers run at 24.0 G updates/s (100 x 100 boxes), in four of 64, which spill, at 20.6; two
+    // nodes per thread in two CTAs of 128 registers at 24.3, and 25.5 against 23.2 on 192 x 192 boxes (F2 21.2
+    // against 18.6).  Fold: two nodes in three CTAs 40.7 against 38.2, a 410 x 410 step 4.8 us against 7.3 in
+    // four; four nodes in two CTAs, 500 x 500, 6.4 us against 7.8 for two in four.  FP64: one node in two CTAs of
+    // 128 registers 9.5, two nodes in one CTA 8.8; for a case alone fewer threads of more registers where they
+    // suffice (200 x 200 P3 4.8 us in 160 threads, 5.85 in 256; 230 x 230 F2 7.6 in 192, 8.9 in 256).
     static constexpr bool F64 = sizeof(S) == 8;
     static constexpr int MIN_CTAS = SHAPE == RES_64 ? (F64 ? 4 : 8) : SHAPE == RES_128 ? (F64 ? 2 : 4) :
-                                    F64 ? 2 : ((SHAPE == RES_256 && !FOLD) || SHAPE == RES_256x2) ? 3 : 4;
+                                    F64 ? 2 : SHAPE == RES_256D ? 4 : SHAPE == RES_256x4 ? 2 :
+                                    FOLD ? (SHAPE == RES_256 ? 4 : 3) : (SHAPE == RES_256 ? 3 : 2);
     // The case's parameters in shared memory, or read through the cache where registers are so short that
     // what the compiler then keeps of them is spilled (FP64 sweep 9.2 against 9.6 G updates/s, FP32 380 x 380
     // 6.6 against 6.2 us per step; elsewhere 2 % faster).
     static constexpr bool OWN_CASE = !(SHAPE == RES_256D || (F64 && SHAPE == RES_256));
     static_assert(10 * RING <= 2 * NP * PS, "ring-1 auxiliaries in the planes' place");
-    static_assert(PHIN <= 1024, "element of phi in 10 bits");
+    static constexpr int EB = NP * PS <= 8192 ? 13 : 14;  // bits of an element of a pack
+    static_assert(NP * PS <= 1 << EB, "element of a pack");
+    static constexpr int HB = PHIN <= 1024 ? 10 : 11;     // bits of an element of phi
+    static_assert(PHIN <= 1 << HB, "element of phi");
 };
 
 int res_occupancy_f64(int prec, int shape);

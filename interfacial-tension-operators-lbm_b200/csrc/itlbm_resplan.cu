@@ -103,7 +103,7 @@ ResPlan res_plan_single(int prec, int tipo, int nx, int ny) {
     ResPlan best;
     double least = 0;
     for (int shape = 0; shape < NRES; shape++) {
-        constexpr double factor[NRES] = {1.0, 1.05, 1.3, 1.5, 1.4, 1.6};  // same work per step
+        constexpr double factor[NRES] = {1.0, 1.05, 1.1, 1.15, 1.2, 1.3, 1.4, 1.5, 1.6};  // same work per step
         const int threads = res_threads(shape);
         ResPlan p;
         const double c = factor[shape] * best_tiling(prec, nx, ny, shape, p, [&](int tiles, int w, int h) {
@@ -128,7 +128,7 @@ ResPlan res_plan_single(int prec, int tipo, int nx, int ny) {
 // ones fit side by side, and slightly smaller tiles may fill the same CTAs (fold F2 256 x 256: 24.7 G
 // updates/s in 256 tiles, 27.2 in 296).
 ResPlan res_plan_batch(int prec, int nx, int ny) {
-    for (int shape = RES_256; shape < NRES; shape++) {
+    for (int shape = prec == ITLBM_PREC_F64 ? RES_256 : RES_256x2; shape < NRES; shape++) {
         const int cap = res_capacity(prec, shape);
         ResPlan p;
         best_tiling(prec, nx, ny, shape, p, [&](int tiles, int w, int h) {

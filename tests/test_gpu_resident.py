@@ -46,11 +46,11 @@ def both_ways(itlbm, nx, ny, tipo, prec, n=N, geometry=0, setup=None):
     return got
 
 
-# the smallest sides, odd and thin boxes, one tile across, and the boxes around which the tile
-# configuration changes (64, 128, 256 and 2 x 256 nodes) or the box no longer fits
-BOXES = {0: [(8, 8), (9, 33), (33, 9), (40, 40), (61, 130), (190, 200), (270, 280), (300, 300)],
-         1: [(8, 8), (9, 33), (33, 9), (40, 40), (61, 130), (270, 280), (380, 390), (400, 400)],
-         2: [(8, 8), (9, 33), (33, 9), (40, 40), (61, 130), (270, 280), (380, 390), (540, 550), (570, 560)]}
+# the smallest sides, odd and thin boxes, one tile across, and a box of each tile configuration and one
+# that no longer fits
+BOXES = {0: [(8, 8), (9, 33), (33, 9), (40, 40), (61, 130), (190, 200), (215, 210), (235, 230), (250, 256), (270, 275), (300, 300)],
+         1: [(8, 8), (9, 33), (33, 9), (40, 40), (61, 130), (270, 280), (330, 340), (380, 380), (388, 380), (400, 400)],
+         2: [(8, 8), (9, 33), (33, 9), (40, 40), (61, 130), (270, 280), (380, 390), (460, 470), (540, 550), (570, 560)]}
 
 
 @pytest.mark.parametrize("prec,nx,ny", [(p, *b) for p in BOXES for b in BOXES[p]])

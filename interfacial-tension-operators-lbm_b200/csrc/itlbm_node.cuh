@@ -134,12 +134,16 @@ __device__ __forceinline__ void node_split(const CaseDev::F32Par &pf, const S (&
         st(std::integral_constant<int, 0>{}, f[0]);
         st(std::integral_constant<int, NK>{}, (float)(sbd - dsum));
     } else if constexpr (std::is_same<S, double>::value) {
-        sfor<0, NV>([&](auto I) {
-            constexpr int i = decltype(I)::value;
-            double r, b;
-            split64<i>(rc, f[i], r, b);
+        st(std::integral_constant<int, 0>{}, rc.cR * f[0]);
+        st(std::integral_constant<int, NV>{}, rc.cB * f[0]);
+        sfor<0, 9>([&](auto M) {
+            constexpr int i = 2 * decltype(M)::value + 1;
+            double r, b, rj, bj;
+            split64_pair<i>(rc, f[i], f[i + 1], r, b, rj, bj);
             st(std::integral_constant<int, i>{}, r);
             st(std::integral_constant<int, NV + i>{}, b);
+            st(std::integral_constant<int, i + 1>{}, rj);
+            st(std::integral_constant<int, NV + i + 1>{}, bj);
         });
     } else {
         // d_0 is the complement of the moving d_i against the incoming D, both summed in

@@ -152,18 +152,17 @@ __device__ __forceinline__ double cos_of(const Recolour64 &r, int i) {
     }
 }
 
-// Post-collision colour populations of direction i from the collided total f_i.
+// Post-collision colour populations of the opposite directions i, i + 1 (i odd) from the collided totals
+// fi, fj: their t_i are exact negatives.
 template <int i>
-__device__ __forceinline__ void split64(const Recolour64 &r, double fi, double &fR, double &fB) {
-    if constexpr (i == 0) {
-        fR = r.cR * fi;
-        fB = r.cB * fi;
-    } else {
-        constexpr double w = wgt<double>(i);
-        const double t = ((r.fator * w) * r.rho) * cos_of(r, i);
-        fR = r.cR * fi - t;
-        fB = r.cB * fi + t;
-    }
+__device__ __forceinline__ void split64_pair(const Recolour64 &r, double fi, double fj, double &Ri, double &Bi,
+                                             double &Rj, double &Bj) {
+    const double t = ((r.fator * wgt<double>(i)) * r.rho) * cos_of(r, i);
+    const double a = r.cR * fi, b = r.cB * fi, c = r.cR * fj, d = r.cB * fj;
+    Ri = a - t;
+    Bi = b + t;
+    Rj = c + t;
+    Bj = d - t;
 }
 
 // Guo forcing, BGK relaxation and class-P perturbation of one site (colisao_comum,
@@ -230,19 +229,30 @@ __device__ __forceinline__ void relax_f64(double (&f)[NV], double rho_R, double 
         vF = Fxr * vxa + Fyr * vya + Fzr * vza;
         fac3 = c.src_factor;
     }
-    sfor<0, NV>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        const double cv = cdot<i>(vxa, vya, vza);
+    // by opposite directions (i, i + 1), c_{i+1} = -c_i: c.v and c.F of the second are the exact negatives, and
+    // (0.5 cv) cv 3 = 1.5 (cv cv) to the bit, 0.5 being a power of two
+    {
+        const double feq = (wgt<double>(0) * r) * (1.0 - t_vq);
+        const double op = (feq - f[0]) * inv_tau;
+        f[0] = f[0] + op;
+        if constexpr (FORCE) f[0] = f[0] + ((fac3 * wgt<double>(0)) * 3.0) * (0.0 - vF);
+    }
+    sfor<0, 9>([&](auto M) {
+        constexpr int i = 2 * decltype(M)::value + 1;
         constexpr double w = wgt<double>(i);
-        const double feq = (w * r) * (((1.0 + cv * 3.0) + (((0.5 * cv) * cv) * 3.0) * 3.0) - t_vq);
-        const double op = (feq - f[i]) * inv_tau;
+        const double cv = cdot<i>(vxa, vya, vza);
+        const double c3 = cv * 3.0, q = ((cv * cv) * 1.5) * 3.0, wr = w * r;
+        const double eqi = wr * (((1.0 + c3) + q) - t_vq), eqj = wr * (((1.0 - c3) + q) - t_vq);
+        const double opi = (eqi - f[i]) * inv_tau, opj = (eqj - f[i + 1]) * inv_tau;
         if constexpr (FORCE) {
-            f[i] = f[i] + op + guo_source_f64<i>(fac3, Fxr, Fyr, Fzr, cv, vF);
+            const double cF = cdot<i>(Fxr, Fyr, Fzr), h = (3.0 * cF) * cv, k = (fac3 * w) * 3.0;
+            f[i] = f[i] + opi + k * ((h + cF) - vF);
+            f[i + 1] = f[i + 1] + opj + k * ((h - cF) - vF);
         } else {
-            f[i] = f[i] + op;
+            f[i] = f[i] + opi;
+            f[i + 1] = f[i + 1] + opj;
         }
     });
-
 }
 template <bool FORCE, class D2, class DA, class DB>
 __device__ __forceinline__ void finish_f64_by(double (&f)[NV], double gmx, double gmy, double gmz, double mod2, double mod,
@@ -297,9 +307,11 @@ __device__ __forceinline__ void colisao_site_f64(double (&fR)[NV], double (&fB)[
     if (rc.skip) return;
     gradient_size(gmx, gmy, gmz, rc);
     finish_f64<FORCE>(f, gmx, gmy, gmz, c, rc);
-    sfor<0, NV>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        split64<i>(rc, f[i], fR[i], fB[i]);
+    fR[0] = rc.cR * f[0];
+    fB[0] = rc.cB * f[0];
+    sfor<0, 9>([&](auto M) {
+        constexpr int i = 2 * decltype(M)::value + 1;
+        split64_pair<i>(rc, f[i], f[i + 1], fR[i], fB[i], fR[i + 1], fB[i + 1]);
     });
 }
 

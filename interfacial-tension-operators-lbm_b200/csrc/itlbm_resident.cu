@@ -94,6 +94,24 @@ __device__ __forceinline__ unsigned long long pair_of(unsigned a, unsigned b) {
     return (unsigned long long)a | ((unsigned long long)b << 32);
 }
 
+// Polls of up to MI items a thread: `load(u)` reads item u, `take(u)` uses it if it has come and says so.
+// False when the wait ran out.  (A delay before the first poll changes nothing, several polls under way at once
+// lengthen the wait by the trips of those not needed any more.)
+template <int MI, class LOAD, class TAKE>
+__device__ __forceinline__ bool poll_items(unsigned pend, LOAD load, TAKE take) {
+    if (!pend) return true;
+    for (int spins = 0; spins < SPIN_LIMIT; spins++) {
+#pragma unroll
+        for (int u = 0; u < MI; u++)
+            if (pend >> u & 1u) load(u);
+#pragma unroll
+        for (int u = 0; u < MI; u++)
+            if ((pend >> u & 1u) && take(u)) pend &= ~(1u << u);
+        if (!pend) return true;
+    }
+    return false;
+}
+
 // first coordinate of tile t of n nodes cut into b tiles (res_tiling keeps the product in 32 bits)
 __device__ __forceinline__ int tile_begin(int t, int n, int b) { return (int)((unsigned)t * (unsigned)n / (unsigned)b); }
 
@@ -330,30 +348,24 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
                     pend |= 1u << u;
                 }
             }
-            int spins = 0;
-            while (pend) {
-                unsigned long long lo[MI], hi[MI];
-#pragma unroll
-                for (int u = 0; u < MI; u++)
-                    if (pend >> u & 1u) {
+            unsigned long long lo[MI], hi[MI];
+            if (!poll_items<MI>(
+                    pend,
+                    [&](int u) {
                         if constexpr (F64) ld_pack(ph + (e[u] >> C::HB), lo[u], hi[u]);
                         else {
                             lo[u] = ld_pair(ph + (e[u] >> C::HB));
                             hi[u] = lo[u] >> 32;
                         }
-                    }
-#pragma unroll
-                for (int u = 0; u < MI; u++)
-                    if ((pend >> u & 1u) && (unsigned)hi[u] == tag) {
-                        if constexpr (F64) phi[e[u] & ((1u << C::HB) - 1u)] = __longlong_as_double((long long)lo[u]);
-                        else phi[e[u] & ((1u << C::HB) - 1u)] = __uint_as_float((unsigned)lo[u]);
-                        pend &= ~(1u << u);
-                    }
-                if (pend && ++spins > SPIN_LIMIT) {
-                    bad = 1;
-                    break;
-                }
-            }
+                    },
+                    [&](int u) {
+                        if ((unsigned)hi[u] != tag) return false;
+                        S *const d = phi + (e[u] & ((1u << C::HB) - 1u));
+                        if constexpr (F64) *d = __longlong_as_double((long long)lo[u]);
+                        else *d = __uint_as_float((unsigned)lo[u]);
+                        return true;
+                    }))
+                bad = 1;
         }
         __syncthreads();
 
@@ -434,28 +446,23 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
                 e[u] = j < g.npacks ? rcv[j / PK] : 0xFFFFFFFFu;
                 if (e[u] != 0xFFFFFFFFu) pend |= 1u << u;
             }
-            int spins = 0;
-            while (pend) {
-                unsigned long long lo[MI], hi[MI];
-#pragma unroll
-                for (int u = 0; u < MI; u++)
-                    if (pend >> u & 1u) ld_pack(pk + (size_t)(e[u] >> C::EB) * PK + (tid + u * NT) % PK, lo[u], hi[u]);
-#pragma unroll
-                for (int u = 0; u < MI; u++)
-                    if ((pend >> u & 1u) && (unsigned)hi[u] == tag) {
+            unsigned long long lo[MI], hi[MI];
+            if (!poll_items<MI>(
+                    pend,
+                    [&](int u) {
+                        ld_pack(pk + (size_t)(e[u] >> C::EB) * PK + (tid + u * NT) % PK, lo[u], hi[u]);
+                    },
+                    [&](int u) {
+                        if ((unsigned)hi[u] != tag) return false;
                         S *const d = pop + (e[u] & ((1u << C::EB) - 1u));
                         if constexpr (F64) d[((tid + u * NT) % PK) * NP * PS] = __longlong_as_double((long long)lo[u]);
                         else {
                             d[0] = __uint_as_float((unsigned)lo[u]);
                             d[NP * PS] = __uint_as_float((unsigned)(lo[u] >> 32));
                         }
-                        pend &= ~(1u << u);
-                    }
-                if (pend && ++spins > SPIN_LIMIT) {
-                    bad = 1;
-                    break;
-                }
-            }
+                        return true;
+                    }))
+                bad = 1;
         }
         if (__syncthreads_or(bad)) {
             if (tid == 0) *a.err = 1;

@@ -261,10 +261,26 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
         if (t < w * h) {
             const int ly = t / w, lx = t - ly * w;
             const bool edge = lx < H || lx >= w - H || ly < H || ly >= h - H;
-            me[r] = 0x80000000u | (edge ? 0x40000000u : 0u) | (unsigned)ly;
+            const bool inner = lx > 0 && lx < w - 1 && ly > 0 && ly < h - 1;
+            me[r] = 0x80000000u | (edge ? 0x40000000u : 0u) | (inner ? 0x20000000u : 0u) | (unsigned)ly;
             const S *src = (const S *)c.buf[g.cur0] + node_off(c, g.x0 + lx, g.y0 + ly);
 #pragma unroll
             for (int q = 0; q < 2 * NP; q++) pop[q * PS + PAD + t] = src[q * PLANE];
+        }
+    }
+    // F1 / F2 in FP32: the thread's node of the two outermost layers of the ring-1 region, row << 16 | element: the
+    // nodes that need the halo's rho^N.  The others' gradients are taken while those are on their way.  (B200, us
+    // per step: FP32 F2 333 x 207 4.12 -> 3.94, fold F2 150 x 150 2.85 -> 2.78.  FP64 has too few registers to gain
+    // by it, and where one pass covers the region two are slower: F1 200 x 200 6.45 -> 6.8.)
+    constexpr bool INNER_FIRST = !F64;
+    unsigned rim = 0xFFFFFFFFu;
+    if (INNER_FIRST && (g.tipo == ITLBM_OP_F1 || g.tipo == ITLBM_OP_F2)) {
+        static_assert(4 * C::WH <= NT, "a thread per node of the rim");
+        const int w = g.w, h = g.h, PW = w + 2, r = tid - 4 * PW;
+        if (tid < 4 * (w + h)) {
+            const int j = tid / PW, k = r & 3;
+            const int qy = r < 0 ? (j < 2 ? j : h - 2 + j) : 2 + (r >> 2), qx = r < 0 ? tid - j * PW : (k < 2 ? k : w - 2 + k);
+            rim = (unsigned)qy << 16 | (unsigned)(qy * PW + qx);
         }
     }
     // the node's element of phi, with its halo of two nodes, and of the ring-1 region
@@ -336,6 +352,19 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
             }
         }
 
+        const int tipo = g.tipo, PW = g.w + 2, PP = g.w + 4;
+        const bool force = tipo >= ITLBM_OP_F1, ring = tipo == ITLBM_OP_F1 || tipo == ITLBM_OP_F2;
+        auto ring_node = [&](int q, int at) {
+            const S *p = phi + at;
+            ring_aux_node<S>(the_case(), tipo, [&](int dx, int dy) { return p[dy * PP + dx]; }, ringg + q * 3, ringa + q * AUXS);
+        };
+        if (INNER_FIRST && ring) {
+            __syncthreads();
+#pragma unroll
+            for (int r = 0; r < R; r++)
+                if (me[r] & 0x20000000u) ring_node(ring_el(r), phi_el(r));
+        }
+
         // ---- 2: the halo's rho^N ----------------------------------------------------------------
         {
             constexpr int MI = (C::NRING + NT - 1) / NT;
@@ -371,14 +400,12 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
 
         // ---- 3: gradient, force, collision, push --------------------------------------------------
         const CaseDev &c = the_case();
-        const int tipo = g.tipo, PW = g.w + 2, PP = g.w + 4;
-        const bool force = tipo >= ITLBM_OP_F1, ring = tipo == ITLBM_OP_F1 || tipo == ITLBM_OP_F2;
         if (ring) {
-            const int nq = PW * (g.h + 2), M = (65536 + PW - 1) / PW;  // q / PW by multiply and shift, exact for q < 65536 / PW
-            for (int q = tid; q < nq; q += NT) {
-                const int qy = (q * M) >> 16, qx = q - qy * PW;
-                const S *p = phi + (qy + 1) * PP + qx + 1;
-                ring_aux_node<S>(c, tipo, [&](int dx, int dy) { return p[dy * PP + dx]; }, ringg + q * 3, ringa + q * AUXS);
+            if constexpr (INNER_FIRST) {
+                if (rim != 0xFFFFFFFFu) ring_node((int)(rim & 0xFFFFu), (int)((rim & 0xFFFFu) + (rim >> 16) * 2) + PP + 1);
+            } else {
+                const int nq = PW * (g.h + 2), M = (65536 + PW - 1) / PW;  // q / PW by multiply and shift, exact for q < 65536 / PW
+                for (int q = tid; q < nq; q += NT) ring_node(q, q + ((q * M) >> 16) * 2 + PP + 1);
             }
             __syncthreads();
         }

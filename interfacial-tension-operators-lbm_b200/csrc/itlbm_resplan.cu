@@ -17,7 +17,6 @@ int pk_of(int prec) { return prec == ITLBM_PREC_F64 ? 2 : 1; }
 size_t phi_bytes(int prec) { return prec == ITLBM_PREC_F64 ? 16 : 8; }
 
 constexpr int MAX_DEVICES = 32;
-constexpr long long RING_BALANCED_NODES = 24000;  // see res_plan_single
 struct Device {
     std::once_flag once;
     int sms = 0;
@@ -91,15 +90,15 @@ double best_tiling(int prec, int nx, int ny, int shape, ResPlan &p, COST cost) {
 // sooner (us per step, P3, 64 / 128 / 256 threads: FP64 100^2 3.6 / 3.8 / 5.4, FP32 100^2 2.70 / 2.75 / 3.2,
 // 256^2 3.46 / 3.42 / 3.9, fold 256^2 2.86 / 2.90 / 3.0; k_step 9.1, 6.8, 8.2, 8.2), in the fewest tiles, or
 // with 256 threads in as many as leave the fewest warps on the fullest SM (FP64 200^2 5.96 against 6.20).
-// F1 / F2 also pass over the ring-1 region, a second time when it has more nodes than the CTA threads:
+// FP64 F1 / F2 also pass over the ring-1 region, a second time when it has more nodes than the CTA threads:
 // there the configuration and tiling with the fewest warps on the fullest SM, the region's counted half
-// (a second pass, one more), as long as the SMs are not full: FP64 F2 100^2 4.84 against 5.19, 150^2 5.45 /
-// 6.0, 200^2 7.8 / 9.75, FP32 F2 100^2 3.06 / 3.18; FP32 F2 150^2 the same, 256^2 4.63 / 4.20.
+// (a second pass, one more), as long as the SMs are not full: F2 100^2 4.84 against 5.19, 150^2 5.45 / 6.0,
+// 200^2 7.8 / 9.75.  (FP32 takes the inner nodes of the region while it waits; balanced in the same way
+// 150^2 boxes are slower, F1 3.22 against 3.04, fold F2 2.78 / 2.69, 100^2 ones within 2 %.)
 ResPlan res_plan_single(int prec, int tipo, int nx, int ny) {
     const Device *v = device();
     if (!v) return ResPlan();
-    const bool ring = (tipo == ITLBM_OP_F1 || tipo == ITLBM_OP_F2) &&
-                      (prec == ITLBM_PREC_F64 || (long long)nx * ny <= RING_BALANCED_NODES);
+    const bool ring = (tipo == ITLBM_OP_F1 || tipo == ITLBM_OP_F2) && prec == ITLBM_PREC_F64;
     ResPlan best;
     double least = 0;
     for (int shape = 0; shape < NRES; shape++) {

@@ -93,7 +93,15 @@ __device__ __forceinline__ void node_force(const CaseDev &c, int tipo, const Cas
 template <class S, bool FOLD>
 using Recolour = std::conditional_t<std::is_same<S, double>::value, Recolour64, std::conditional_t<FOLD, RecolourFold, Recolour32>>;
 
-// First part of the collision of a node: f (the totals, or their deviations in FP32) relaxed, from the
+// What the collision takes from the node's populations alone (nothing in the fold: with its few moments apart the
+// compiler contracts other products of the relaxation in one kernel than in the other).
+template <class S, bool FOLD, int NP>
+__device__ __forceinline__ void node_moments(const CaseDev::F32Par &pf, const S (&f)[NP], S sa, S sb, Recolour<S, FOLD> &rc) {
+    if constexpr (std::is_same<S, double>::value) moments_f64(f, rc);
+    else if constexpr (!FOLD) moments_f32(f, sa, sb, pf, rc);
+}
+
+// First part of the collision of a node, after node_moments: f (the totals, or their deviations in FP32) relaxed, from the
 // colour sums and the force.  rc.skip is set, and f left, when rho <= 1e-30: such a site is streamed
 // unchanged (Operadores_tensao.cpp:347).
 template <bool FORCE, class S, bool FOLD, int NP>
@@ -101,7 +109,7 @@ __device__ __forceinline__ void node_relax(const CaseDev &c, const CaseDev::F32P
                                            S Fz, Recolour<S, FOLD> &rc) {
     if constexpr (FOLD) relax_fold<FORCE>(f, sa, sb, Fx, Fy, pf, rc);
     else if constexpr (std::is_same<S, double>::value) relax_f64<FORCE>(f, sa, sb, Fx, Fy, Fz, c, rc);
-    else relax_f32<FORCE>(f, sa, sb, Fx, Fy, Fz, pf, rc);
+    else relax_f32<FORCE>(f, sa, Fx, Fy, Fz, pf, rc);
 }
 
 // Second part, for a node that is not skipped: perturbation and the recolouring's coefficients.

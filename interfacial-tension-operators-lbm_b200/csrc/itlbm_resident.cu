@@ -273,6 +273,9 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
     // per step: FP32 F2 333 x 207 4.12 -> 3.94, fold F2 150 x 150 2.85 -> 2.78.  FP64 has too few registers to gain
     // by it, and where one pass covers the region two are slower: F1 200 x 200 6.45 -> 6.8.)
     constexpr bool INNER_FIRST = !F64;
+    // Class F: the moments too are taken while the halo's rho^N are on their way (FP64 F1 200 x 200 6.45 -> 6.28,
+    // FP32 F2 333 x 207 3.94 -> 3.86).
+    constexpr bool EARLY_MOMENTS = !FOLD;
     unsigned rim = 0xFFFFFFFFu;
     if (INNER_FIRST && (g.tipo == ITLBM_OP_F1 || g.tipo == ITLBM_OP_F2)) {
         static_assert(4 * C::WH <= NT, "a thread per node of the rim");
@@ -343,11 +346,14 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
                 }
 #pragma unroll
                 for (int i = 0; i < NP; i++) f[r][i] = F64 ? va[i] + vb[i] : va[i];
-                if (g.tipo < ITLBM_OP_F1) {  // class P: while the halo's rho^N are on their way
+                // what needs no force, while the halo's rho^N are on their way: for class P the relaxation too
+                if (EARLY_MOMENTS || g.tipo < ITLBM_OP_F1) {
                     const CaseDev &c = the_case();
                     CaseDev::F32Par pf{};
                     if constexpr (!F64) pf = load_pf(c);
-                    node_relax<false, S, FOLD>(c, pf, f[r], sa[r], sb[r], S(0), S(0), S(0), rc[r]);
+                    node_moments<S, FOLD>(pf, f[r], sa[r], sb[r], rc[r]);
+                    if (!EARLY_MOMENTS || g.tipo < ITLBM_OP_F1)
+                        node_relax<false, S, FOLD>(c, pf, f[r], sa[r], sb[r], S(0), S(0), S(0), rc[r]);
                 }
             }
         }
@@ -421,6 +427,7 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
                 node_force<S>(c, tipo, pf, [&](int dx, int dy) { return p[dy * PP + dx]; },
                               [&](int dx, int dy) { return q + (dy * PW + dx) * AUXS; }, ringg + o * 3, gmx[r], gmy[r],
                               gmz[r], Fx[r], Fy[r], Fz[r]);
+                if (!EARLY_MOMENTS && force) node_moments<S, FOLD>(pf, f[r], sa[r], sb[r], rc[r]);
                 if (force) node_relax<true, S, FOLD>(c, pf, f[r], sa[r], sb[r], Fx[r], Fy[r], Fz[r], rc[r]);
             }
         if (ring) __syncthreads();  // the push overwrites the auxiliaries

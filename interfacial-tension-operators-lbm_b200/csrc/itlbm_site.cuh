@@ -122,6 +122,7 @@ struct Recolour64 {
     double cR, cB, frho;   // frho = (beta c_R c_B)... times rho: t_i = (frho_w_i) cos_i
     double fator, rho;
     double mod2, mod;      // |g|^2 and |g| (gradient_size)
+    double r, vx, vy, vz;  // sum f_i and sum c_i f_i / r (moments_f64)
     double k[9];           // cos(phi) of the directions 1, 3, 5, 7, 9, 11, 13, 16, 17
     bool skip;             // rho <= 1e-30: the reference leaves the site unchanged
 };
@@ -165,6 +166,33 @@ __device__ __forceinline__ void split64_pair(const Recolour64 &r, double fi, dou
     Bj = d - t;
 }
 
+// What the collision takes from the totals f_i alone.
+__device__ __forceinline__ void moments_f64(const double (&f)[NV], Recolour64 &rc) {
+    // calcula (LBM_functions.cpp:1100-1171)
+    double r = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
+    sfor<0, NV>([&](auto I) {
+        constexpr int i = decltype(I)::value;
+        r = r + f[i];
+        if constexpr (cx(i) == 1) mx = mx + f[i];
+        if constexpr (cx(i) == -1) mx = mx - f[i];
+        if constexpr (cy(i) == 1) my = my + f[i];
+        if constexpr (cy(i) == -1) my = my - f[i];
+        if constexpr (cz(i) == 1) mz = mz + f[i];
+        if constexpr (cz(i) == -1) mz = mz - f[i];
+    });
+    double vx = 0., vy = 0., vz = 0.;
+    if (r != 0.0) {
+        const double inv = 1.0 / (r);
+        vx = mx * inv;
+        vy = my * inv;
+        vz = mz * inv;
+    }
+    rc.r = r;
+    rc.vx = vx;
+    rc.vy = vy;
+    rc.vz = vz;
+}
+
 // Guo forcing, BGK relaxation and class-P perturbation of one site (colisao_comum,
 // Operadores_tensao.cpp:340-373, and the library functions it calls).  On entry f holds
 // f_i = f_R,i + f_B,i (Operadores_tensao.cpp:360) and rho_R, rho_B the colour sums (density(),
@@ -197,25 +225,7 @@ __device__ __forceinline__ void relax_f64(double (&f)[NV], double rho_R, double 
     }
     rc.cB = 1.0 - rc.cR;
     rc.rho = rho;
-    // calcula (LBM_functions.cpp:1100-1171)
-    double r = 0.0, mx = 0.0, my = 0.0, mz = 0.0;
-    sfor<0, NV>([&](auto I) {
-        constexpr int i = decltype(I)::value;
-        r = r + f[i];
-        if constexpr (cx(i) == 1) mx = mx + f[i];
-        if constexpr (cx(i) == -1) mx = mx - f[i];
-        if constexpr (cy(i) == 1) my = my + f[i];
-        if constexpr (cy(i) == -1) my = my - f[i];
-        if constexpr (cz(i) == 1) mz = mz + f[i];
-        if constexpr (cz(i) == -1) mz = mz - f[i];
-    });
-    double vx = 0., vy = 0., vz = 0.;
-    if (r != 0.0) {
-        const double inv = 1.0 / (r);
-        vx = mx * inv;
-        vy = my * inv;
-        vz = mz * inv;
-    }
+    const double r = rc.r, vx = rc.vx, vy = rc.vy, vz = rc.vz;
     const double vxa = vx + 0.5 * ax, vya = vy + 0.5 * ay, vza = vz + 0.5 * az;
     // dist_eq (LBM_functions.cpp:890-945) and source (LBM_functions.cpp:1603-1673)
     const double vquad = (vxa * vxa + vya * vya + vza * vza);
@@ -303,6 +313,7 @@ __device__ __forceinline__ void colisao_site_f64(double (&fR)[NV], double (&fB)[
 #pragma unroll
     for (int i = 0; i < NV; i++) f[i] = fR[i] + fB[i];
     Recolour64 rc;
+    moments_f64(f, rc);
     relax_f64<FORCE>(f, sa, sb, Fx, Fy, Fz, c, rc);
     if (rc.skip) return;
     gradient_size(gmx, gmy, gmz, rc);
@@ -379,6 +390,7 @@ __device__ __forceinline__ T cdotp(T a, T b, T c3) {  // c_i . (a, b, c3), non-z
 // d_0 is the complement D - sum_{i>=1} d_i, formed by the step kernel with FP64 sums.
 struct Recolour32 {
     float phi, rho, k1, k2, gx, gy, gz;
+    float inv_rho, jx, jy, jz;  // 1 / rho and the momentum of the deviations (moments_f32)
     bool skip;
 };
 
@@ -392,23 +404,14 @@ __device__ __forceinline__ void split32_pair(const Recolour32 &r, float ei, floa
     dj = fmaf(r.phi, __fmaf_rn(wgt<float>(i), Sj, ej), K);
 }
 
-// e_i = f_i - s_i in, post-collision e_i out; drho = sum e_i, D = sum d_i = rho_R - rho_B.
-template <bool FORCE>
-__device__ __forceinline__ void relax_f32(float (&e)[NV], float drho, float D, float Fx, float Fy, float Fz,
-                                          const CaseDev::F32Par &p, Recolour32 &rc) {
-    const float rho0 = p.rho0;
-    const float rho = rho0 + drho;
+// What the collision takes from the populations alone: e_i = f_i - s_i, drho = sum e_i, D = sum d_i = rho_R - rho_B.
+__device__ __forceinline__ void moments_f32(const float (&e)[NV], float drho, float D, const CaseDev::F32Par &p,
+                                            Recolour32 &rc) {
+    const float rho = p.rho0 + drho;
     rc.skip = !(rho > 1.0e-30f);
-    if (rc.skip) return;
-    const float inv_rho = 1.0f / rho;
-    rc.phi = D * inv_rho;  // rho^N = (rho_R - rho_B) / rho
+    rc.inv_rho = 1.0f / rho;
+    rc.phi = D * rc.inv_rho;  // rho^N = (rho_R - rho_B) / rho
     rc.rho = rho;
-    float ax = 0.f, ay = 0.f, az = 0.f;
-    if constexpr (FORCE) {
-        ax = Fx * inv_rho;
-        ay = Fy * inv_rho;
-        az = Fz * inv_rho;
-    }
     float jx = 0.f, jy = 0.f, jz = 0.f;
     sfor<0, 9>([&](auto M) {
         constexpr int i = 2 * decltype(M)::value + 1;
@@ -420,6 +423,22 @@ __device__ __forceinline__ void relax_f32(float (&e)[NV], float drho, float D, f
         if constexpr (cz(i) == 1) jz += p;
         if constexpr (cz(i) == -1) jz -= p;
     });
+    rc.jx = jx;
+    rc.jy = jy;
+    rc.jz = jz;
+}
+// e_i in, relaxed e_i out.
+template <bool FORCE>
+__device__ __forceinline__ void relax_f32(float (&e)[NV], float drho, float Fx, float Fy, float Fz,
+                                          const CaseDev::F32Par &p, Recolour32 &rc) {
+    if (rc.skip) return;
+    const float rho = rc.rho, inv_rho = rc.inv_rho, jx = rc.jx, jy = rc.jy, jz = rc.jz;
+    float ax = 0.f, ay = 0.f, az = 0.f;
+    if constexpr (FORCE) {
+        ax = Fx * inv_rho;
+        ay = Fy * inv_rho;
+        az = Fz * inv_rho;
+    }
     // Delta = sum c_i e_i + F / 2 and the velocity u* = (rho0 U0 + Delta) / rho
     const float Dx = FORCE ? fmaf(0.5f, Fx, jx) : jx, Dy = FORCE ? fmaf(0.5f, Fy, jy) : jy;
     const float Dz = FORCE ? fmaf(0.5f, Fz, jz) : jz;

@@ -251,6 +251,7 @@ __device__ __forceinline__ void step_tile(const CaseDev &c, int tile, int k, int
         const bool force = tipo >= ITLBM_OP_F1;
         Recolour<S, FOLD> rc;
         if constexpr (std::is_same<S, double>::value) gradient_size(gmx, gmy, gmz, rc);
+        node_moments<S, FOLD>(pf, f[jr], sa[jr], sb[jr], rc);
         if (force) {
             node_relax<true, S, FOLD>(c, pf, f[jr], sa[jr], sb[jr], Fx, Fy, Fz, rc);
             if (!rc.skip) node_finish<true, S, FOLD>(c, pf, f[jr], sa[jr], gmx, gmy, gmz, rc);

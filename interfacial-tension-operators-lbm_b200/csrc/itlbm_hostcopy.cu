@@ -20,17 +20,21 @@ namespace itlbm {
 
 namespace {
 
-constexpr size_t CHUNK = (size_t)2 << 20;
-constexpr int SLOTS = 8;      // chunks in flight: at most 16 MB pinned for the process
+constexpr int SLOTS = 8;      // chunks in flight
 constexpr int WORKERS = 8;
-constexpr size_t SMALL = (size_t)4 << 20;  // up to this in one copy, by the calling thread
+// Pinned memory is dear to allocate, and a program that reads each case once pays for it each time: 1 MB is had from
+// what the driver holds, 4 MB take 2 to 5 ms, 16 MB 11 ms.  So small reads take 1 MB, and what large ones take
+// grows with what they save: the first read of five fields of 1024 x 768 takes 4 to 7 ms (plain 8.5, with 16 MB 10
+// to 18), further ones 1.6; of 2048 x 2048 25 and 11 ms (plain 37; with 4 MB 18 and 13).
+constexpr size_t SMALL = (size_t)1 << 20;  // up to this in one copy, by the calling thread
+constexpr size_t HUGE_READ = (size_t)64 << 20, MEDIUM_STAGE = (size_t)4 << 20, HUGE_STAGE = (size_t)16 << 20;
 // From this on in chunks.  Between the two the plain copies: their arrays still come from the host
 // allocator's own pages, and the threads cost more than they save (five fields of 512 x 512, 10.5 MB:
 // 0.69 ms plain, 1.0 ms in chunks; of 1024 x 768, 31 MB: 8.5 and 2.2 ms).
 constexpr size_t LARGE = (size_t)16 << 20;
 
 // The pinned memory, shared by all cases and batches and used by one call at a time (a second call
-// meanwhile takes the plain copy); it grows to what calls need and is freed with the last of them.
+// meanwhile takes the plain copy); it grows to what calls need, at most 16 MB, and is freed with the last of them.
 struct Stage {
     std::mutex lock;
     char *buf = nullptr;
@@ -45,13 +49,12 @@ bool reserve(size_t bytes) {
     if (g_stage.buf) cudaFreeHost(g_stage.buf);
     g_stage.buf = nullptr;
     g_stage.cap = 0;
-    const size_t cap = bytes <= (1u << 20) ? (1u << 20) : (bytes <= SMALL ? SMALL : CHUNK * SLOTS);
-    if (cudaHostAlloc((void **)&g_stage.buf, cap, cudaHostAllocPortable) != cudaSuccess) {
+    if (cudaHostAlloc((void **)&g_stage.buf, bytes, cudaHostAllocPortable) != cudaSuccess) {
         cudaGetLastError();
         g_stage.buf = nullptr;
         return false;
     }
-    g_stage.cap = cap;
+    g_stage.cap = bytes;
     return true;
 }
 
@@ -86,7 +89,7 @@ cudaError_t fetch_large(const std::vector<Chunk> &chunks, cudaStream_t st) {
     cudaError_t e = cudaSuccess;
     for (auto &v : ev)
         if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
-    const size_t n = chunks.size();
+    const size_t n = chunks.size(), slot = g_stage.cap / SLOTS;
     std::mutex m;
     std::condition_variable cv;
     size_t issued = 0, next = 0;
@@ -106,7 +109,7 @@ cudaError_t fetch_large(const std::vector<Chunk> &chunks, cudaStream_t st) {
             if (issued <= c) return;
             g.unlock();
             const cudaError_t w = cudaEventSynchronize(ev[c % SLOTS]);
-            if (w == cudaSuccess) std::memcpy(chunks[c].dst, g_stage.buf + (c % SLOTS) * CHUNK, chunks[c].bytes);
+            if (w == cudaSuccess) std::memcpy(chunks[c].dst, g_stage.buf + (c % SLOTS) * slot, chunks[c].bytes);
             g.lock();
             if (w != cudaSuccess) worker_error = w;
             done[c] = 1;
@@ -132,7 +135,7 @@ cudaError_t fetch_large(const std::vector<Chunk> &chunks, cudaStream_t st) {
             std::unique_lock<std::mutex> g(m);
             if (c >= SLOTS) cv.wait(g, [&] { return done[c - SLOTS] != 0; });
         }
-        e = cudaMemcpyAsync(g_stage.buf + (c % SLOTS) * CHUNK, chunks[c].src, chunks[c].bytes, cudaMemcpyDeviceToHost, st);
+        e = cudaMemcpyAsync(g_stage.buf + (c % SLOTS) * slot, chunks[c].src, chunks[c].bytes, cudaMemcpyDeviceToHost, st);
         if (e == cudaSuccess) e = cudaEventRecord(ev[c % SLOTS], st);
         if (e != cudaSuccess) break;
         std::lock_guard<std::mutex> g(m);
@@ -175,15 +178,16 @@ cudaError_t fetch_arrays(double *const *dst, int n, size_t each, const double *s
     std::unique_lock<std::mutex> g(g_stage.lock, std::try_to_lock);
     if (!g.owns_lock()) return fetch_plain(dst, n, each, src, st);
     if (whole <= SMALL) {
-        if (!reserve(whole)) return fetch_plain(dst, n, each, src, st);
+        if (!reserve(SMALL)) return fetch_plain(dst, n, each, src, st);
         return fetch_small(dst, n, each, src, st);
     }
-    if (total < LARGE || !reserve(CHUNK * SLOTS)) return fetch_plain(dst, n, each, src, st);
+    if (total < LARGE || !reserve(total < HUGE_READ ? MEDIUM_STAGE : HUGE_STAGE)) return fetch_plain(dst, n, each, src, st);
+    const size_t most = g_stage.cap / SLOTS;
     std::vector<Chunk> chunks;
     for (int k = 0; k < n; k++)
-        for (size_t at = 0; dst[k] && at < sizeof(double) * each; at += CHUNK)
+        for (size_t at = 0; dst[k] && at < sizeof(double) * each; at += most)
             chunks.push_back(Chunk{(char *)dst[k] + at, (const char *)(src + k * each) + at,
-                                   std::min(CHUNK, sizeof(double) * each - at)});
+                                   std::min(most, sizeof(double) * each - at)});
     const cudaError_t e = fetch_large(chunks, st);
     return e == cudaErrorNotReady ? fetch_plain(dst, n, each, src, st) : e;
 }

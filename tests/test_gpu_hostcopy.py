@@ -25,8 +25,8 @@ def moments(fR, fB):
     return out
 
 
-# in one copy up to 4 MB (313 x 335 fields: 4.19 MB), plainly up to 16 MB, in chunks of 2 MB beyond
-@pytest.mark.parametrize("nx,ny", [(8, 8), (313, 334), (313, 335), (640, 655), (656, 655), (1031, 517)])
+# in one copy up to 1 MB, plainly up to 16 MB, in chunks of 512 kB up to 64 MB and of 2 MB beyond
+@pytest.mark.parametrize("nx,ny", [(8, 8), (160, 163), (160, 165), (313, 335), (640, 655), (656, 655), (1031, 517), (1290, 1310)])
 def test_fields_of_every_size(gpu, nx, ny):
     with make(gpu, nx, ny) as c:
         c.step(2, keep_aux=True)

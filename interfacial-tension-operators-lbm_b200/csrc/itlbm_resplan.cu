@@ -126,13 +126,27 @@ ResPlan res_plan_single(int prec, int tipo, int nx, int ny) {
 // Small cases fill what larger ones leave; of one that takes more than a sixth of the CTAs only whole
 // ones fit side by side, and slightly smaller tiles may fill the same CTAs (fold F2 256 x 256: 24.7 G
 // updates/s in 256 tiles, 27.2 in 296).
+// An FP64 case of which only one fits at a time in tiles of 256 threads takes the smallest configuration that
+// holds it, as a case alone does (sweeps of twelve boxes of 200 to 256 nodes a side 38.7 -> 31.3 ms, P3 36.2 ->
+// 28.5); smaller ones gain more by company (60 to 200 nodes a side in 160 or 192 threads 20.5 ms, in 256 16.2), and
+// so do the FP32 forms (12 x 200 to 330: two nodes a thread 22.3 ms, one 23.8).
 ResPlan res_plan_batch(int prec, int nx, int ny) {
-    for (int shape = prec == ITLBM_PREC_F64 ? RES_256 : RES_256x2; shape < NRES; shape++) {
+    auto plan = [&](int shape) {
         const int cap = res_capacity(prec, shape);
         ResPlan p;
         best_tiling(prec, nx, ny, shape, p, [&](int tiles, int w, int h) {
             return (10 + up(w * h, 32)) / (6 * tiles <= cap ? (double)cap / tiles : (double)(cap / tiles));
         });
+        return p;
+    };
+    const int first = prec == ITLBM_PREC_F64 ? RES_256 : RES_256x2;
+    if (prec == ITLBM_PREC_F64 && 2 * (long long)nx * ny > (long long)res_capacity(prec, RES_256) * res_nodes(RES_256))
+        for (int shape = RES_160; shape < RES_256; shape++) {
+            const ResPlan p = plan(shape);
+            if (p.shape >= 0) return p;
+        }
+    for (int shape = first; shape < NRES; shape++) {
+        const ResPlan p = plan(shape);
         if (p.shape >= 0) return p;
     }
     return ResPlan();

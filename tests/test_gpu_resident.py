@@ -142,3 +142,28 @@ def test_threads_and_streams(gpu):
     assert not wrong, wrong
     for a, b in zip(want, got):
         assert same(a, b)
+
+
+def test_batch_of_large_boxes(gpu):
+    """FP64 boxes on both sides of the size from which a batch takes them one at a time, in each configuration."""
+    boxes = [(194, 194, 12), (195, 196, 3), (230, 229, 11), (256, 250, 13), (60, 50, 1)]
+
+    def desc(nx, ny, t):
+        return gpu.desc(nx, ny, gpu.make_op(t, 0.5), tau=0.83, A_fact=0.2 if t < 11 else 0.08, radius=0.23 * min(nx, ny))
+
+    with gpu.Batch() as b:
+        b.hold_finished(True)
+        for tag, box in enumerate(boxes):
+            b.submit(desc(*box), 14, tag)
+        while b.stats().finished < len(boxes):
+            b.advance()
+            b.poll()
+        for tag, (nx, ny, t) in enumerate(boxes):
+            got = b.read_fields(tag, nx * ny, gpu.FIELDS_VTK)
+            with gpu.Case(desc(nx, ny, t)) as c:
+                for _ in range(13):
+                    c.step(1)
+                c.step(1, keep_aux=True)
+                want = c.read_fields()
+            assert all(np.array_equal(got[k], want[k]) for k in want), tag
+            b.release(tag)

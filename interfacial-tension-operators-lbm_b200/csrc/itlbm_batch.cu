@@ -246,8 +246,6 @@ int build_resident(itlbm_batch *b) {
             }
             if ((e = res_queues_upload(X.args, q, X.queues, b->stream)) != cudaSuccess)
                 return cuda_fail(e, "resident tile queues");
-            // the copies read q, and pageable copies may return before they are done
-            if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) return cuda_fail(e, "resident tile queues");
             X.ctas = ctas;
             X.cases = (int)cs.size();
         }

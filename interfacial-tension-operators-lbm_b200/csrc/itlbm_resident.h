@@ -121,7 +121,8 @@ struct ResQueues {
     size_t bytes() const { return sizeof(ResTile) * tiles.size() + sizeof(int) * (first.size() + slots.size()); }
 };
 ResQueues res_queues(const std::vector<ResCase> &cases, int ctas);
-// The queues copied to device memory of bytes() bytes, on a stream, and bound to the launch arguments.
+// The queues copied to device memory of bytes() bytes, on a stream that is then waited for, and bound to the
+// launch arguments.
 cudaError_t res_queues_upload(ResArgs &a, const ResQueues &q, void *mem, cudaStream_t st);
 // Bytes of exchange memory for `slots` CTAs, and its binding in a block of that many bytes.
 size_t res_exchange_bytes(int prec, int shape, int slots);

@@ -4,6 +4,7 @@
 
 #include <algorithm>
 #include <cstdlib>
+#include <cstring>
 #include <mutex>
 
 namespace itlbm {
@@ -63,23 +64,29 @@ double best_tiling(int prec, int nx, int ny, int shape, ResPlan &p, COST cost) {
     int size = 0, edge = 0;
     p = ResPlan();
     if (nx < RES_MIN_SIDE || ny < RES_MIN_SIDE || (long long)nx * ny > (long long)cap * nodes) return 0;
-    // tiles at least HMAX wide, so that a halo lies in the tiles beside; begins of tiles in 32 bits
-    for (int bx = 1; bx <= nx / HMAX && bx <= std::min(cap, 65535) && (long long)bx * nx < 1LL << 31; bx++) {
+    // Tiles at least HMAX wide, so that a halo lies in the tiles beside; begins of tiles in 32 bits.  Of the counts
+    // that give the same largest tile only the smallest is looked at (the cost does not fall with the tiles): a
+    // 256 x 256 F2 box took 0.4 ms over all of them, a case's creation in all 1.3.
+    for (int bx = 1; bx <= nx / HMAX && bx <= std::min(cap, 65535) && (long long)bx * nx < 1LL << 31;) {
         const int w = up(nx, bx), hmax = std::min(nodes / w, wh - w);
-        if (hmax < HMAX) continue;
-        for (int by = up(ny, hmax); by <= std::min(ny / HMAX, cap / bx) && by <= 65535 && (long long)by * ny < 1LL << 31; by++) {
-            const int h = up(ny, by);
-            const double v = cost(bx * by, w, h);
-            if (p.shape < 0 || v < least || (v == least && (w * h < size || (w * h == size && w + h < edge)))) {
-                least = v;
-                size = w * h;
-                edge = w + h;
-                p.shape = shape;
-                p.bx = bx;
-                p.by = by;
-                p.tiles = bx * by;
+        if (hmax >= HMAX)
+            for (int by = up(ny, hmax); by <= std::min(ny / HMAX, cap / bx) && by <= 65535 && (long long)by * ny < 1LL << 31;) {
+                const int h = up(ny, by);
+                const double v = cost(bx * by, w, h);
+                if (p.shape < 0 || v < least || (v == least && (w * h < size || (w * h == size && w + h < edge)))) {
+                    least = v;
+                    size = w * h;
+                    edge = w + h;
+                    p.shape = shape;
+                    p.bx = bx;
+                    p.by = by;
+                    p.tiles = bx * by;
+                }
+                if (h == 1) break;
+                by = up(ny, h - 1);
             }
-        }
+        if (w == 1) break;
+        bx = up(nx, w - 1);
     }
     return least;
 }
@@ -180,16 +187,20 @@ ResQueues res_queues(const std::vector<ResCase> &cases, int ctas) {
 }
 
 cudaError_t res_queues_upload(ResArgs &a, const ResQueues &q, void *mem, cudaStream_t st) {
-    char *p = (char *)mem;
-    a.tiles = (const ResTile *)p;
-    cudaError_t e = cudaMemcpyAsync(p, q.tiles.data(), sizeof(ResTile) * q.tiles.size(), cudaMemcpyHostToDevice, st);
-    p += sizeof(ResTile) * q.tiles.size();
-    a.first = (const int *)p;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(p, q.first.data(), sizeof(int) * q.first.size(), cudaMemcpyHostToDevice, st);
-    p += sizeof(int) * q.first.size();
-    a.slots = (const int *)p;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(p, q.slots.data(), sizeof(int) * q.slots.size(), cudaMemcpyHostToDevice, st);
-    return e;
+    std::vector<char> all(q.bytes());
+    size_t at = 0;
+    auto put = [&](const void *src, size_t n) {
+        const size_t o = at;
+        std::memcpy(all.data() + at, src, n);
+        at += n;
+        return (char *)mem + o;
+    };
+    a.tiles = (const ResTile *)put(q.tiles.data(), sizeof(ResTile) * q.tiles.size());
+    a.first = (const int *)put(q.first.data(), sizeof(int) * q.first.size());
+    a.slots = (const int *)put(q.slots.data(), sizeof(int) * q.slots.size());
+    const cudaError_t e = cudaMemcpyAsync(mem, all.data(), at, cudaMemcpyHostToDevice, st);
+    const cudaError_t w = cudaStreamSynchronize(st);  // pageable copies may return before they have read
+    return e == cudaSuccess ? w : e;
 }
 
 size_t res_exchange_bytes(int prec, int shape, int slots) {

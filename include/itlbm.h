@@ -230,7 +230,7 @@ int  itlbm_snapshot_info(const char *path, itlbm_case_desc *desc, long long *ste
 /* ---- batches: many cases stepped together ------------------------------------------------- */
 /* The batched form of the loop Imm_OPS.cpp:246-372 / Imm_INCL.cpp:358-442 for many independent
  * cases, replacing the process pool of rodar_lote.py (rodar_lote.py:231-243, :300-318).  Admitted
- * cases keep their state on the device; each advance runs a CUDA graph of persistent step launches
+ * cases keep their state on the device; each advance runs the resident kernel or a CUDA graph of step launches
  * over a device-resident tile work table (every case's tiles, FP32 and FP64 cases side by side),
  * stops every case at its next diagnostic step (every 500 steps and the last, Imm_OPS.cpp:293),
  * measures it there and retires it at its step count or when it becomes unstable

@@ -123,7 +123,8 @@ struct itlbm_batch {
     bool tables_dirty = true;
     // resident launches of the current tables, one per storage form and tile configuration (none when the
     // caller fixed the launch shape or tiling, or in a replay too short for them)
-    bool resident_ok = false, resident_on = false;
+    bool resident_ok = false;
+    int resident_steps = 0;  // replays the tables are built for: of at least so many sub-steps (0: no resident launches)
     struct Resident {
         void *queues = nullptr, *mem = nullptr;  // queues and exchange memory (device)
         size_t cap = 0;
@@ -205,6 +206,9 @@ void set_grids(itlbm_batch *b) {
     }
 }
 
+// Whether a storage form's cases take the resident kernel in the replay the tables are built for.
+bool resident_form(const itlbm_batch *b, int prec) { return b->resident_steps >= res_min_replay(prec); }
+
 // The resident launches of the active cases: per storage form and configuration the cases with the most
 // tiles first (they need the most CTAs at once; the small ones fill what those leave), in queues over all
 // the CTAs the device holds.
@@ -215,7 +219,7 @@ int build_resident(itlbm_batch *b) {
             const int prec = prec_of_table(pi * NSHAPE);
             std::vector<ResCase> cs;
             X.ctas = X.cases = 0;
-            if (!b->resident_on) continue;
+            if (!resident_form(b, prec)) continue;
             for (const Active *a : b->slots)
                 if (a && !a->held && a->desc.precision == prec && a->plan.shape == shape)
                     // a tile of F1 / F2 takes about 1.3 times as long per step as the others
@@ -255,11 +259,12 @@ int build_resident(itlbm_batch *b) {
 int upload_tables(itlbm_batch *b) {
     std::vector<TileRef> t[NTAB];
     if (build_resident(b) != ITLBM_OK) {  // no room for the exchange memory: every case from the work tables
-        b->resident_on = b->resident_ok = false;
+        b->resident_ok = false;
+        b->resident_steps = 0;
         build_resident(b);
     }
     for (Active *a : b->slots) {
-        if (!a || a->held || (b->resident_on && a->plan.shape >= 0)) continue;
+        if (!a || a->held || (resident_form(b, a->desc.precision) && a->plan.shape >= 0)) continue;
         const CaseDev &c = b->h_cases[a->slot];
         case_tiles(c, b->narrow, a->slot, &t[table_of(a->desc.precision) * NSHAPE]);
     }
@@ -1025,15 +1030,17 @@ int itlbm_batch_advance(itlbm_batch *b, void *stream) {
     cudaError_t e = cudaMemcpyAsync(b->d_cases, b->h_cases.data(), sizeof(CaseDev) * (size_t)(hi + 1),
                                     cudaMemcpyHostToDevice, b->stream);
     if (e != cudaSuccess) return cuda_fail(e, "case table upload");
-    const bool resident = b->resident_ok && K >= RES_MIN_STEPS;
-    if (b->tables_dirty || resident != b->resident_on) {
+    int resident = 0;
+    for (int prec : {ITLBM_PREC_F64, ITLBM_PREC_F32, ITLBM_PREC_F32_FOLD})
+        if (b->resident_ok && K >= res_min_replay(prec)) resident = std::max(resident, res_min_replay(prec));
+    if (b->tables_dirty || resident != b->resident_steps) {
         TileRef *old[NTAB];
         int g[NTAB];
         for (int p = 0; p < NTAB; p++) {
             old[p] = b->d_tiles[p];
             g[p] = b->grid[p];
         }
-        b->resident_on = resident;
+        b->resident_steps = resident;
         r = upload_tables(b);
         if (r) return r;
         for (int p = 0; p < NTAB; p++)

@@ -97,6 +97,12 @@ inline cudaError_t res_launch(int prec, int shape, const ResArgs &a, int grid, c
 // 39 / 29 us; 6 steps: 76 / 64, 46 / 42, 56 / 34 us.
 constexpr int RES_MIN_STEPS = 6;
 constexpr int RES_MAX_STEPS = 4096;
+// Sub-steps a batch's replay must have: its tables keep the GPU busy with k_step, and a resident tile's first loads
+// and tables are hidden by nothing.  Tables / resident, G updates/s, 150 mixed cases of 64 to 512 nodes a side and 100
+// of 64 to 256: FP64 10 steps 7.25 / 6.85 and 6.4 / 5.7, 20 steps 7.25 / 7.24 and 6.4 / 6.7; FP32 20 steps 14.8 / 15.0
+// and 12.8 / 15.4 (600 cases 15.2 / 14.9), 40 steps 14.5 / 16.4 and 12.8 / 17.2; fold 20 steps 28.9 / 25.7 and
+// 24.3 / 25.9, 40 steps 28.9 / 28.8 and 24.2 / 27.4, 80 steps 28.0 / 30.7 and 24.3 / 30.4.
+inline int res_min_replay(int prec) { return prec == ITLBM_PREC_F32_FOLD ? 40 : 24; }
 
 
 // How a case is held on chip: the tile configuration and the bx x by tiles, or shape < 0 when the box

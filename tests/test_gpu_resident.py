@@ -154,14 +154,42 @@ def test_batch_of_large_boxes(gpu):
     with gpu.Batch() as b:
         b.hold_finished(True)
         for tag, box in enumerate(boxes):
-            b.submit(desc(*box), 14, tag)
+            b.submit(desc(*box), 44, tag)
         while b.stats().finished < len(boxes):
             b.advance()
             b.poll()
         for tag, (nx, ny, t) in enumerate(boxes):
             got = b.read_fields(tag, nx * ny, gpu.FIELDS_VTK)
             with gpu.Case(desc(nx, ny, t)) as c:
-                for _ in range(13):
+                for _ in range(43):
+                    c.step(1)
+                c.step(1, keep_aux=True)
+                want = c.read_fields()
+            assert all(np.array_equal(got[k], want[k]) for k in want), tag
+            b.release(tag)
+
+
+@pytest.mark.parametrize("steps", [24, 25, 26, 40, 41, 42])
+def test_short_replays(gpu, steps):
+    """A batch of all storage forms at the replay lengths from which each takes the resident kernel (the replay after
+    the first step has steps - 1 sub-steps)."""
+    boxes = [(50, 40, 12, 0), (61, 70, 3, 1), (90, 40, 11, 2)]
+
+    def desc(nx, ny, t, prec):
+        return gpu.desc(nx, ny, gpu.make_op(t, 0.5), tau=0.83, A_fact=0.2 if t < 11 else 0.08, radius=0.23 * min(nx, ny),
+                        precision=prec)
+
+    with gpu.Batch() as b:
+        b.hold_finished(True)
+        for tag, box in enumerate(boxes):
+            b.submit(desc(*box), steps, tag)
+        while b.stats().finished < len(boxes):
+            b.advance()
+            b.poll()
+        for tag, box in enumerate(boxes):
+            got = b.read_fields(tag, box[0] * box[1], gpu.FIELDS_VTK)
+            with gpu.Case(desc(*box)) as c:
+                for _ in range(steps - 1):
                     c.step(1)
                 c.step(1, keep_aux=True)
                 want = c.read_fields()

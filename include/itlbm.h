@@ -154,6 +154,14 @@ int  itlbm_case_step(itlbm_case *c, int nsteps, int flags, void *stream);
 int  itlbm_case_sync(itlbm_case *c);
 long long itlbm_case_steps_done(const itlbm_case *c);
 
+/* No counterpart in the reference.  How steps run: a call of many steps on a box whose tiles fit the
+ * device at once is one launch that keeps the state on chip, in bx x by tiles of at most `nodes` nodes,
+ * each held by `threads` threads, `per_sm` of them on an SM; bx = 0 when the box's steps are launched one by one. */
+typedef struct itlbm_plan {
+    int bx, by, threads, nodes, per_sm;
+} itlbm_plan;
+int  itlbm_case_plan(const itlbm_case *c, itlbm_plan *out);
+
 /* Sync.  The drop measures of one diagnostic step (Imm_OPS.cpp:299-304): calc_galilean
  * (Galilean_diagnostics.cpp:24-105) with calc_laplace_tension / calc_drop_radius
  * (SimBoltz_Functions/Other_functions.cpp:60-276, 453-554), calc_perfil_logistico
@@ -301,6 +309,8 @@ int  itlbm_batch_advance(itlbm_batch *b, void *stream);
 /* Copies up to `max` waiting events (oldest first) and removes them from the queue. */
 int  itlbm_batch_poll(itlbm_batch *b, itlbm_batch_event *ev, int max);
 int  itlbm_batch_stats_get(const itlbm_batch *b, itlbm_batch_stats *out);
+/* How the last advance stepped the active or held case `tag` (see itlbm_plan). */
+int  itlbm_batch_plan(const itlbm_batch *b, long long tag, itlbm_plan *out);
 
 /* Final fields of batch cases (the files Imm_OPS.cpp:357-364 and Imm_INCL.cpp:101-162 write at the
  * last step).  With itlbm_batch_hold_finished(b, 1), a case that retires (ITLBM_EV_DONE, or

@@ -116,6 +116,11 @@ class BatchStats(C.Structure):
                 ("launch_mode", C.c_int), ("held", C.c_int), ("narrow_edges", C.c_int)]
 
 
+class Plan(C.Structure):
+    """How steps run (itlbm_plan): bx x by tiles held on chip; bx = 0: steps launched one by one."""
+    _fields_ = [(k, C.c_int) for k in ("bx", "by", "threads", "nodes", "per_sm")]
+
+
 class ItlbmError(RuntimeError):
     def __init__(self, code, what):
         super().__init__(f"{what}: {ERRORS.get(code, code)} ({code})")
@@ -147,6 +152,7 @@ def lib():
         "itlbm_case_step": (C.c_int, [vp, C.c_int, C.c_int, vp]),
         "itlbm_case_sync": (C.c_int, [vp]),
         "itlbm_case_steps_done": (C.c_longlong, [vp]),
+        "itlbm_case_plan": (C.c_int, [vp, P(Plan)]),
         "itlbm_case_diag_drop": (C.c_int, [vp, C.c_int, C.c_double, C.c_double, P(DropDiag), vp]),
         "itlbm_case_diag_drop_static": (C.c_int, [vp, C.c_int, C.c_double, C.c_double, P(DropDiag), vp]),
         "itlbm_case_diag_strip": (C.c_int, [vp, C.c_int, P(StripDiag), vp]),
@@ -165,6 +171,7 @@ def lib():
         "itlbm_batch_advance": (C.c_int, [vp, vp]),
         "itlbm_batch_poll": (C.c_int, [vp, P(BatchEvent), C.c_int]),
         "itlbm_batch_stats_get": (C.c_int, [vp, P(BatchStats)]),
+        "itlbm_batch_plan": (C.c_int, [vp, C.c_longlong, P(Plan)]),
         "itlbm_batch_hold_finished": (C.c_int, [vp, C.c_int]),
         "itlbm_batch_read_fields": (C.c_int, [vp, C.c_longlong, C.c_int, dp, dp, dp, dp, dp]),
         "itlbm_batch_release": (C.c_int, [vp, C.c_longlong]),
@@ -257,6 +264,11 @@ class Case:
     @property
     def steps_done(self):
         return lib().itlbm_case_steps_done(self._h)
+
+    def plan(self) -> Plan:
+        out = Plan()
+        check(lib().itlbm_case_plan(self._h, C.byref(out)), "itlbm_case_plan")
+        return out
 
     def diag_drop(self, step, x_ini=None, y_ini=None, stream=None) -> DropDiag:
         out = DropDiag()
@@ -394,6 +406,11 @@ class Batch:
         st = BatchStats()
         check(lib().itlbm_batch_stats_get(self._h, C.byref(st)), "itlbm_batch_stats_get")
         return st
+
+    def plan(self, tag) -> Plan:
+        out = Plan()
+        check(lib().itlbm_batch_plan(self._h, tag, C.byref(out)), "itlbm_batch_plan")
+        return out
 
 
 def dev_perturbacao(op, A, g, f):

@@ -423,6 +423,13 @@ int itlbm_case_sync(itlbm_case *c) {
 
 long long itlbm_case_steps_done(const itlbm_case *c) { return c ? c->steps : -1; }
 
+int itlbm_case_plan(const itlbm_case *c, itlbm_plan *out) {
+    if (!c || !out) return fail(ITLBM_E_ARG, "NULL argument");
+    if (int rd = use_device(c->device)) return rd;
+    *out = res_describe(c->host.prec, c->plan);
+    return ITLBM_OK;
+}
+
 int itlbm_case_save(itlbm_case *c, const char *path) {
     if (!c || !path) return fail(ITLBM_E_ARG, "NULL argument");
     if (int rd = use_device(c->device)) return rd;

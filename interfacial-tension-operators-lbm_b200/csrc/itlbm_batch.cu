@@ -67,6 +67,7 @@ struct Active {
     bool measured = false;  // its last advance ended at one of its diagnostic steps (aux kept there)
     bool held = false;      // retired, state kept for itlbm_batch_read_fields until released
     ResPlan plan;           // tiles in the resident kernel (shape < 0: the box does not fit it)
+    bool resident = false;  // whether the current tables step it there
 };
 
 
@@ -264,7 +265,9 @@ int upload_tables(itlbm_batch *b) {
         build_resident(b);
     }
     for (Active *a : b->slots) {
-        if (!a || a->held || (resident_form(b, a->desc.precision) && a->plan.shape >= 0)) continue;
+        if (!a || a->held) continue;
+        a->resident = resident_form(b, a->desc.precision) && a->plan.shape >= 0;
+        if (a->resident) continue;
         const CaseDev &c = b->h_cases[a->slot];
         case_tiles(c, b->narrow, a->slot, &t[table_of(a->desc.precision) * NSHAPE]);
     }
@@ -1135,12 +1138,21 @@ int itlbm_batch_hold_finished(itlbm_batch *b, int on) {
 }
 
 namespace {
-Active *find_tag(itlbm_batch *b, long long tag) {
+Active *find_tag(const itlbm_batch *b, long long tag) {
     for (Active *a : b->slots)
         if (a && a->tag == tag) return a;
     return nullptr;
 }
 }  // namespace
+
+int itlbm_batch_plan(const itlbm_batch *b, long long tag, itlbm_plan *out) {
+    if (!b || !out) return fail(ITLBM_E_ARG, "bad argument");
+    const Active *a = find_tag(b, tag);
+    if (!a) return fail(ITLBM_E_ARG, "no active or held case with this tag");
+    if (int rd = use_device(b->device)) return rd;
+    *out = a->resident ? res_describe(a->desc.precision, a->plan) : itlbm_plan{};
+    return ITLBM_OK;
+}
 
 int itlbm_batch_read_fields(itlbm_batch *b, long long tag, int form, double *rho_R, double *rho_B,
                             double *ux, double *uy, double *uz) {

@@ -113,6 +113,8 @@ struct ResPlan {
 };
 // CTAs of configuration `shape` the current device holds at once (0: no cooperative launch).
 int res_capacity(int prec, int shape);
+// A plan as the C ABI reports it.
+itlbm_plan res_describe(int prec, const ResPlan &p);
 ResPlan res_plan_single(int prec, int tipo, int nx, int ny);  // one case alone on the device
 ResPlan res_plan_batch(int prec, int nx, int ny);   // one of many cases that share it
 // The queues of a launch: cases in order, each on the least loaded of `ctas` CTAs.  A CTA's load is the time its queue ends, with `cost` the time of one tile.

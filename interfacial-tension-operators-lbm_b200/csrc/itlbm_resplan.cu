@@ -51,6 +51,12 @@ int res_capacity(int prec, int shape) {
     return v ? v->ctas[prec][shape] * v->sms : 0;
 }
 
+itlbm_plan res_describe(int prec, const ResPlan &p) {
+    const Device *v = device();
+    if (!v || p.shape < 0) return itlbm_plan{};
+    return itlbm_plan{p.bx, p.by, res_threads(p.shape), res_nodes(p.shape), v->ctas[prec][p.shape]};
+}
+
 namespace {
 
 int up(int a, int b) { return (a + b - 1) / b; }

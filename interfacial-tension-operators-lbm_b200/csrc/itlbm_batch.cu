@@ -135,6 +135,7 @@ struct itlbm_batch {
         unsigned tag = 0;   // tags used so far in the exchange memory
     } res[NPREC][NRES];
     int *res_flag = nullptr;
+    int polls = RES_POLLS;  // limit of a wait in the resident launches
     bool graph_stale = true;
     int grid[NTAB] = {};
     int ntab[NTAB] = {};  // current table lengths
@@ -388,6 +389,7 @@ cudaError_t enqueue_resident(itlbm_batch *b, int K) {
                 ResArgs a = X.args;
                 a.cases = b->d_cases;
                 a.err = b->res_flag;
+                a.polls = b->polls;
                 a.k0 = k0;
                 a.nsteps = std::min(K - k0, most);
                 a.aux_k = -1;
@@ -1219,6 +1221,12 @@ int itlbm_batch_stats_get(const itlbm_batch *b, itlbm_batch_stats *out) {
     out->admit_ms = b->admit_ms;
     out->capture_ms = b->capture_ms;
     out->launch_mode = b->mode;
+    return ITLBM_OK;
+}
+
+// Not in include/itlbm.h: for tests of the waits' limit.
+int itlbm_internal_batch_polls(itlbm_batch *b, int polls) {
+    b->polls = polls;
     return ITLBM_OK;
 }
 

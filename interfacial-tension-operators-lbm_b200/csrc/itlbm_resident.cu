@@ -29,6 +29,9 @@
 // A launch may hold more tiles than the device does at once: each CTA takes the tiles of its queue one
 // after the other.  All queues follow one order of the cases, so the first unfinished case always has
 // all its CTAs, and no wait is circular.
+// A CTA that comes to a case before its neighbours waits until these are through the cases before it, which
+// can take as long as those do; so a tile first waits for the tiles beside it to have begun, as long as any
+// tile of the launch is being finished, and only then steps, in exchanges that take microseconds.
 // Every wait is bounded: a wait that runs out sets *err and the CTA returns at the end of its step,
 // as do its neighbours in turn.
 //
@@ -45,7 +48,7 @@ namespace itlbm {
 
 namespace {
 
-constexpr int SPIN_LIMIT = 1 << 23;  // polls of one wait, each a trip to L2: some seconds
+constexpr int SPIN_LIMIT = 1 << 23;  // polls of an exchange, each a trip to L2: some seconds
 
 // planes that leave a tile through a side (0 +x, 1 -x, 2 +y, 3 -y): the axis ones, then the two
 // diagonals
@@ -90,6 +93,9 @@ __device__ __forceinline__ unsigned ld_word(const unsigned *p) {
     asm volatile("ld.relaxed.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
     return v;
 }
+__device__ __forceinline__ void count_word(unsigned *p) {
+    asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
+}
 __device__ __forceinline__ unsigned long long pair_of(unsigned a, unsigned b) {
     return (unsigned long long)a | ((unsigned long long)b << 32);
 }
@@ -110,6 +116,20 @@ __device__ __forceinline__ bool poll_items(unsigned pend, LOAD load, TAKE take) 
         if (!pend) return true;
     }
     return false;
+}
+
+// Waits until the CTA of `done` has come as far as tag.  False when it has not after a.polls polls during which no
+// tile was finished.
+__device__ __forceinline__ bool wait_for(const ResArgs &a, const unsigned *done, unsigned tag) {
+    unsigned finished = 0;
+    for (int polls = 0; (int)(ld_word(done) - tag) < 0;)
+        if (++polls >= a.polls) {
+            const unsigned now = ld_word(a.finished);
+            if (now == finished) return false;
+            finished = now;
+            polls = 0;
+        }
+    return true;
 }
 
 // first coordinate of tile t of n nodes cut into b tiles (res_tiling keeps the product in 32 bits)
@@ -294,6 +314,15 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
         const int t = tid + r * NT, ly = t / g.w, lx = t - ly * g.w;
         return node_off(the_case(), g.x0 + lx, g.y0 + ly);
     };
+    // where CTAs take several tiles, those of the tiles beside this one have begun it too (or finished the case before)
+    if (a.queued) {
+        if (tid == 0) st_word(a.done + blockIdx.x, g.tag0);
+        if (tid < 9 && !wait_for(a, a.done + g.slot[tid], g.tag0)) bad = 1;
+        if (__syncthreads_or(bad)) {
+            if (tid == 0) *a.err = 1;
+            return;
+        }
+    }
     // the buffer the launch does not end in: a site that is streamed unchanged waits there
     auto spare = [&]() { return (S *)the_case().buf[(g.cur0 ^ (g.nsteps & 1)) ^ 1]; };
     __syncthreads();
@@ -514,18 +543,12 @@ __global__ void __launch_bounds__(res_threads(SHAPE), (ResCfg<S, FOLD, SHAPE>::M
         }
     // Before its next tile writes into its exchange slot, the CTA knows that the tiles beside this one have
     // taken what it posted last: each says so when it is done.
-    if (qi + 1 < qend) {
-        const unsigned last = g.tag0 + (unsigned)g.nsteps;
-        if (tid == 0) st_word(a.done + blockIdx.x, last);
-        if (tid < 9) {
-            int spins = 0;
-            while ((int)(ld_word(a.done + g.slot[tid]) - last) < 0)
-                if (++spins > SPIN_LIMIT) {
-                    bad = 1;
-                    break;
-                }
-        }
-    } else if (tid == 0) st_word(a.done + blockIdx.x, g.tag0 + (unsigned)g.nsteps);
+    const unsigned last = g.tag0 + (unsigned)g.nsteps;
+    if (tid == 0) {
+        st_word(a.done + blockIdx.x, last);
+        count_word(a.finished);
+    }
+    if (qi + 1 < qend && tid < 9 && !wait_for(a, a.done + g.slot[tid], last)) bad = 1;
     if (__syncthreads_or(bad)) {
         if (tid == 0) *a.err = 1;
         return;

@@ -34,7 +34,10 @@ struct ResArgs {
     const ResTile *tiles;   // the queues of the CTAs, one after the other
     const int *first;       // CTA b takes tiles [first[b], first[b + 1])
     const int *slots;       // CTA of each tile of each case, from ResTile::peers on
-    unsigned *done;         // per CTA: the last tag of the last tile it finished
+    unsigned *done;         // per CTA: the last tag of the last tile it finished, or the one before the first of its tile
+    unsigned *finished;     // tiles finished in this exchange memory, over all CTAs and launches
+    int polls;              // of `done`, after which a wait for a CTA runs out unless tiles are being finished
+    int queued;             // whether a CTA of the launch has more than one tile
     uint4 *packs;      // exchange of populations: 2 parities x slots x NPK x PK packs
     void *phis;        // exchange of rho^N: 2 parities x slots x NODES entries of 8 (FP32) or 16 bytes
     int *err;          // set when a wait ran out
@@ -97,6 +100,9 @@ inline cudaError_t res_launch(int prec, int shape, const ResArgs &a, int grid, c
 // 39 / 29 us; 6 steps: 76 / 64, 46 / 42, 56 / 34 us.
 constexpr int RES_MIN_STEPS = 6;
 constexpr int RES_MAX_STEPS = 4096;
+// Polls without a finished tile, each a trip to L2: some 3 s.  The longest that a tile takes is RES_MAX_STEPS
+// steps, below 0.1 s.
+constexpr int RES_POLLS = 1 << 23;
 // Sub-steps a batch's replay must have: its tables keep the GPU busy with k_step, and a resident tile's first loads
 // and tables are hidden by nothing.  Tables / resident, G updates/s, 150 mixed cases of 64 to 512 nodes a side and 100
 // of 64 to 256: FP64 10 steps 7.25 / 6.85 and 6.4 / 5.7, 20 steps 7.25 / 7.24 and 6.4 / 6.7; FP32 20 steps 14.8 / 15.0

@@ -203,6 +203,7 @@ cudaError_t res_queues_upload(ResArgs &a, const ResQueues &q, void *mem, cudaStr
     };
     a.tiles = (const ResTile *)put(q.tiles.data(), sizeof(ResTile) * q.tiles.size());
     a.first = (const int *)put(q.first.data(), sizeof(int) * q.first.size());
+    a.queued = q.tiles.size() + 1 > q.first.size();
     a.slots = (const int *)put(q.slots.data(), sizeof(int) * q.slots.size());
     const cudaError_t e = cudaMemcpyAsync(mem, all.data(), at, cudaMemcpyHostToDevice, st);
     const cudaError_t w = cudaStreamSynchronize(st);  // pageable copies may return before they have read
@@ -210,13 +211,15 @@ cudaError_t res_queues_upload(ResArgs &a, const ResQueues &q, void *mem, cudaStr
 }
 
 size_t res_exchange_bytes(int prec, int shape, int slots) {
-    return (size_t)slots * (2 * (npk_of(prec, shape) * pk_of(prec) * 16 + res_nodes(shape) * phi_bytes(prec)) + sizeof(unsigned));
+    return (size_t)slots * (2 * (npk_of(prec, shape) * pk_of(prec) * 16 + res_nodes(shape) * phi_bytes(prec)) + sizeof(unsigned)) + sizeof(unsigned);
 }
 void res_exchange_bind(ResArgs &a, void *base, int prec, int shape, int slots) {
     a.packs = (uint4 *)base;
     a.phis = (char *)base + (size_t)2 * slots * npk_of(prec, shape) * pk_of(prec) * 16;
     a.done = (unsigned *)((char *)a.phis + (size_t)2 * slots * res_nodes(shape) * phi_bytes(prec));
+    a.finished = a.done + slots;
     a.nslots = slots;
+    a.polls = RES_POLLS;
 }
 
 int *res_flag_get() {

@@ -12,7 +12,8 @@
  *     default stream).  Calls marked "async" only enqueue work on that stream.
  *   - Every int-returning call returns ITLBM_OK (0) or a negative ITLBM_E_* code; the text of the
  *     last failure on the calling thread is returned by itlbm_last_error().  No call traps or hangs
- *     the device: waits are bounded and report ITLBM_E_TIMEOUT.
+ *     the device: waits are bounded and report ITLBM_E_TIMEOUT.  After it the object's state is undefined: a
+ *     case returns ITLBM_E_TIMEOUT until itlbm_case_write_pops gives it a new state, a batch from then on.
  *   - The library owns all device memory of a case.  Populations handed across the ABI are FP64 in
  *     the reference's array-of-structures order, f[pto * 19 + i] with pto = x + nx * y, exactly the
  *     layout of LATTICE::inif_R / inif_B (SimBoltz_Functions/Definitions.cpp:52-114).

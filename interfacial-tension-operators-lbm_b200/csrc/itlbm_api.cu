@@ -174,7 +174,8 @@ struct itlbm_case {
 };
 
 namespace {
-// After a synchronisation: whether a wait of a resident launch ran out (the state is then undefined).
+// Whether a wait of a resident launch ran out, as far as the device has got: after a synchronisation, of any
+// launch so far.  The state is undefined from then on, until it is written anew.
 int waited(const itlbm_case *c) {
     if (!c->res_flag || *(volatile int *)c->res_flag == 0) return ITLBM_OK;
     return fail(ITLBM_E_TIMEOUT, "a wait between the tiles of a step ran out");
@@ -371,6 +372,7 @@ int itlbm_case_step(itlbm_case *c, int nsteps, int flags, void *stream) {
     if (!c || nsteps < 0) return fail(ITLBM_E_ARG, "bad argument");
     if (nsteps == 0) return ITLBM_OK;
     if (int rd = use_device(c->device)) return rd;
+    if (int r = waited(c)) return r;
     const bool keep = (flags & ITLBM_STEP_KEEP_AUX) != 0;
     if (keep) {
         int r = ensure_aux(c);
@@ -591,7 +593,11 @@ int itlbm_case_write_pops(itlbm_case *c, const double *fR, const double *fB) {
     if (e == cudaSuccess) e = launch_import(c->dev, c->host.nx, c->host.ny, cur, c->tmp, c->tmp + NV * n, 0);
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
     c->aux_valid = 0;
-    return e == cudaSuccess ? ITLBM_OK : cuda_fail(e, "write_pops");
+    if (e != cudaSuccess) return cuda_fail(e, "write_pops");
+    // a whole new state, and nothing under way: the steps go on from here (on tags of their own, a launch that gave up
+    // counts as its steps)
+    if (c->res_flag) *(volatile int *)c->res_flag = 0;
+    return ITLBM_OK;
 }
 
 static int read_fields_as(itlbm_case *c, int form, double *rho_R, double *rho_B, double *ux, double *uy,
@@ -631,6 +637,13 @@ int itlbm_case_read_fields(itlbm_case *c, double *rho_R, double *rho_B, double *
 
 int itlbm_case_read_profile(itlbm_case *c, double *rho_R, double *rho_B, double *ux, double *uy) {
     return read_fields_as(c, ITLBM_FIELDS_PROFILE, rho_R, rho_B, ux, uy, nullptr, nullptr);
+}
+
+// Not in include/itlbm.h: for tests, as a launch whose wait ran out leaves the case.
+int itlbm_internal_case_expire(itlbm_case *c) {
+    if (!c->res_flag) return ITLBM_E_STATE;
+    *(volatile int *)c->res_flag = 1;
+    return ITLBM_OK;
 }
 
 }  // extern "C"

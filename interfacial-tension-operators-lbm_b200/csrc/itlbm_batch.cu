@@ -411,6 +411,12 @@ cudaError_t enqueue_resident(itlbm_batch *b, int K) {
     return e;
 }
 
+// Whether a wait of a resident launch ran out: the states of the cases it held are then undefined.
+int waited(const itlbm_batch *b) {
+    if (!b->res_flag || *(volatile int *)b->res_flag == 0) return ITLBM_OK;
+    return fail(ITLBM_E_TIMEOUT, "a wait between the tiles of a step ran out");
+}
+
 // Adds the host wall time of its scope to a counter of the batch, in ms.
 struct ScopeTimer {
     const itlbm_batch *b;
@@ -977,6 +983,7 @@ int itlbm_batch_submit_saved(itlbm_batch *b, const char *path, int n_steps, long
 int itlbm_batch_save(itlbm_batch *b, long long tag, const char *path) {
     if (!b || !path) return fail(ITLBM_E_ARG, "bad argument");
     if (int rd = use_device(b->device)) return rd;
+    if (int r = waited(b)) return r;
     for (Active *a : b->slots) {
         if (!a || a->held || a->tag != tag) continue;
         cudaError_t e = cudaStreamSynchronize(b->stream);
@@ -1007,6 +1014,7 @@ int itlbm_batch_advance(itlbm_batch *b, void *stream) {
     ScopeTimer timer(b, b->advance_ms);
     if (int rd = use_device(b->device)) return rd;
     int r;
+    if ((r = waited(b)) != ITLBM_OK) return r;
     {
         ScopeTimer t_admit(b, b->admit_ms);
         r = admit(b);
@@ -1089,7 +1097,7 @@ int itlbm_batch_advance(itlbm_batch *b, void *stream) {
         if (e != cudaSuccess) return cuda_fail(e, "diagnostic copy");
     }
     if ((e = cudaStreamSynchronize(b->stream)) != cudaSuccess) return cuda_fail(e, "replay");
-    if (b->res_flag && *(volatile int *)b->res_flag) return fail(ITLBM_E_TIMEOUT, "a wait between the tiles of a step ran out");
+    if ((r = waited(b)) != ITLBM_OK) return r;
     float ms = 0;
     cudaEventElapsedTime(&ms, b->ev0, b->ev1);
     b->device_ms += ms;
@@ -1165,6 +1173,7 @@ int itlbm_batch_read_fields(itlbm_batch *b, long long tag, int form, double *rho
     if (a->next_step < 1 || (force && !a->measured))
         return fail(ITLBM_E_STATE, "the case's last step was not a measured one (class F needs its force)");
     if (int rd = use_device(b->device)) return rd;
+    if (int r = waited(b)) return r;
     const size_t n = (size_t)a->desc.nx * a->desc.ny;
     double *t = nullptr;
     cudaError_t e = cudaMallocFromPoolAsync(&t, sizeof(double) * 5 * n, b->pool, b->stream);

@@ -48,7 +48,7 @@ namespace itlbm {
 
 namespace {
 
-constexpr int SPIN_LIMIT = 1 << 23;  // polls of an exchange, each a trip to L2: some seconds
+constexpr int SPIN_LIMIT = 1 << 21;  // polls of an exchange, each a trip to L2: about a second
 
 // planes that leave a tile through a side (0 +x, 1 -x, 2 +y, 3 -y): the axis ones, then the two
 // diagonals

@@ -54,3 +54,55 @@ def test_a_case_waits_for_its_neighbours_earlier_cases(gpu, tmp_path):
         for t in last:
             got = b.read_fields(t, 48 * 32, gpu.FIELDS_VTK)
             assert all(np.array_equal(got[k], want[k]) for k in want)
+
+
+def expired(itlbm, call):
+    with pytest.raises(itlbm.ItlbmError) as e:
+        call()
+    assert e.value.code == -7  # ITLBM_E_TIMEOUT
+
+
+def test_a_case_whose_wait_ran_out(gpu, tmp_path):
+    """Every call that steps it or reads it says so, until it is given a new state; then it goes on as any other."""
+    with gpu.Case(desc(gpu, 40, 50)) as c, gpu.Case(desc(gpu, 40, 50)) as d:
+        c.step(10)
+        pops = c.read_pops(0)
+        c.step(10, keep_aux=True)
+        c.sync()
+        f = gpu.lib().itlbm_internal_case_expire
+        f.argtypes = [C.c_void_p]
+        assert f(c.handle) == 0
+        done = c.steps_done
+        for call in (lambda: c.step(10), lambda: c.step(1), c.sync, lambda: c.read_pops(0), c.read_fields, lambda: c.diag_drop(19),
+                     lambda: c.save(tmp_path / "s")):
+            expired(gpu, call)
+        assert c.steps_done == done
+        c.write_pops(*pops)
+        c.step(30)
+        d.step(40)
+        assert all(np.array_equal(x, y) for x, y in zip(c.read_pops(0), d.read_pops(0)))
+
+
+def test_a_batch_whose_wait_ran_out(gpu, tmp_path):
+    """The cases of test_a_case_waits_for_its_neighbours_earlier_cases, in fewer rounds of longer tiles, with a limit
+    below the time of one: the launch ends by itself, the advance says so, and so does every one after it."""
+    with gpu.Case(desc(gpu, 64, 32)) as c:
+        c.step(1)
+        c.save(tmp_path / "long")
+    with gpu.Case(desc(gpu, 48, 32)) as c:
+        c.step(1)
+        c.save(tmp_path / "last")
+    with gpu.Batch() as b:
+        polls(gpu, b, 200)
+        for k in range(0, 37 * 8, 37):
+            b.submit_saved(tmp_path / "long", 10 ** 6, k)
+            for j in range(36):
+                b.submit(desc(gpu, 64, 32), 10 ** 6, k + 1 + j)
+        for t in (1000, 1001):
+            b.submit_saved(tmp_path / "last", 10 ** 6, t)
+        for call in (b.advance, b.advance, lambda: b.save(1000, tmp_path / "s")):
+            expired(gpu, call)
+    with gpu.Batch() as b:  # the device is none the worse
+        b.submit(desc(gpu, 64, 32), 30, 1)
+        while b.stats().finished < 1:
+            b.advance()

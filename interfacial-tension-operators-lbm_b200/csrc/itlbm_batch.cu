@@ -1238,5 +1238,23 @@ int itlbm_internal_batch_polls(itlbm_batch *b, int polls) {
     b->polls = polls;
     return ITLBM_OK;
 }
+// The same, as a batch that has used its exchange memory's tags up to `tag`: how many of its launches these are.
+int itlbm_internal_batch_tag(itlbm_batch *b, unsigned tag) {
+    int n = 0;
+    for (auto &row : b->res)
+        for (auto &X : row)
+            if (X.ctas > 0 && X.tag <= tag) {
+                X.tag = tag;
+                n++;
+            }
+    return n;
+}
+unsigned itlbm_internal_batch_tag_of(const itlbm_batch *b) {
+    unsigned tag = 0;
+    for (auto &row : b->res)
+        for (auto &X : row)
+            if (X.ctas > 0) tag = std::max(tag, X.tag);
+    return tag;
+}
 
 }  // extern "C"

@@ -106,3 +106,53 @@ def test_a_batch_whose_wait_ran_out(gpu, tmp_path):
         b.submit(desc(gpu, 64, 32), 30, 1)
         while b.stats().finished < 1:
             b.advance()
+
+
+MIXED = [(100, 100, 3, 0), (61, 70, 11, 0), (40, 90, 12, 0), (120, 110, 3, 1), (64, 64, 11, 1), (90, 95, 13, 2), (50, 60, 12, 2)]
+
+
+def check_against_single_steps(itlbm, b, steps, boxes):
+    for tag, box in enumerate(boxes):
+        got = b.read_fields(tag, box[0] * box[1], itlbm.FIELDS_VTK)
+        with itlbm.Case(desc(itlbm, *box)) as c:
+            for _ in range(steps - 1):
+                c.step(1)
+            c.step(1, keep_aux=True)
+            want = c.read_fields()
+        assert all(np.array_equal(got[k], want[k]) for k in want), box
+
+
+@pytest.mark.parametrize("room", [0, 1, 60 * 3 + 1, 60 * 7 + 10])
+def test_tags_start_again(gpu, room):
+    """A batch comes to the end of its tags before, in and after the replay that would use the last `room` of them."""
+    L = gpu.lib()
+    L.itlbm_internal_batch_tag.argtypes = [C.c_void_p, C.c_uint]
+    L.itlbm_internal_batch_tag_of.argtypes = [C.c_void_p]
+    L.itlbm_internal_batch_tag_of.restype = C.c_uint
+    with gpu.Batch(chunk=60, diag_every=60) as b:
+        b.hold_finished(True)
+        for tag, box in enumerate(MIXED):
+            b.submit(desc(gpu, *box), 361, tag)
+        b.advance()
+        b.advance()
+        assert all(b.plan(tag).bx > 0 for tag in range(len(MIXED)))
+        assert L.itlbm_internal_batch_tag(b._h, 2 ** 31 - 1 - room) == 3
+        tags = []
+        while b.stats().finished < len(MIXED):
+            b.advance()
+            b.poll()
+            tags.append(L.itlbm_internal_batch_tag_of(b._h))
+        assert min(tags[:-1]) < 2000 and max(tags) < 2 ** 31
+        check_against_single_steps(gpu, b, 361, MIXED)
+
+
+def test_a_replay_longer_than_a_launch(gpu):
+    boxes = [(16, 16, 12, 0), (20, 17, 3, 1), (33, 9, 11, 2), (24, 24, 3, 0)]
+    with gpu.Batch(chunk=5000, diag_every=5000) as b:
+        b.hold_finished(True)
+        for tag, box in enumerate(boxes):
+            b.submit(desc(gpu, *box), 4801, tag)
+        b.advance()
+        b.advance()
+        assert b.stats().finished == len(boxes) and all(b.plan(tag).bx > 0 for tag in range(len(boxes)))
+        check_against_single_steps(gpu, b, 4801, boxes)

@@ -394,9 +394,12 @@ int itlbm_case_step(itlbm_case *c, int nsteps, int flags, void *stream) {
                 a.aux_k = keep ? (int)(c->steps + nsteps - 1) : -1;
                 a.tag0 = (unsigned)a.k0;  // the step counter never returns to a value: neither do the tags
                 const cudaError_t e = res_launch(c->host.prec, c->plan.shape, a, c->plan.tiles, s);
+                if (e == cudaErrorCooperativeLaunchTooLarge) {  // a stream with fewer SMs than the device (a green context's)
+                    cudaGetLastError();
+                    break;
+                }
                 if (e != cudaSuccess) return cuda_fail(e, "resident step kernel");
             }
-            i0 = nsteps;
         }
     }
     for (int i = i0; i < nsteps; i++) {

@@ -875,6 +875,7 @@ int itlbm_batch_create(const itlbm_batch_config *cfg, itlbm_batch **out) {
     cudaMemsetAsync(b->d_cases, 0, sizeof(CaseDev) * M, b->stream);
     cudaMemsetAsync(b->d_ntiles, 0, sizeof(int) * NTAB, b->stream);
     cudaStreamSynchronize(b->stream);
+    b->resident_ok = b->resident_ok && res_whole_device(b->stream);
     // work tables with room for a first batch, so the graph can be captured with their addresses
     for (int p = 0; p < NTAB; p++) {
         b->tiles_cap[p] = 1 << 16;

@@ -51,6 +51,29 @@ int res_capacity(int prec, int shape) {
     return v ? v->ctas[prec][shape] * v->sms : 0;
 }
 
+__global__ void __launch_bounds__(1024) k_places() {}
+
+bool res_whole_device(cudaStream_t st) {
+    const Device *v = device();
+    int n = 0;
+    if (!v || v->sms == 0 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_places, 1024, 0) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(n * v->sms));
+    cfg.blockDim = dim3(1024);
+    cfg.stream = st;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const bool ok = cudaLaunchKernelEx(&cfg, k_places) == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    return ok;
+}
+
 itlbm_plan res_describe(int prec, const ResPlan &p) {
     const Device *v = device();
     if (!v || p.shape < 0) return itlbm_plan{};

@@ -1,5 +1,7 @@
 """Which kernel steps which box: the comparisons of test_gpu_resident.py are of two kernels only where the
 library reports a plan, so the plans are asserted here over the same boxes."""
+import ctypes as C
+
 import pytest
 
 from test_gpu_resident import BOXES, OPS, both_ways, make, same
@@ -59,3 +61,62 @@ def test_batch_replays_take_it_from_their_length_on(gpu, prec, longest):
             b.advance()
             b.advance()
             assert (b.plan(1).bx > 0) == (chunk == longest)
+
+
+class GreenContext:
+    """Sixteen of the device's SMs as a green context, by the driver API."""
+
+    def __init__(self):
+        self.L = L = C.CDLL("libcuda.so.1")
+        resource = C.c_char * 144
+        every, part, rest = resource(), resource(), resource()
+        n, self.desc, self.ctx, self.stream = C.c_uint(1), C.c_void_p(), C.c_void_p(), C.c_void_p()
+        for code in (L.cuDeviceGetDevResource(0, every, 1), L.cuDevSmResourceSplitByCount(part, C.byref(n), every, rest, 0, 16),
+                     L.cuDevResourceGenerateDesc(C.byref(self.desc), part, 1),
+                     L.cuGreenCtxCreate(C.byref(self.ctx), self.desc, 0, 1),
+                     L.cuGreenCtxStreamCreate(C.byref(self.stream), self.ctx, 1, 0)):
+            if code:
+                pytest.skip(f"no green context ({code})")
+
+    def __enter__(self):
+        return self
+
+    def __exit__(self, *a):
+        self.L.cuStreamDestroy_v2(self.stream)
+        self.L.cuGreenCtxDestroy(self.ctx)
+
+
+@pytest.mark.parametrize("prec,nx,ny", [(0, 100, 100), (1, 300, 310), (2, 40, 40)])
+def test_a_stream_with_fewer_sms(gpu, prec, nx, ny):
+    """What a stream of a green context cannot hold at once is stepped launch by launch, in the same bits."""
+    with make(gpu, nx, ny, 12, prec) as c, make(gpu, nx, ny, 12, prec) as d, GreenContext() as g:
+        assert c.plan().bx
+        c.step(9, stream=g.stream)
+        c.step(7, keep_aux=True, stream=g.stream)
+        c.sync()
+        d.step(16, keep_aux=True)
+        assert all((x == y).all() for x, y in zip(c.read_pops(0), d.read_pops(0)))
+        f, h = c.read_fields(force=True), d.read_fields(force=True)
+        assert all((f[k] == h[k]).all() for k in f)
+
+
+def test_a_batch_with_fewer_sms(gpu):
+    desc = gpu.desc(100, 100, gpu.make_op(3, 0.5), tau=0.83, radius=23)
+    with gpu.Case(desc) as d, GreenContext() as g:
+        old, ctx = C.c_void_p(), C.c_void_p()
+        assert g.L.cuCtxGetCurrent(C.byref(old)) == 0 and g.L.cuCtxFromGreenCtx(C.byref(ctx), g.ctx) == 0
+        assert g.L.cuCtxSetCurrent(ctx) == 0
+        try:
+            b = gpu.Batch()
+        finally:
+            assert g.L.cuCtxSetCurrent(old) == 0
+        with b:
+            b.hold_finished(True)
+            b.submit(desc, 101, 1)
+            while b.stats().finished < 1:
+                b.advance()
+            assert b.plan(1).bx == 0
+            got = b.read_fields(1, 100 * 100)
+        d.step(101, keep_aux=True)
+        want = d.read_fields()
+        assert all((got[k] == want[k]).all() for k in got)

@@ -308,8 +308,17 @@ int itlbm_case_create(const itlbm_case_desc *d, itlbm_case **out) {
         queues = res_queues({ResCase{c->plan, 0, 1.0}}, c->plan.tiles);
         xbytes = res_exchange_bytes(d->precision, c->plan.shape, c->plan.tiles);
     }
-    const size_t mem_bytes = 2 * per_buf + xbytes + (c->plan.shape >= 0 ? queues.bytes() : 0);
-    if ((e = cudaMalloc(&c->mem, mem_bytes)) != cudaSuccess) {
+    size_t mem_bytes = 2 * per_buf + xbytes + (c->plan.shape >= 0 ? queues.bytes() : 0);
+    e = cudaMalloc(&c->mem, mem_bytes);
+    if (e == cudaErrorMemoryAllocation && c->plan.shape >= 0) {  // room for the state alone: its steps one by one
+        cudaGetLastError();
+        c->plan = ResPlan();
+        res_flag_put(c->res_flag);
+        c->res_flag = nullptr;
+        mem_bytes = 2 * per_buf;
+        e = cudaMalloc(&c->mem, mem_bytes);
+    }
+    if (e != cudaSuccess) {
         itlbm_case_destroy(c);
         return cuda_fail(e, "cudaMalloc(state)");
     }

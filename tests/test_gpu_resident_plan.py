@@ -120,3 +120,30 @@ def test_a_batch_with_fewer_sms(gpu):
         d.step(101, keep_aux=True)
         want = d.read_fields()
         assert all((got[k] == want[k]).all() for k in got)
+
+
+def test_room_for_the_state_alone(gpu):
+    """On a device with too little memory for a case's exchange between tiles, but enough for its state, the case is
+    created and stepped launch by launch."""
+    import torch
+    for spare_mb in range(38, 70, 2):  # the state takes 40 MB, the exchange 9
+        free, _ = torch.cuda.mem_get_info()
+        try:
+            hog = torch.empty(free - (spare_mb << 20), dtype=torch.uint8, device="cuda")
+        except torch.OutOfMemoryError:
+            torch.cuda.empty_cache()
+            continue
+        try:
+            c = make(gpu, 250, 250, 3, 0)
+        except gpu.ItlbmError as e:
+            assert e.code == -2
+            c = None
+        del hog
+        torch.cuda.empty_cache()
+        if c:
+            break
+    with c, make(gpu, 250, 250, 3, 0) as d:
+        assert c.plan().bx == 0 and d.plan().bx
+        c.step(8)
+        d.step(8)
+        assert all((x == y).all() for x, y in zip(c.read_pops(0), d.read_pops(0)))

@@ -3,6 +3,7 @@
 #include "itlbm_resident.h"
 
 #include <algorithm>
+#include <atomic>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
@@ -20,23 +21,32 @@ size_t phi_bytes(int prec) { return prec == ITLBM_PREC_F64 ? 16 : 8; }
 constexpr int MAX_DEVICES = 32;
 struct Device {
     std::once_flag once;
-    int sms = 0;
-    int ctas[3][NRES] = {};  // resident CTAs per SM by storage form and configuration
+    int sms = 0;  // 0: no cooperative launches
+    // resident CTAs per SM by storage form and configuration, each asked when a plan comes to it: the question loads
+    // the kernel, and all sixteen kept the first case of a process waiting for 5 ms
+    std::once_flag asked[3][NRES];
+    int ctas[3][NRES] = {};
+    std::atomic<int> loaded{0};
 };
 Device g_dev[MAX_DEVICES];
 
-const Device *device() {
+Device *device() {
     int d = 0;
     if (cudaGetDevice(&d) != cudaSuccess || d < 0 || d >= MAX_DEVICES) return nullptr;
     Device &v = g_dev[d];
     std::call_once(v.once, [&] {
         int coop = 0;
         cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, d);
-        if (!coop || cudaDeviceGetAttribute(&v.sms, cudaDevAttrMultiProcessorCount, d) != cudaSuccess) return;
-        for (int prec = 0; prec < 3; prec++)
-            for (int shape = 0; shape < NRES; shape++) v.ctas[prec][shape] = res_occupancy(prec, shape);
+        if (!coop || cudaDeviceGetAttribute(&v.sms, cudaDevAttrMultiProcessorCount, d) != cudaSuccess) v.sms = 0;
     });
-    return &v;
+    return v.sms ? &v : nullptr;
+}
+int ctas_per_sm(Device &v, int prec, int shape) {
+    std::call_once(v.asked[prec][shape], [&] {
+        v.ctas[prec][shape] = res_occupancy(prec, shape);
+        v.loaded += v.ctas[prec][shape] > 0;
+    });
+    return v.ctas[prec][shape];
 }
 
 std::mutex g_flag_lock;
@@ -47,8 +57,8 @@ constexpr int NFLAGS = 1 << 14;
 }  // namespace
 
 int res_capacity(int prec, int shape) {
-    const Device *v = device();
-    return v ? v->ctas[prec][shape] * v->sms : 0;
+    Device *v = device();
+    return v ? ctas_per_sm(*v, prec, shape) * v->sms : 0;
 }
 
 __global__ void __launch_bounds__(1024) k_places() {}
@@ -56,7 +66,7 @@ __global__ void __launch_bounds__(1024) k_places() {}
 bool res_whole_device(cudaStream_t st) {
     const Device *v = device();
     int n = 0;
-    if (!v || v->sms == 0 || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_places, 1024, 0) != cudaSuccess) {
+    if (!v || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_places, 1024, 0) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
@@ -75,9 +85,9 @@ bool res_whole_device(cudaStream_t st) {
 }
 
 itlbm_plan res_describe(int prec, const ResPlan &p) {
-    const Device *v = device();
+    Device *v = device();
     if (!v || p.shape < 0) return itlbm_plan{};
-    return itlbm_plan{p.bx, p.by, res_threads(p.shape), res_nodes(p.shape), v->ctas[prec][p.shape]};
+    return itlbm_plan{p.bx, p.by, res_threads(p.shape), res_nodes(p.shape), ctas_per_sm(*v, prec, p.shape)};
 }
 
 namespace {
@@ -269,3 +279,9 @@ void res_flag_put(int *f) {
 }
 
 }  // namespace itlbm
+
+// Not in include/itlbm.h: for tests, the configurations loaded so far on the current device.
+extern "C" int itlbm_internal_configurations(void) {
+    itlbm::Device *v = itlbm::device();
+    return v ? v->loaded.load() : 0;
+}

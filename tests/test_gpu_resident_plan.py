@@ -1,12 +1,16 @@
 """Which kernel steps which box: the comparisons of test_gpu_resident.py are of two kernels only where the
 library reports a plan, so the plans are asserted here over the same boxes."""
 import ctypes as C
+import subprocess
+import sys
+from pathlib import Path
 
 import pytest
 
 from test_gpu_resident import BOXES, OPS, both_ways, make, same
 
 pytestmark = pytest.mark.gpu
+REPO = Path(__file__).resolve().parent.parent
 
 # (threads, nodes, CTAs per SM) of every configuration compiled for a storage form
 CONFIGS = {0: {(64, 64), (128, 128), (160, 160), (192, 192), (224, 224), (256, 256)},
@@ -147,3 +151,12 @@ def test_room_for_the_state_alone(gpu):
         c.step(8)
         d.step(8)
         assert all((x == y).all() for x, y in zip(c.read_pops(0), d.read_pops(0)))
+
+
+@pytest.mark.parametrize("nx,prec,most", [(40, 0, 1), (200, 0, 3), (40, 1, 1), (300, 2, 3)])
+def test_a_case_loads_only_what_its_plan_looks_at(gpu, nx, prec, most):
+    """The first case of a process does not load the kernels of every storage form and configuration."""
+    code = (f"import sys; sys.path.insert(0, 'oracle'); import oracle; m = oracle.load_package()\n"
+            f"c = m.Case(m.desc({nx}, {nx}, m.make_op(3, 0.5), radius=9, precision={prec}))\n"
+            f"assert c.plan().bx and 1 <= m.lib().itlbm_internal_configurations() <= {most}")
+    subprocess.run([sys.executable, "-c", code], cwd=REPO, check=True)

@@ -94,12 +94,12 @@ void fill_shift(CaseDev &c, double rho0, double u0x) {
 
 cudaError_t launch_step(const CaseDev *cases_dev, const TileRef *tiles, int ntiles,
                         const int *ntiles_dev, int grid, int k, int aux_k, int prec,
-                        int shape, cudaStream_t s) {
+                        int shape, bool early, cudaStream_t s) {
     if (prec == ITLBM_PREC_F64)
-        return launch_step_f64(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, s);
+        return launch_step_f64(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, early, s);
     if (prec == ITLBM_PREC_F32_FOLD)
-        return launch_step_fold(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, s);
-    return launch_step_f32(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, s);
+        return launch_step_fold(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, early, s);
+    return launch_step_f32(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, early, s);
 }
 
 bool narrow_edges_default() {
@@ -389,13 +389,13 @@ int itlbm_case_step(itlbm_case *c, int nsteps, int flags, void *stream) {
     }
     cudaStream_t s = (cudaStream_t)stream;
     if (c->steps + nsteps > (long long)INT_MAX - 2) return fail(ITLBM_E_STATE, "step counter overflow");
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    const bool captured = cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone;
+    if (captured) cudaGetLastError();
     int i0 = 0;
     if (c->plan.shape >= 0 && nsteps >= RES_MIN_STEPS) {
-        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
         // a captured launch would be replayed with the tags of its capture
-        if (cudaStreamIsCapturing(s, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
-            cudaGetLastError();
-        } else {
+        if (!captured) {
             for (; i0 < nsteps; i0 += RES_MAX_STEPS) {
                 ResArgs a = c->res;
                 a.k0 = (int)(c->steps + i0);
@@ -418,7 +418,7 @@ int itlbm_case_step(itlbm_case *c, int nsteps, int flags, void *stream) {
             const int n = c->tile_off[sh + 1] - c->tile_off[sh];
             if (n == 0) continue;
             cudaError_t e = launch_step(c->dev, c->tiles + c->tile_off[sh], n, nullptr, n, k, aux_k,
-                                        c->host.prec, sh, s);
+                                        c->host.prec, sh, !captured, s);
             if (e != cudaSuccess) return cuda_fail(e, "step kernel");
         }
     }

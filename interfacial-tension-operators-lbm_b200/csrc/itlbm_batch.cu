@@ -301,14 +301,14 @@ int upload_tables(itlbm_batch *b) {
 // single table runs in line on st; several run side by side, the 32 x 8 table on st and each narrow
 // table on a stream of its own, every launch of sub-step k > k0 waiting for the other shapes'
 // launches of sub-step k - 1, so that the small narrow-tile launches overlap the large one.
-cudaError_t enqueue_chain(itlbm_batch *b, int pi, int k0, int k1, cudaStream_t st) {
+cudaError_t enqueue_chain(itlbm_batch *b, int pi, int k0, int k1, bool early, cudaStream_t st) {
     int shapes[NSHAPE], n = 0;
     for (int sh = 0; sh < NSHAPE; sh++)
         if (b->grid[pi * NSHAPE + sh] > 0) shapes[n++] = sh;
     auto launch = [&](int sh, int k, cudaStream_t on) {
         const int p = pi * NSHAPE + sh;
         return launch_step(b->d_cases, b->d_tiles[p], 0, b->d_ntiles + p, b->grid[p], k, -1, prec_of_table(p),
-                           sh, on);
+                           sh, early, on);
     };
     cudaError_t e = cudaSuccess;
     if (n == 1) {
@@ -340,8 +340,8 @@ cudaError_t enqueue_chain(itlbm_batch *b, int pi, int k0, int k1, cudaStream_t s
 
 // Sub-steps [k0, k1) of every table on the batch stream: the storage forms hold different cases, so
 // one form runs in line and several run as parallel chains (fork, one chain per form on its own
-// stream, join), in a capture or directly.
-cudaError_t enqueue_steps(itlbm_batch *b, int k0, int k1) {
+// stream, join), in a capture or directly (`early`, see launch_step).
+cudaError_t enqueue_steps(itlbm_batch *b, int k0, int k1, bool early) {
     bool busy[NPREC] = {};
     int used = 0;
     for (int pi = 0; pi < NPREC; pi++) {
@@ -351,14 +351,14 @@ cudaError_t enqueue_steps(itlbm_batch *b, int k0, int k1) {
     cudaError_t e = cudaSuccess;
     if (used <= 1) {
         for (int pi = 0; pi < NPREC && e == cudaSuccess; pi++)
-            if (busy[pi]) e = enqueue_chain(b, pi, k0, k1, b->stream);
+            if (busy[pi]) e = enqueue_chain(b, pi, k0, k1, early, b->stream);
         return e;
     }
     if ((e = cudaEventRecord(b->ev_fork, b->stream)) != cudaSuccess) return e;
     for (int pi = 0; pi < NPREC; pi++) {
         if (!busy[pi]) continue;
         if ((e = cudaStreamWaitEvent(b->side[pi], b->ev_fork, 0)) != cudaSuccess) return e;
-        if ((e = enqueue_chain(b, pi, k0, k1, b->side[pi])) != cudaSuccess) return e;
+        if ((e = enqueue_chain(b, pi, k0, k1, early, b->side[pi])) != cudaSuccess) return e;
         if ((e = cudaEventRecord(b->ev_join[pi], b->side[pi])) != cudaSuccess) return e;
         if ((e = cudaStreamWaitEvent(b->stream, b->ev_join[pi], 0)) != cudaSuccess) return e;
     }
@@ -436,7 +436,7 @@ int capture_graph(itlbm_batch *b) {
     cudaGraph_t g;
     cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
     if (e != cudaSuccess) return cuda_fail(e, "begin capture");
-    const cudaError_t el = enqueue_steps(b, 0, b->cfg.chunk);
+    const cudaError_t el = enqueue_steps(b, 0, b->cfg.chunk, false);
     e = cudaStreamEndCapture(b->stream, &g);
     if (el != cudaSuccess) {
         if (e == cudaSuccess) cudaGraphDestroy(g);
@@ -475,7 +475,7 @@ int tune_and_run(itlbm_batch *b, int K) {
         b->mode = mode;
         set_grids(b);
         cudaEventRecord(b->tev[0], b->stream);
-        cudaError_t e = enqueue_steps(b, k0, k0 + M);
+        cudaError_t e = enqueue_steps(b, k0, k0 + M, true);
         cudaEventRecord(b->tev[1], b->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(b->tev[1]);
         float ms = 0;
@@ -507,7 +507,7 @@ int tune_and_run(itlbm_batch *b, int K) {
     b->tuning = false;
     set_grids(b);
     cudaError_t e;
-    if ((e = enqueue_steps(b, k0, K)) != cudaSuccess) return cuda_fail(e, "step launches");
+    if ((e = enqueue_steps(b, k0, K, true)) != cudaSuccess) return cuda_fail(e, "step launches");
     return capture_graph(b);
 }
 
@@ -1073,7 +1073,7 @@ int itlbm_batch_advance(itlbm_batch *b, void *stream) {
         e = cudaGraphLaunch(b->graph, b->stream);
         if (e != cudaSuccess) return cuda_fail(e, "graph launch");
     } else if (stepped) {
-        if ((e = enqueue_steps(b, 0, K)) != cudaSuccess) return cuda_fail(e, "step launches");
+        if ((e = enqueue_steps(b, 0, K, true)) != cudaSuccess) return cuda_fail(e, "step launches");
     }
     cudaEventRecord(b->ev1, b->stream);
     b->replays++;

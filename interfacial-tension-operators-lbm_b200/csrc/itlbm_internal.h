@@ -204,11 +204,11 @@ void fill_shift(CaseDev &c, double rho0, double u0x);
 
 // ---- kernel launchers (defined in the .cu files) -------------------------------------------
 cudaError_t launch_step_f64(const CaseDev *cases_dev, const TileRef *tiles, int ntiles,
-                            const int *ntiles_dev, int grid, int k, int aux_k, int shape, cudaStream_t s);
+                            const int *ntiles_dev, int grid, int k, int aux_k, int shape, bool early, cudaStream_t s);
 cudaError_t launch_step_f32(const CaseDev *cases_dev, const TileRef *tiles, int ntiles,
-                            const int *ntiles_dev, int grid, int k, int aux_k, int shape, cudaStream_t s);
+                            const int *ntiles_dev, int grid, int k, int aux_k, int shape, bool early, cudaStream_t s);
 cudaError_t launch_step_fold(const CaseDev *cases_dev, const TileRef *tiles, int ntiles,
-                             const int *ntiles_dev, int grid, int k, int aux_k, int shape, cudaStream_t s);
+                             const int *ntiles_dev, int grid, int k, int aux_k, int shape, bool early, cudaStream_t s);
 int step_occupancy_f64();
 int step_occupancy_f32();
 int step_occupancy(int prec);
@@ -227,9 +227,10 @@ cudaError_t case_bind(CaseDev &h, void *mem, size_t per_buf);
 // by default, since each shape is a launch of its own and a single case's steps are launch-bound
 // below about 10^6 nodes; the batch's autotuner chooses for itself.
 bool narrow_edges_default();
-// The step kernel of storage form `prec`; `shape` is the tile shape of every entry of `tiles`.
+// The step kernel of storage form `prec`; `shape` is the tile shape of every entry of `tiles`; `early` lets the
+// launch begin while the one before it in the stream ends (not in a graph, see launch_shape).
 cudaError_t launch_step(const CaseDev *cases_dev, const TileRef *tiles, int ntiles,
-                        const int *ntiles_dev, int grid, int k, int aux_k, int prec, int shape,
+                        const int *ntiles_dev, int grid, int k, int aux_k, int prec, int shape, bool early,
                         cudaStream_t s);
 cudaError_t launch_init(const CaseDev &c, const CaseDev *c_dev, const itlbm_case_desc &d,
                         cudaStream_t s);  // single cases: stages the profile, waits

@@ -308,8 +308,7 @@ __global__ void __launch_bounds__(STEP_THREADS, ITLBM_STEP_MIN_BLOCKS(FOLD)) k_s
     constexpr int Hh = R * STEP_THREADS / W;
     __shared__ SmemT<S, W, Hh> sm;
     // The next step's launch may begin while this one runs (its CTAs take the places that the last ones
-    // leave); each waits here until the step before it is complete.  Measured on B200, us per step: FP64 P3
-    // 300 x 300 16.6 -> 14.0, FP32 P3 512 x 512 18.4 -> 16.8, 2048 x 2048 235.6 -> 232.2, fold 125.1 -> 120.9.
+    // leave); each waits here until the step before it is complete.
     cudaTriggerProgrammaticLaunchCompletion();
     cudaGridDependencySynchronize();
     const int nt = ntiles_dev ? *ntiles_dev : ntiles;
@@ -323,7 +322,7 @@ __global__ void __launch_bounds__(STEP_THREADS, ITLBM_STEP_MIN_BLOCKS(FOLD)) k_s
 
 template <class S, bool FOLD>
 cudaError_t launch_shape(const CaseDev *cases_dev, const TileRef *tiles, int ntiles, const int *ntiles_dev,
-                         int grid, int k, int aux_k, int shape, cudaStream_t s) {
+                         int grid, int k, int aux_k, int shape, bool early, cudaStream_t s) {
     if (grid <= 0) return cudaSuccess;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3((unsigned)grid);
@@ -333,7 +332,11 @@ cudaError_t launch_shape(const CaseDev *cases_dev, const TileRef *tiles, int nti
     at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at.val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = &at;
-    cfg.numAttrs = 1;
+    // On a stream the early begin hides what lies between two launches; measured on B200, us per step: FP64 P3
+    // 300 x 300 16.6 -> 14.0, FP32 P3 512 x 512 18.4 -> 16.8, 2048 x 2048 235.6 -> 232.2, fold 125.1 -> 120.9.  In a
+    // graph there is less to hide and an early edge costs more: FP32 100 x 100 5.3 -> 8.0, eight of them 7.8 -> 9.8,
+    // 512 x 512 16.7 -> 17.4, fold 600 x 600 12.9 -> 13.6; larger launches differ by less than 1 %.
+    cfg.numAttrs = early ? 1 : 0;
     switch (shape) {
         case SHAPE_32x8: return cudaLaunchKernelEx(&cfg, k_step<S, FOLD, 32>, cases_dev, tiles, ntiles, ntiles_dev, k, aux_k);
         case SHAPE_16x16: return cudaLaunchKernelEx(&cfg, k_step<S, FOLD, 16>, cases_dev, tiles, ntiles, ntiles_dev, k, aux_k);
@@ -348,8 +351,8 @@ cudaError_t launch_shape(const CaseDev *cases_dev, const TileRef *tiles, int nti
 // rounds exactly as the reference's own code compiled with strict IEEE semantics) and without it.
 #ifdef ITLBM_STEP_F64
 cudaError_t launch_step_f64(const CaseDev *cases_dev, const TileRef *tiles, int ntiles,
-                            const int *ntiles_dev, int grid, int k, int aux_k, int shape, cudaStream_t s) {
-    return launch_shape<double, false>(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, s);
+                            const int *ntiles_dev, int grid, int k, int aux_k, int shape, bool early, cudaStream_t s) {
+    return launch_shape<double, false>(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, early, s);
 }
 // The occupancy queries also load every shape's kernel (with lazy module loading a kernel is loaded
 // at its first launch, which would otherwise fall inside the batch's first timed tuning window).
@@ -363,8 +366,8 @@ int step_occupancy_f64() {
 }
 #else
 cudaError_t launch_step_f32(const CaseDev *cases_dev, const TileRef *tiles, int ntiles,
-                            const int *ntiles_dev, int grid, int k, int aux_k, int shape, cudaStream_t s) {
-    return launch_shape<float, false>(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, s);
+                            const int *ntiles_dev, int grid, int k, int aux_k, int shape, bool early, cudaStream_t s) {
+    return launch_shape<float, false>(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, early, s);
 }
 int step_occupancy_f32() {
     int n = 0;
@@ -378,8 +381,8 @@ int step_occupancy_f32() {
     return n;
 }
 cudaError_t launch_step_fold(const CaseDev *cases_dev, const TileRef *tiles, int ntiles,
-                             const int *ntiles_dev, int grid, int k, int aux_k, int shape, cudaStream_t s) {
-    return launch_shape<float, true>(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, s);
+                             const int *ntiles_dev, int grid, int k, int aux_k, int shape, bool early, cudaStream_t s) {
+    return launch_shape<float, true>(cases_dev, tiles, ntiles, ntiles_dev, grid, k, aux_k, shape, early, s);
 }
 #endif
 

@@ -160,3 +160,20 @@ def test_a_case_loads_only_what_its_plan_looks_at(gpu, nx, prec, most):
             f"c = m.Case(m.desc({nx}, {nx}, m.make_op(3, 0.5), radius=9, precision={prec}))\n"
             f"assert c.plan().bx and 1 <= m.lib().itlbm_internal_configurations() <= {most}")
     subprocess.run([sys.executable, "-c", code], cwd=REPO, check=True)
+
+
+@pytest.mark.parametrize("prec", [0, 1, 2])
+def test_captured_steps_have_full_dependencies(gpu, prec):
+    """Steps in a graph follow one another by plain edges: an early begin makes a graph of small steps slower."""
+    L = C.CDLL("libcuda.so.1")
+    s, g, n = C.c_void_p(), C.c_void_p(), C.c_size_t(64)
+    with make(gpu, 40, 50, 3, prec) as c:
+        c.step(2)
+        c.sync()
+        assert L.cuStreamCreate(C.byref(s), 1) == 0 and L.cuStreamBeginCapture_v2(s, 1) == 0
+        c.step(5, stream=s)
+        assert L.cuStreamEndCapture(s, C.byref(g)) == 0
+        src, dst, data = (C.c_void_p * 64)(), (C.c_void_p * 64)(), ((C.c_ubyte * 8) * 64)()
+        assert L.cuGraphGetEdges_v2(g, src, dst, data, C.byref(n)) == 0
+        assert n.value == 4 and all(data[i][2] == 0 for i in range(4))  # CU_GRAPH_DEPENDENCY_TYPE_DEFAULT
+        assert L.cuGraphDestroy(g) == 0 and L.cuStreamDestroy_v2(s) == 0

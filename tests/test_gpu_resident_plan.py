@@ -177,3 +177,24 @@ def test_captured_steps_have_full_dependencies(gpu, prec):
         assert L.cuGraphGetEdges_v2(g, src, dst, data, C.byref(n)) == 0
         assert n.value == 4 and all(data[i][2] == 0 for i in range(4))  # CU_GRAPH_DEPENDENCY_TYPE_DEFAULT
         assert L.cuGraphDestroy(g) == 0 and L.cuStreamDestroy_v2(s) == 0
+
+
+@pytest.mark.parametrize("prec,small,large", [(1, 128, 160), (2, 128, 256)])
+def test_steps_one_by_one_do_not_crowd(gpu, prec, small, large):
+    """The CTAs of both boxes find an SM each, so single steps of the larger take about as long (1.6 times where those
+    of several steps waited side by side)."""
+    import torch
+    us = []
+    for n in (small, large):
+        with make(gpu, n, n, 12, prec) as c:
+            times = []
+            for _ in range(7):
+                e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+                e0.record(torch.cuda.default_stream())
+                for _ in range(200):
+                    c.step(1)
+                e1.record(torch.cuda.default_stream())
+                torch.cuda.synchronize()
+                times.append(e0.elapsed_time(e1))
+            us.append(min(times))
+    assert us[1] < 1.3 * us[0], us

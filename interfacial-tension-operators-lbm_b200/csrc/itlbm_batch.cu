@@ -458,7 +458,9 @@ long long updates_in(const itlbm_batch *b, int k0, int k1) {
 }
 
 // Autotuning on the first full replay of at least 18 sub-steps, in timed windows of
-// M = max(6, K / 16) sub-steps (CUDA events, rate per node update): the tiling -- narrow tiles at the partial last tile column of a case against
+// M = max(6, K / 16) sub-steps (CUDA events, rate per node update; launched with the graph's full dependencies, since
+// an early begin favours one CTA per entry: fold F1 800 x 800 24.4 us per step with persistent CTAs, which it chooses
+// so, 26.3 without): the tiling -- narrow tiles at the partial last tile column of a case against
 // 32 x 8 tiles throughout -- with one CTA per table entry, then persistent CTAs at the occupancy limit
 // with the better tiling.  The faster of each runs the rest of the replay and is captured into the
 // graph.  Every choice runs the same arithmetic on every node, so the results do not depend on it.
@@ -475,7 +477,7 @@ int tune_and_run(itlbm_batch *b, int K) {
         b->mode = mode;
         set_grids(b);
         cudaEventRecord(b->tev[0], b->stream);
-        cudaError_t e = enqueue_steps(b, k0, k0 + M, true);
+        cudaError_t e = enqueue_steps(b, k0, k0 + M, false);
         cudaEventRecord(b->tev[1], b->stream);
         if (e == cudaSuccess) e = cudaEventSynchronize(b->tev[1]);
         float ms = 0;

@@ -213,20 +213,30 @@ bool resident_form(const itlbm_batch *b, int prec) { return b->resident_steps >=
 
 // The resident launches of the active cases: per storage form and configuration the cases with the most
 // tiles first (they need the most CTAs at once; the small ones fill what those leave), in queues over all
-// the CTAs the device holds.
+// the CTAs the device holds.  Where the work tables have cases anyway, those of a launch too small to pay for its
+// time go there too (res_min_nodes).
 int build_resident(itlbm_batch *b) {
+    bool tables = false;
+    for (Active *a : b->slots) {
+        if (!a) continue;
+        a->resident = false;
+        tables = tables || (!a->held && !(resident_form(b, a->desc.precision) && a->plan.shape >= 0));
+    }
     for (int pi = 0; pi < NPREC; pi++)
         for (int shape = 0; shape < NRES; shape++) {
             itlbm_batch::Resident &X = b->res[pi][shape];
             const int prec = prec_of_table(pi * NSHAPE);
             std::vector<ResCase> cs;
+            double nodes = 0;
             X.ctas = X.cases = 0;
             if (!resident_form(b, prec)) continue;
             for (const Active *a : b->slots)
-                if (a && !a->held && a->desc.precision == prec && a->plan.shape == shape)
+                if (a && !a->held && a->desc.precision == prec && a->plan.shape == shape) {
                     // a tile of F1 / F2 takes about 1.3 times as long per step as the others
                     cs.push_back(ResCase{a->plan, a->slot,
                                          a->desc.op.tipo == ITLBM_OP_F1 || a->desc.op.tipo == ITLBM_OP_F2 ? 1.3 : 1.0});
+                    nodes += (double)a->desc.nx * a->desc.ny;
+                }
             if (cs.empty()) continue;
             std::stable_sort(cs.begin(), cs.end(),
                              [](const ResCase &x, const ResCase &y) { return x.plan.tiles > y.plan.tiles; });
@@ -234,6 +244,7 @@ int build_resident(itlbm_batch *b) {
             for (const ResCase &k : cs) tiles = std::min(tiles + k.plan.tiles, 1 << 24);
             const int cap = res_capacity(prec, shape), ctas = std::min(cap, tiles);
             const ResQueues q = res_queues(cs, ctas);
+            if (tables && nodes < res_min_nodes(prec, shape) * q.length) continue;
             cudaError_t e = cudaSuccess;
             if (q.bytes() > X.cap) {
                 if (X.queues) cudaFree(X.queues);
@@ -254,6 +265,7 @@ int build_resident(itlbm_batch *b) {
                 return cuda_fail(e, "resident tile queues");
             X.ctas = ctas;
             X.cases = (int)cs.size();
+            for (const ResCase &k : cs) b->slots[k.case_id]->resident = true;
         }
     return ITLBM_OK;
 }
@@ -266,9 +278,7 @@ int upload_tables(itlbm_batch *b) {
         build_resident(b);
     }
     for (Active *a : b->slots) {
-        if (!a || a->held) continue;
-        a->resident = resident_form(b, a->desc.precision) && a->plan.shape >= 0;
-        if (a->resident) continue;
+        if (!a || a->held || a->resident) continue;
         const CaseDev &c = b->h_cases[a->slot];
         case_tiles(c, b->narrow, a->slot, &t[table_of(a->desc.precision) * NSHAPE]);
     }

@@ -109,6 +109,17 @@ constexpr int RES_POLLS = 1 << 23;
 // and 12.8 / 15.4 (600 cases 15.2 / 14.9), 40 steps 14.5 / 16.4 and 12.8 / 17.2; fold 20 steps 28.9 / 25.7 and
 // 24.3 / 25.9, 40 steps 28.9 / 28.8 and 24.2 / 27.4, 80 steps 28.0 / 30.7 and 24.3 / 30.4.
 inline int res_min_replay(int prec) { return prec == ITLBM_PREC_F32_FOLD ? 40 : 24; }
+// Nodes that a batch's launch must hold per unit of its queues' length (the time of one tile), where the batch has
+// cases for the work tables too: added to these, a node costs what it does at their full rate (FP64 7.4 G updates/s,
+// FP32 12, fold 22), while a launch takes as long for one tile as for all its places (4.3 to 7 us per step by FP64
+// configuration, 4.1 and 3.6 us).  One FP32 512 x 512 box and m others, ms per 500 steps with all in the tables / the
+// others resident first: FP64 1 x 64^2 8.9 / 11.3, 4 x 100^2 (40 000 nodes, one unit) 11.1 / 12.0, 16 x 64^2 (65 500, one)
+// 12.4 / 12.2, 16 x 100^2 21.2 / 18.7, 1 x 200^2 (40 000 in smaller tiles) 10.7 / 10.9, 4 x 200^2 18.5 / 17.5; FP32
+// 1 x 64^2 8.7 / 10.7, 4 x 100^2 10.3 / 10.8, 16 x 64^2 10.4 / 10.7, 4 x 200^2 15.7 / 13.5; fold 1 x 64^2 9.0 / 10.3,
+// 4 x 200^2 10.4 / 11.2, 16 x 100^2 (160 000, one) 11.1 / 11.2, 16 x 200^2 18.6 / 18.3.  (Run beside the tables instead
+// of before them, small launches gain a little on that, 1 x 64^2 fold 8.7, but both slow down when they share SMs:
+// 4 x 100^2 FP64 13.5, beside an FP32 1024 x 1024 box 51 against 35.)
+double res_min_nodes(int prec, int shape);
 
 
 // How a case is held on chip: the tile configuration and the bx x by tiles, or shape < 0 when the box
@@ -135,6 +146,7 @@ struct ResCase {
 struct ResQueues {
     std::vector<ResTile> tiles;
     std::vector<int> first, slots;
+    double length = 0;  // when the last queue ends
     size_t bytes() const { return sizeof(ResTile) * tiles.size() + sizeof(int) * (first.size() + slots.size()); }
 };
 ResQueues res_queues(const std::vector<ResCase> &cases, int ctas);

@@ -198,6 +198,10 @@ ResPlan res_plan_batch(int prec, int nx, int ny) {
     return ResPlan();
 }
 
+double res_min_nodes(int prec, int shape) {
+    return prec == ITLBM_PREC_F64 ? 0.65 * res_capacity(prec, shape) * res_nodes(shape) : prec == ITLBM_PREC_F32 ? 60e3 : 180e3;
+}
+
 ResQueues res_queues(const std::vector<ResCase> &cases, int ctas) {
     ResQueues Q;
     std::vector<std::vector<ResTile>> queue(ctas);
@@ -215,6 +219,7 @@ ResQueues res_queues(const std::vector<ResCase> &cases, int ctas) {
             queue[c].push_back(ResTile{k.case_id, t, peers, order, (unsigned short)k.plan.bx, (unsigned short)k.plan.by});
             load[t].first = end;
         }
+        Q.length = std::max(Q.length, end);
         order++;
     }
     Q.first.push_back(0);

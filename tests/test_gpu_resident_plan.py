@@ -198,3 +198,30 @@ def test_steps_one_by_one_do_not_crowd(gpu, prec, small, large):
                 times.append(e0.elapsed_time(e1))
             us.append(min(times))
     assert us[1] < 1.3 * us[0], us
+
+
+@pytest.mark.parametrize("prec,few,many", [(0, 4, 16), (1, 4, 16), (2, 4, 60)])
+def test_few_small_cases_go_with_the_tables(gpu, prec, few, many):
+    """Beside a box that the device does not hold, small cases are resident only where they are enough to fill it;
+    which way they go changes no bit.  When that box is gone, and when there is none, they always are."""
+    def desc(n, t, p):
+        return gpu.desc(n, n, gpu.make_op(t, 0.5), tau=0.83, A_fact=0.2 if t < 11 else 0.08, radius=0.23 * n, precision=p)
+
+    fields = []
+    for boxes, steps in (([(640, 3, 1)] + [(100, 3, prec)] * few, 121), ([(640, 3, 1)] + [(100, 3, prec)] * many, 121),
+                         ([(100, 3, prec)] * few, 121)):
+        with gpu.Batch(chunk=60, diag_every=60) as b:
+            b.hold_finished(True)
+            for tag, box in enumerate(boxes):
+                b.submit(desc(*box), steps if box[0] == 100 else 61, tag)
+            b.advance()
+            b.advance()
+            large = boxes[0][0] == 640
+            assert (b.plan(len(boxes) - 1).bx > 0) == (not large or len(boxes) > 1 + few)
+            if large:
+                assert b.plan(0).bx == 0 and b.stats().finished == 1
+            b.advance()
+            assert b.plan(len(boxes) - 1).bx > 0 and b.stats().finished == len(boxes)
+            fields.append(b.read_fields(len(boxes) - 1, 100 * 100))
+    for f in fields[1:]:
+        assert all((f[k] == fields[0][k]).all() for k in f)

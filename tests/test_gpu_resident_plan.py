@@ -225,3 +225,13 @@ def test_few_small_cases_go_with_the_tables(gpu, prec, few, many):
             fields.append(b.read_fields(len(boxes) - 1, 100 * 100))
     for f in fields[1:]:
         assert all((f[k] == fields[0][k]).all() for k in f)
+
+
+def test_boxes_without_a_partial_column_do_not_choose_narrow_tiles(gpu):
+    """Their tilings are the same, and the choice holds for every case that the batch gets later."""
+    for _ in range(8):
+        with gpu.Batch(chunk=40) as b:
+            b.submit(gpu.desc(512, 512, gpu.make_op(3, 0.5), tau=0.83, radius=100, precision=1), 1000, 1)
+            for _ in range(3):
+                b.advance()
+            assert b.stats().narrow_edges == 0

@@ -141,11 +141,13 @@ struct itlbm_batch {
     int ntab[NTAB] = {};  // current table lengths
     int occ[NTAB] = {};   // resident CTAs per SM of each table's step kernel
     // launch shape: -1 = one CTA per table entry, 0 = persistent CTAs at the occupancy limit, k > 0 =
-    // k persistent CTAs per SM; with ctas_per_sm = 0 the first full replay times -1 against 0
+    // k persistent CTAs per SM; with ctas_per_sm = 0 a full replay times -1 against 0: the first, and one whose
+    // tables have grown to twice those of the last time (a choice made on one case is not that of a mix)
     int mode = -1;
     bool tuning = false;
+    int tuned = 0;  // entries of the tables it was last timed on
     // a partial last tile column of a case in narrow tiles (16 x 16, 8 x 32) instead of 32 x 8; with
-    // ctas_per_sm = 0 the first full replay times both tilings and keeps the faster (on the measured
+    // ctas_per_sm = 0 the same replays time both tilings and keep the faster (on the measured
     // mixes 32 x 8 throughout, which is also the tiling without autotuning)
     bool narrow = false;
     bool tile_fixed = false;  // the tiling was set by the caller, not timed
@@ -467,7 +469,7 @@ long long updates_in(const itlbm_batch *b, int k0, int k1) {
     return u;
 }
 
-// Autotuning on the first full replay of at least 18 sub-steps, in timed windows of
+// Autotuning on the first full replay of at least 18 sub-steps, and again when the tables have doubled since, in timed windows of
 // M = max(6, K / 16) sub-steps (CUDA events, rate per node update; launched with the graph's full dependencies, since
 // an early begin favours one CTA per entry: fold F1 800 x 800 24.4 us per step with persistent CTAs, which it chooses
 // so, 26.3 without): the tiling -- narrow tiles at the partial last tile column of a case against
@@ -520,7 +522,8 @@ int tune_and_run(itlbm_batch *b, int K) {
         if ((r = upload_tables(b)) != ITLBM_OK) return r;
     }
     b->mode = mode;
-    b->tuning = false;
+    b->tuned = 0;
+    for (int p = 0; p < NTAB; p++) b->tuned += b->ntab[p];
     set_grids(b);
     cudaError_t e;
     if ((e = enqueue_steps(b, k0, K, true)) != cudaSuccess) return cuda_fail(e, "step launches");
@@ -1078,10 +1081,14 @@ int itlbm_batch_advance(itlbm_batch *b, void *stream) {
         b->tables_dirty = false;
     }
     bool stepped = false;  // cases stepped from the work tables
-    for (int p = 0; p < NTAB; p++) stepped = stepped || b->grid[p] > 0;
+    int entries = 0;
+    for (int p = 0; p < NTAB; p++) {
+        stepped = stepped || b->grid[p] > 0;
+        entries += b->ntab[p];
+    }
     cudaEventRecord(b->ev0, b->stream);
     if ((e = enqueue_resident(b, K)) != cudaSuccess) return cuda_fail(e, "resident step launches");
-    if (stepped && b->tuning && K == b->cfg.chunk && K >= 3 * TUNE_MIN_WINDOW) {
+    if (stepped && b->tuning && entries >= 2 * b->tuned && K == b->cfg.chunk && K >= 3 * TUNE_MIN_WINDOW) {
         r = tune_and_run(b, K);
         if (r) return r;
     } else if (stepped && K == b->cfg.chunk) {

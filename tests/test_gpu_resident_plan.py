@@ -235,3 +235,28 @@ def test_boxes_without_a_partial_column_do_not_choose_narrow_tiles(gpu):
             for _ in range(3):
                 b.advance()
             assert b.stats().narrow_edges == 0
+
+
+def test_tables_that_grow_are_timed_again(gpu):
+    """The windows of a second timing, on tables that have doubled, are steps like any others."""
+    def desc(n, t, p):
+        return gpu.desc(n, n, gpu.make_op(t, 0.5), tau=0.83, A_fact=0.2 if t < 11 else 0.08, radius=0.23 * n, precision=p)
+
+    boxes = [(430, 3, 1), (301, 12, 0), (433, 11, 1), (590, 13, 2), (420, 1, 1)]
+    with gpu.Batch(chunk=40, diag_every=40) as b:
+        b.hold_finished(True)
+        b.submit(desc(*boxes[0]), 161, 0)
+        b.advance()
+        b.advance()
+        for tag, box in enumerate(boxes[1:], 1):
+            b.submit(desc(*box), 81, tag)
+        while b.stats().finished < len(boxes):
+            b.advance()
+        for tag, (n, t, p) in enumerate(boxes):
+            got = b.read_fields(tag, n * n)
+            with gpu.Case(desc(n, t, p)) as c:
+                for _ in range(160 if tag == 0 else 80):
+                    c.step(1)
+                c.step(1, keep_aux=True)
+                want = c.read_fields()
+            assert all((got[k] == want[k]).all() for k in want), tag

@@ -28,9 +28,9 @@ namespace itlbm {
 // four operations: q = a (y + yl) to half an ulp and a bit, its exact remainder, and Markstein's final
 // step q + (a - b q) y (P. Markstein, IBM J. Res. Dev. 34, 1990), which rounds as a / b does: it lands
 // within |a/b - q| |1 - b y| <= (1/2 + 2^-50) 2^-54 m_b ulp of a / b, m_b the mantissa of b, and no
-// quotient lies nearer than 2^-53 / m_b ulp to a rounding boundary -- unless the mantissa of b is all
-// ones, which `ok` leaves to the plain division, like operands whose exponents could make a product
-// or a remainder inexact.  A zero dividend gives a zero whose sign may differ: it is only added to or
+// quotient lies nearer than 2^-53 / m_b ulp to a rounding boundary.  The first is the smaller as long as
+// m_b^2 (1 + 2^-49) < 4, that is for m_b up to 2 - 9 x 2^-52; `ok` leaves the divisors above 2 - 17 x 2^-52 to
+// the plain division, like operands whose exponents could make a product or a remainder inexact.  A zero dividend gives a zero whose sign may differ: it is only added to or
 // multiplied with other terms.  Measured on B200, resident FP64 step: 100 x 100 P3 6.3 -> 3.6 us, 256 x 256
 // F2 10.9 -> 9.2 us (the divisions' dependent chains were most of a small tile's step); k_step, which
 // waits for memory, F1 1000 x 1000 164 -> 159 us.
@@ -41,8 +41,8 @@ struct Recip64 {
         const double q = __fma_rn(a, y, a * yl);
         return __fma_rn(__fma_rn(-b, q, a), y, q);
     }
-    // mantissa of a divisor not all ones (its low word is enough)
-    __device__ __forceinline__ static bool ok(double d) { return __double2loint(d) != -1; }
+    // mantissa of a divisor not among the largest (its low word is enough)
+    __device__ __forceinline__ static bool ok(double d) { return (unsigned)__double2loint(d) < 0xFFFFFFF0u; }
 };
 // a / b by a call: the rare operands outside Recip64's range, kept out of the kernels' instruction stream
 static __device__ __noinline__ double div_plain(double a, double b) { return a / b; }

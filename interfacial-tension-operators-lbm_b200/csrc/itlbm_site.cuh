@@ -774,21 +774,6 @@ __device__ __forceinline__ T chem_pot_at(P phi, T kf, T bf) {
     return T(4) * bf * ph * (ph * ph - T(1)) - kf * lap;
 }
 
-// the same on a staged 2-D tile at position (px, py)
-template <class T, int W_>
-__device__ __forceinline__ void mediator_grad(const T (*phi)[W_], int px, int py, T &gx, T &gy,
-                                              T &gz) {
-    mediator_grad_at<T>([&](int dx, int dy) { return phi[py + dy][px + dx]; }, gx, gy, gz);
-}
-template <class T, int W_>
-__device__ __forceinline__ void iso_grad(const T (*phi)[W_], int px, int py, T &gx, T &gy, T &gz) {
-    iso_grad_at<T>([&](int dx, int dy) { return phi[py + dy][px + dx]; }, gx, gy, gz);
-}
-template <class T, int W_>
-__device__ __forceinline__ T chem_pot(const T (*phi)[W_], int px, int py, T kf, T bf) {
-    return chem_pot_at<T>([&](int dx, int dy) { return phi[py + dy][px + dx]; }, kf, bf);
-}
-
 // F1 unit normal (Operadores_tensao.cpp:251-258) and F2 stress (:259-272) from the gradient.
 template <class T>
 __device__ __forceinline__ void aux_normal(T gx, T gy, T gz, T *a) {
@@ -864,16 +849,6 @@ __device__ __forceinline__ void stress_div_at(A aux, T &Fx, T &Fy, T &Fz) {
     Fx = T(3) * ax;
     Fy = T(3) * ay;
     Fz = T(3) * az;
-}
-
-template <class T, int AS, int W_>
-__device__ __forceinline__ T curvature(const T (*aux)[W_][AS], int qx, int qy) {
-    return curvature_at<T>([&](int dx, int dy) { return aux[qy + dy][qx + dx]; });
-}
-template <class T, int AS, int W_>
-__device__ __forceinline__ void stress_div(const T (*aux)[W_][AS], int qx, int qy, T &Fx, T &Fy,
-                                           T &Fz) {
-    stress_div_at<T>([&](int dx, int dy) { return aux[qy + dy][qx + dx]; }, Fx, Fy, Fz);
 }
 
 }  // namespace itlbm

@@ -12,8 +12,9 @@
 #include <atomic>
 #include <condition_variable>
 #include <cstring>
+#include <exception>
 #include <mutex>
-#include <system_error>
+#include <new>
 #include <thread>
 
 namespace itlbm {
@@ -85,15 +86,17 @@ struct Chunk {
 // Chunk c comes into slot c mod SLOTS once the chunk before it there is copied out; the workers take the
 // chunks in order.
 cudaError_t fetch_large(const std::vector<Chunk> &chunks, cudaStream_t st) {
-    cudaEvent_t ev[SLOTS] = {};
-    cudaError_t e = cudaSuccess;
-    for (auto &v : ev)
-        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
     const size_t n = chunks.size(), slot = g_stage.cap / SLOTS;
     std::mutex m;
     std::condition_variable cv;
     size_t issued = 0, next = 0;
     std::vector<char> done(n, 0);
+    std::vector<std::thread> pool;
+    pool.reserve(WORKERS);
+    cudaEvent_t ev[SLOTS] = {};
+    cudaError_t e = cudaSuccess;
+    for (auto &v : ev)
+        if (e == cudaSuccess) e = cudaEventCreateWithFlags(&v, cudaEventDisableTiming);
     cudaError_t worker_error = cudaSuccess;
     bool stop = false;
     int device = 0;
@@ -116,13 +119,11 @@ cudaError_t fetch_large(const std::vector<Chunk> &chunks, cudaStream_t st) {
             cv.notify_all();
         }
     };
-    std::vector<std::thread> pool;
-    pool.reserve(WORKERS);
     if (e == cudaSuccess) {
         const size_t want = std::min<size_t>({n, (size_t)WORKERS, std::max(1u, std::thread::hardware_concurrency())});
         try {
             while (pool.size() < want) pool.emplace_back(work);
-        } catch (const std::system_error &) {  // fewer threads
+        } catch (const std::exception &) {  // no thread or no memory to be had: fewer threads
         }
         if (pool.empty()) {
             for (auto &v : ev)
@@ -183,12 +184,16 @@ cudaError_t fetch_arrays(double *const *dst, int n, size_t each, const double *s
     }
     if (total < LARGE || !reserve(total < HUGE_READ ? MEDIUM_STAGE : HUGE_STAGE)) return fetch_plain(dst, n, each, src, st);
     const size_t most = g_stage.cap / SLOTS;
-    std::vector<Chunk> chunks;
-    for (int k = 0; k < n; k++)
-        for (size_t at = 0; dst[k] && at < sizeof(double) * each; at += most)
-            chunks.push_back(Chunk{(char *)dst[k] + at, (const char *)(src + k * each) + at,
-                                   std::min(most, sizeof(double) * each - at)});
-    const cudaError_t e = fetch_large(chunks, st);
+    cudaError_t e = cudaErrorNotReady;
+    try {
+        std::vector<Chunk> chunks;
+        for (int k = 0; k < n; k++)
+            for (size_t at = 0; dst[k] && at < sizeof(double) * each; at += most)
+                chunks.push_back(Chunk{(char *)dst[k] + at, (const char *)(src + k * each) + at,
+                                       std::min(most, sizeof(double) * each - at)});
+        e = fetch_large(chunks, st);
+    } catch (const std::bad_alloc &) {  // before any copy began
+    }
     return e == cudaErrorNotReady ? fetch_plain(dst, n, each, src, st) : e;
 }
 

@@ -239,11 +239,11 @@ int  itlbm_snapshot_info(const char *path, itlbm_case_desc *desc, long long *ste
 /* ---- batches: many cases stepped together ------------------------------------------------- */
 /* The batched form of the loop Imm_OPS.cpp:246-372 / Imm_INCL.cpp:358-442 for many independent
  * cases, replacing the process pool of rodar_lote.py (rodar_lote.py:231-243, :300-318).  Admitted
- * cases keep their state on the device; each advance runs the resident kernel or a CUDA graph of step launches
- * over a device-resident tile work table (every case's tiles, FP32 and FP64 cases side by side),
- * stops every case at its next diagnostic step (every 500 steps and the last, Imm_OPS.cpp:293),
- * measures it there and retires it at its step count or when it becomes unstable
- * (Imm_OPS.cpp:346-352). */
+ * cases keep their state on the device; each advance steps the cases that fit it on chip in launches of many
+ * steps (see itlbm_plan) and the others by a CUDA graph of single-step launches over a device-resident tile
+ * work table (every such case's tiles, FP32 and FP64 cases side by side), stops every case at its next
+ * diagnostic step (every 500 steps and the last, Imm_OPS.cpp:293), measures it there and retires it at its
+ * step count or when it becomes unstable (Imm_OPS.cpp:346-352). */
 typedef struct itlbm_batch itlbm_batch;
 
 typedef struct itlbm_batch_config {
@@ -253,10 +253,10 @@ typedef struct itlbm_batch_config {
     int    diag_every;        /* diagnostic interval; 0 = 500                                     */
     int    ctas_per_sm;       /* launch shape of the step kernels: < 0 = one CTA per tile of the   */
                               /* work table; > 0 = that many persistent CTAs per SM striding over */
-                              /* it; 0 = autotune: the first full replay times the tilings (narrow */
-                              /* edge tiles or 32 x 8 throughout) and the two launch shapes        */
-                              /* (persistent at the occupancy limit) and keeps the faster of each  */
-                              /* (same results)                                                     */
+                              /* it; 0 = autotune: the first full replay, and one whose tables have */
+                              /* doubled since, times the tilings (narrow edge tiles or 32 x 8      */
+                              /* throughout) and the two launch shapes (persistent at the occupancy */
+                              /* limit) and keeps the faster of each (same results)                 */
 } itlbm_batch_config;
 
 enum { ITLBM_EV_DIAG = 0, ITLBM_EV_DONE = 1, ITLBM_EV_UNSTABLE = 2 };

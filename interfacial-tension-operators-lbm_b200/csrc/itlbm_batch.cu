@@ -8,7 +8,8 @@
 //   * tile work tables list the TX x TY tiles of every active case, one per storage form (FP64, FP32,
 //     FP32 fold), with their lengths in device memory;
 //   * cases whose tiles fit the device run a whole replay in the resident kernel (itlbm_resident.cu), as
-//     one launch per storage form; the rest are stepped from the work tables;
+//     one launch per storage form and tile configuration; the rest are stepped from the work tables, and with them
+//     the cases of a launch that would hold too few nodes (res_min_nodes);
 //   * one replay of the tables is a CUDA graph of `chunk` sub-steps: each non-empty table is a chain of launches on
 //     its own stream between a fork and a join, one CTA per table entry (the grid is the table length
 //     rounded up to a bucket); a case whose chunk is shorter skips its tiles in the remaining

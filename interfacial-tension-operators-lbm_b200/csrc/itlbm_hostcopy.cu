@@ -5,7 +5,7 @@
 // box, a quarter of a 500-step interval's time), and every small array costs a synchronous copy of its
 // own (five fields of a 40 x 40 box: 90 us).  Here the data comes through pinned memory: what fits it in
 // one copy and one wait, larger data in chunks that several threads copy out (and fault in) while the
-// next ones arrive: 2048 x 2048 in 9 ms, 40 x 40 in 37 us.
+// next ones arrive: 2048 x 2048 in 11 ms, 40 x 40 in 37 us.
 #include "itlbm_internal.h"
 
 #include <algorithm>

@@ -1,14 +1,14 @@
 // itlbm_resident.cu -- many time steps in one launch, the state of every case held on chip.
 //
 // k_step (itlbm_step.cu) reads and writes the whole state in HBM every step, and a box of a few
-// hundred nodes a side cannot hide what that costs: on B200 one FP64 step of a 100 x 100 drop took
-// 11 us, of which the launch, the dependent loads of the tile's descriptors and the two round trips
-// for the node and halo loads are most.  Here a CTA keeps one tile of one case for all the steps of a
+// hundred nodes a side cannot hide what that costs: on B200 one FP64 step of a 100 x 100 drop takes
+// 7.1 us (3.4 here), of which the launch, the dependent loads of the tile's descriptors and the two round
+// trips for the node and halo loads are most.  Here a CTA keeps one tile of one case for all the steps of a
 // launch: its populations live in shared memory, and per step only what crosses a tile's edge goes
 // through L2, to the CTAs that hold the neighbouring tiles.  All CTAs are resident at once (a
 // cooperative launch), since they wait for one another.
 //
-// Step of a tile of w x h nodes, one node per thread (R in the fold):
+// Step of a tile of w x h nodes, R per thread (one; two or four in some FP32 and fold configurations):
 //   1. each thread takes its node's planes from shared memory, forms rho^N, and posts it when the
 //      node lies within the stencil's reach of the tile's edge;
 //   2. the halo's rho^N are taken from the tiles that own those nodes;
@@ -35,8 +35,8 @@
 // Every wait is bounded: a wait that runs out sets *err and the CTA returns at the end of its step,
 // as do its neighbours in turn.
 //
-// The tile's shape is free (w h <= threads, see res_plan): a 100 x 100 box is 4 x 10 tiles of 25 x 10
-// nodes.  A node's arithmetic does not depend on the tile, so the results are those of k_step to the
+// The tile's shape is free within a configuration's nodes and half perimeter (best_tiling in itlbm_resplan.cu): a
+// 100 x 100 FP64 box alone is 13 x 13 tiles of 8 x 8 nodes at most.  A node's arithmetic does not depend on the tile, so the results are those of k_step to the
 // bit.
 #include "itlbm_node.cuh"
 #include "itlbm_resident.h"
@@ -132,7 +132,7 @@ __device__ __forceinline__ bool wait_for(const ResArgs &a, const unsigned *done,
     return true;
 }
 
-// first coordinate of tile t of n nodes cut into b tiles (res_tiling keeps the product in 32 bits)
+// first coordinate of tile t of n nodes cut into b tiles (best_tiling keeps the product in 32 bits)
 __device__ __forceinline__ int tile_begin(int t, int n, int b) { return (int)((unsigned)t * (unsigned)n / (unsigned)b); }
 
 // Of a CTA's tile: its case, its place and size, and what the loop needs of them.

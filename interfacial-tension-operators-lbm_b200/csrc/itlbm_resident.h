@@ -94,10 +94,12 @@ inline cudaError_t res_launch(int prec, int shape, const ResArgs &a, int grid, c
 }
 
 
-// Steps a call must ask for to take the resident kernel, and the most one launch runs.  Its launch
-// costs 20 us (tables, first loads) where a k_step launch costs 8, so it gains from about four steps on:
-// call and synchronisation on a 100^2 drop, k_step / resident, 4 steps: FP64 53 / 52, FP32 34 / 37, fold
-// 39 / 29 us; 6 steps: 76 / 64, 46 / 42, 56 / 34 us.
+// Steps a call must ask for to take the resident kernel, and the most one launch runs.  Its launch costs 20 us
+// (tables, first loads) where a k_step launch costs 8, so most boxes gain from about five steps on, the largest from
+// seven or eight: call and synchronisation, us, k_step / resident, 6 steps: FP64 40 x 40 51.6 / 41.4, 100 x 100
+// 52.3 / 46.5, F2 256 x 256 86.7 / 73.8; FP32 100 x 100 40.6 / 42.1, 256 x 256 49.1 / 44.0, 380 x 380 70.1 / 72.3; fold
+// 100 x 100 42.8 / 33.9, 500 x 500 68.3 / 75.9; 10 steps: 77.7 / 55.1, 80.6 / 60.1, 136.8 / 108.1; 61.5 / 52.3,
+// 75.5 / 56.8, 110.3 / 94.2; 64.8 / 43.0, 107.5 / 101.3.
 constexpr int RES_MIN_STEPS = 6;
 constexpr int RES_MAX_STEPS = 4096;
 // Polls without a finished tile, each a trip to L2: some 3 s.  The longest that a tile takes is RES_MAX_STEPS

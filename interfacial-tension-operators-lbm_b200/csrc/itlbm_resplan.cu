@@ -134,7 +134,7 @@ double best_tiling(int prec, int nx, int ny, int shape, ResPlan &p, COST cost) {
 
 // A case alone.  The smallest configuration that holds it: few warps share an SM, and each step ends the
 // sooner (us per step, P3, 64 / 128 / 256 threads: FP64 100^2 3.6 / 3.8 / 5.4, FP32 100^2 2.70 / 2.75 / 3.2,
-// 256^2 3.46 / 3.42 / 3.9, fold 256^2 2.86 / 2.90 / 3.0; k_step 9.1, 6.8, 8.2, 8.2), in the fewest tiles, or
+// 256^2 3.46 / 3.42 / 3.9, fold 256^2 2.86 / 2.90 / 3.0; k_step 7.1, 5.1, 6.6, 5.8), in the fewest tiles, or
 // with 256 threads in as many as leave the fewest warps on the fullest SM (FP64 200^2 5.96 against 6.20).
 // FP64 F1 / F2 also pass over the ring-1 region, a second time when it has more nodes than the CTA threads:
 // there the configuration and tiling with the fewest warps on the fullest SM, the region's counted half

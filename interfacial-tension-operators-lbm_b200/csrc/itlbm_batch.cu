@@ -504,13 +504,15 @@ int tune_and_run(itlbm_batch *b, int K) {
     int r;
     bool narrow = b->narrow;
     if (!b->tile_fixed) {
-        if ((r = window(-1, true, r_narrow)) != ITLBM_OK || (r = window(-1, false, r_uniform)) != ITLBM_OK)
-            return r;
-        // Narrow tiles only when faster by a tenth.  The choice holds for the cases that come later: a first table of
-        // boxes without a partial column measures nothing, and one large box may gain 3 to 5 % by them, where mixes
+        if ((r = window(-1, true, r_narrow)) != ITLBM_OK) return r;
+        bool cut = false;  // whether any case has a partial column
+        for (int p = 0; p < NTAB; p++) cut = cut || (shape_of_table(p) != SHAPE_32x8 && b->ntab[p] > 0);
+        if (cut && (r = window(-1, false, r_uniform)) != ITLBM_OK) return r;
+        // Narrow tiles only when faster by a tenth.  The choice holds for the cases that come later: boxes without a
+        // partial column measure nothing, and one large box may gain 3 to 5 % by them, where mixes
         // lose a quarter and each capture of a graph of three tables takes 10 ms instead of 1 (a served stream that
         // chose them by 2 % had a median of 0.29 s instead of 0.17).
-        narrow = r_narrow > 1.1 * r_uniform;
+        narrow = cut && r_narrow > 1.1 * r_uniform;
     } else {
         if ((r = window(-1, narrow, r_narrow)) != ITLBM_OK) return r;
         r_uniform = r_narrow;

@@ -132,8 +132,7 @@ struct ResPlan {
 };
 // CTAs of configuration `shape` the current device holds at once (0: no cooperative launch).
 int res_capacity(int prec, int shape);
-// Whether a stream has all the device's SMs (a green context's has not): asked by a cooperative launch of an empty
-// kernel that fills them.
+// Whether a stream has all the device's SMs: not one of a green context.
 bool res_whole_device(cudaStream_t st);
 // A plan as the C ABI reports it.
 itlbm_plan res_describe(int prec, const ResPlan &p);

@@ -61,27 +61,16 @@ int res_capacity(int prec, int shape) {
     return v ? ctas_per_sm(*v, prec, shape) * v->sms : 0;
 }
 
-__global__ void __launch_bounds__(1024) k_places() {}
-
 bool res_whole_device(cudaStream_t st) {
-    const Device *v = device();
-    int n = 0;
-    if (!v || cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_places, 1024, 0) != cudaSuccess) {
+    void *f = nullptr;
+    cudaDriverEntryPointQueryResult found = cudaDriverEntryPointSymbolNotFound;
+    if (cudaGetDriverEntryPointByVersion("cuStreamGetGreenCtx", &f, 12040, cudaEnableDefault, &found) != cudaSuccess ||
+        found != cudaDriverEntryPointSuccess) {
         cudaGetLastError();
-        return false;
+        return true;  // a driver without them
     }
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3((unsigned)(n * v->sms));
-    cfg.blockDim = dim3(1024);
-    cfg.stream = st;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeCooperative;
-    at.val.cooperative = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    const bool ok = cudaLaunchKernelEx(&cfg, k_places) == cudaSuccess;
-    if (!ok) cudaGetLastError();
-    return ok;
+    CUgreenCtx g = nullptr;
+    return ((decltype(&cuStreamGetGreenCtx))f)((CUstream)st, &g) == CUDA_SUCCESS && g == nullptr;
 }
 
 itlbm_plan res_describe(int prec, const ResPlan &p) {
